@@ -460,8 +460,10 @@ int tune_sweep(ske_engine e, const SdemLaunch& base, const std::vector<uint64_t>
 // so_masked (batched total viewshed, every sector's rows within dim_i): SO is
 // not zeroed first; the sweep writes every valid cell and the deskew reads the
 // others as zero.
+// bins_only (batched cepstrum): SO only feeds the max+angle deskew, so a cell may
+// hold any value of its 1000-wide bin.
 int run_operator(ske_engine e, int kernel, const Batch& b, float povh, int counts_only, bool rows_only = false,
-                 bool so_masked = false) {
+                 bool so_masked = false, bool bins_only = false) {
     switch (kernel) {
         case SKE_KERNEL_SDEM: {
             ItemPlan* plan = nullptr;
@@ -511,6 +513,13 @@ int run_operator(ske_engine e, int kernel, const Batch& b, float povh, int count
                                               e->d_tw + e->lr_taper_off, e->d_tw + e->tw_off_host[6], e->stream));
         }
         case SKE_KERNEL_CEPSTRUM: {
+            if (bins_only) {
+                SKE_CK(cudaMemsetAsync(e->d_SO, 0, sizeof(float) * e->stride * b.count, e->stream));
+                LaunchScope ls(e, "cepstrum", 2);
+                return ls.done(launch_cepstrum_bins(e->dg, b, e->d_SI, e->d_SO, e->stride, e->len, e->geo.max_H,
+                                                    std::max(e->dimx, e->dimy), e->d_tw + e->tw_off_host[6],
+                                                    e->d_tw + e->tw_off_host[5], e->stream));
+            }
             LaunchScope ls(e, "cepstrum", 1);
             return ls.done(launch_cepstrum(e->dg, b, e->d_SI, e->d_SO, e->stride, e->len, e->d_tw + e->tw_off_host[6],
                                            e->d_tw + e->tw_off_host[5], e->stream));
@@ -656,7 +665,7 @@ int accumulate_angles(ske_engine e, int kernel, const float* input, int input_on
         const bool rows_only = kernel == SKE_KERNEL_RADON && in_width;
         const bool so_masked = kernel == SKE_KERNEL_SDEM && in_width;
         if (!rows_only) SKE_TRY(run_skew(e, b, false));
-        SKE_TRY(run_operator(e, kernel, b, prm->povh, 0, rows_only, so_masked));
+        SKE_TRY(run_operator(e, kernel, b, prm->povh, 0, rows_only, so_masked, kernel == SKE_KERNEL_CEPSTRUM));
         SKE_TRY(run_deskew(e, b, is_max, prm->accum, rows_only, so_masked));
     }
     e->accum_mode = prm->accum;

@@ -244,10 +244,18 @@ cudaError_t launch_local_radon_f32(const DevGeometry& g, const Batch& b, const f
                                    int max_H, int max_cols, const double* gauss, const double* taper,
                                    cudaStream_t st);
 
-// Cepstrum blur estimation (k_cepstrum.cu).
+// Cepstrum blur estimation (k_cepstrum.cu): the reference's value of every valid
+// cell, zero elsewhere.
 cudaError_t launch_cepstrum(const DevGeometry& g, const Batch& b, const float* SI, float* SO,
                             int64_t stride, int64_t len, const double* tw64, const double* tw32,
                             cudaStream_t st);
+// The same for callers that only deskew SO with the maximum: a cell holds some
+// value of the reference value's 1000-wide bin (all the max+angle deskew sees),
+// decided in float where that is proven, else the reference's value.  SO holds
+// zeros.  max_H, max_cols: the batch's most rows and longest row.
+cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
+                                 int64_t len, int max_H, int max_cols, const double* tw64, const double* tw32,
+                                 cudaStream_t st);
 
 // Constant tables used by the SDEM sweep, uploaded once per device.
 cudaError_t sdem_init_tables();
