@@ -57,6 +57,7 @@ int ensure_device_tables(int device) {
     SKE_CK(sdem_init_tables());
     SKE_CK(cepstrum_f32_init_tables());
     if (lradon_f32_init_tables() != 0) return fail(SKE_ERR_CUDA, "local Radon float32 tables");
+    SKE_CK(lradon_init_tables());
     g_tables_ready[device] = 1;
     return SKE_OK;
 }
@@ -150,6 +151,8 @@ struct ske_engine_s {
     SkewMaps skew_maps;
     int4* d_lists = nullptr;  // survivor lists of the viewshed sweep
     size_t list_bytes = 0;
+    char* d_lradon = nullptr;  // window sums of the local Radon transform
+    size_t lradon_bytes = 0;
     float* h_pin = nullptr;
     std::map<std::vector<int>, ItemPlan> item_plans;
     // Per angle: every skewed row's valid range lies within dim_i (no row
@@ -333,6 +336,32 @@ int ensure_lists(ske_engine e, size_t bytes) {
     return SKE_OK;
 }
 
+// Scratch of the local Radon transform for as many of `want` sectors as 4 GB or
+// a quarter of the free memory hold (at least one); *slots: how many that is.
+int ensure_lradon(ske_engine e, int want, int* slots) {
+    const size_t one = lradon_scratch_bytes(e->geo.max_H, std::max(e->dimx, e->dimy), 1);
+    ske_engine own = e->parent ? e->parent : e;  // a child engine borrows its parent's
+    if (own->lradon_bytes < one * want) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+            cudaGetLastError();
+            free_b = (size_t)1 << 30;
+        }
+        const size_t budget = std::min((size_t)4 << 30, free_b / 4);
+        const size_t bytes = one * std::min<size_t>(want, std::max<size_t>(1, budget / one));
+        if (bytes > own->lradon_bytes) {
+            SKE_CK(cudaStreamSynchronize(e->stream));
+            cudaFree(own->d_lradon);
+            own->d_lradon = nullptr;
+            own->lradon_bytes = 0;
+            SKE_TRY(dev_alloc(&own->d_lradon, bytes));
+            own->lradon_bytes = bytes;
+        }
+    }
+    *slots = (int)std::min<size_t>(want, own->lradon_bytes / one);
+    return SKE_OK;
+}
+
 // Sectors per launch: as many as fit in a quarter of free memory (at most 180).
 int batch_capacity(ske_engine e, int nangles) {
     size_t free_b = 0, total_b = 0;
@@ -503,14 +532,22 @@ int run_operator(ske_engine e, int kernel, const Batch& b, float povh, int count
         }
         case SKE_KERNEL_LOCAL_RADON: {
             SKE_CK(cudaMemsetAsync(e->d_SO, 0, sizeof(float) * e->stride * b.count, e->stream));
-            LaunchScope ls(e, "local_radon", 1);
-            if (e->flags & SKE_FLAG_LOCAL_RADON_F32)
+            if (e->flags & SKE_FLAG_LOCAL_RADON_F32) {
+                LaunchScope ls(e, "local_radon", 1);
                 return ls.done(launch_local_radon_f32(e->dg, b, e->d_SI, e->d_SO, e->stride, e->geo.max_H,
                                                       std::max(e->dimx, e->dimy), e->d_tw + e->lr_gauss_off,
                                                       e->d_tw + e->lr_taper_off, e->stream));
-            return ls.done(launch_local_radon(e->dg, b, e->d_SI, e->d_SO, e->stride, e->geo.max_H,
-                                              std::max(e->dimx, e->dimy), e->d_tw + e->lr_gauss_off,
-                                              e->d_tw + e->lr_taper_off, e->d_tw + e->tw_off_host[6], e->stream));
+            }
+            int step = 1;
+            SKE_TRY(ensure_lradon(e, b.count, &step));
+            for (int s0 = 0; s0 < b.count; s0 += step) {
+                LaunchScope ls(e, "local_radon", kLocalRadonLaunches);
+                SKE_TRY(ls.done(launch_local_radon(
+                    e->dg, b, s0, std::min(step, b.count - s0), e->d_SI, e->d_SO, e->stride, e->len, e->geo.max_H,
+                    std::max(e->dimx, e->dimy), e->d_tw + e->lr_gauss_off, e->d_tw + e->lr_taper_off,
+                    e->d_tw + e->tw_off_host[6], (e->parent ? e->parent : e)->d_lradon, e->stream)));
+            }
+            return SKE_OK;
         }
         case SKE_KERNEL_CEPSTRUM: {
             if (bins_only) {
@@ -1472,7 +1509,7 @@ int ske_destroy(ske_engine e) {
     for (cudaEvent_t ev : e->event_pool) cudaEventDestroy(ev);
     void* bufs[] = {e->d_desc, e->d_target, e->d_first, e->d_last, e->d_weight, e->d_in, e->d_orient, e->d_acc,
                     e->d_comp, e->d_out, e->d_SI, e->d_SO, e->d_P, e->d_tw, e->d_tw_off, e->d_counter, e->d_status,
-                    e->d_lists};
+                    e->d_lists, e->d_lradon};
     for (void* b : bufs) cudaFree(b);
     if (e->h_pin) cudaFreeHost(e->h_pin);
     if (e->own_stream) cudaStreamDestroy(e->stream);

@@ -9,26 +9,39 @@
 //   Z       = FFT(Y) / 8;  out = getParameter(Z): from m = 5 the first
 //             |Z_m|^2 > |Z_{m-1}|^2 gives |Z_{m-1}|^2 (none: 0), stored as float.
 //
-// GB300 mapping
-//  * W(k, j) is shared by the 64 cells (k-32 .. k+31, j): a CTA takes a tile of
-//    kTI x kTJ cells, stages the skewed rows it needs (kTI+63 rows, kTJ+64
-//    columns, zeros outside the valid ranges) in shared memory and forms every
-//    W of the tile once, each as the reference's sequential binary64 sum, so
-//    the result is the reference's to the bit.
-//  * One warp per cell then gathers its column of 64 W values, applies the
-//    weights and runs both 64-point FFTs with one butterfly per lane per stage
-//    (warp_fft: the reference's DIF order and twiddle sequence, binary64,
-//    no fused operations).  The 1/sqrt(64) scaling is the reference's complex
-//    multiplication by (0.125, 0).
-//  * Tiles whose staged values are all finite use warp_fft_real (real-input
-//    first stage, multiplication-free last stage) and real scalings: the same
-//    values up to the sign of zeros, so the squared magnitudes, and the output,
-//    are bit-identical; other tiles keep every operation of the reference.
-//  * The Gaussian weights and the taper use host libm (local_radon_tables), as
-//    the reference computes them on the host.
-//  * Output cells past a row's span of the flat grid belong to the last row
-//    covering them (owner_row), as in the reference's row-order writes.
+// The output is the reference's, bit for bit, but most cells never run its two
+// binary64 transforms.  GB300 does 1/64 as many binary64 as float operations,
+// and the transforms alone held the operator at the FP64 pipe's rate (279 ms
+// per 512 x 512 image at all 180 angles, that pipe 83% busy).  Every value the
+// output depends on is a comparison or one rounding to float, so a cheaper
+// evaluation with a proven error decides it unless it falls within that error
+// of a tie (the whole run of that image: 278.7 ms before, 7.53 ms so):
+//  1. k_lradon_sums: W of every row, once per column (the tile-by-tile form
+//     recomputed each about three times), as exact 64-bit integer prefix sums
+//     where the reference's sequential binary64 sums make no rounding.
+//  2. k_lradon_cells, two cells per thread.  Both transforms and the weights
+//     compose into Z_m = sum over q of (W(i-q, j) + W(i+q, j)) F_m[q], q = 0..32
+//     (gauss and the kept bins' cosines are even around row i), so one Z_m is
+//     66 multiply-adds, and m runs from 4 only until the first ascent (m = 6 or
+//     7 on textures).  Float decides the ascent; the one Z_{m-1} the output
+//     needs is then formed in float pairs (about 2^-40) and rounded.
+//  3. k_lradon_exact: the cells neither step could decide (under 1% of a
+//     texture's) run the reference's transforms, one warp per cell.
+//
+// Error bounds (u = 2^-24, maxW = the largest |W| of the cell's column, SF_m =
+// sum over q of |F_m[q]| times the number of W it multiplies):
+//  * float Z_m: truncation of W to 24 bits 2u, the pair's sum u, F_m's rounding
+//    u, two chains of 17 multiply-adds 17u: within 24 u maxW SF_m.
+//  * float-pair Z_m: pairs of W, filters and products are good to a few u^2
+//    each; the four chains' rests (below 14 u maxW SF_m each) and their merge
+//    round at most 260 u^2 maxW SF_m away: 2^-39 maxW SF_m is used.
+//  * the reference's own binary64 result differs from the exact one by the
+//    rounding of its 12 stages and its iterated twiddles (up to 15 * 2^-53 off
+//    the unit circle in a stage of 64 points, 61 over a transform's stages): at
+//    most 45 * 2^-53 S, S = sum of |W| gauss <= maxW sum gauss; 2^-46 maxW sum
+//    gauss is used.
 #include <climits>
+#include <cmath>
 
 #include "kernels.h"
 
@@ -38,178 +51,523 @@ namespace {
 
 constexpr int kW = kLocalRadonWindow;  // 64
 constexpr int kHalf = kW / 2;          // 32
-constexpr int kTI = 32;                // cell rows per tile
-constexpr int kTJ = 32;                // cell columns per tile
-constexpr int kRows = kTI + kW - 1;    // W rows a tile needs
-constexpr int kCols = kTJ + kW;        // staged columns: kTJ windows of 65
 constexpr int kWarps = 8;
 
-struct Smem {
-    float s[kRows][kCols];
-    double w[kRows][kTJ];
-    cd x[kWarps][kW];  // per-warp FFT buffer; before the cell loop, a row's prefix sums
-    double gauss[kW];
-    double taper[kLocalRadonKeep];
-    double tw[2 * (kW - 1)];
-};
+// ---- window sums -------------------------------------------------------------
+// One warp per (row, 128 columns): the 192 cells the windows cover are staged,
+// every float is an integer multiple of 2^(e - 150), and when the cells'
+// exponents span at most 28 binades and the sum of their magnitudes in units of
+// the smallest 2^e stays below 2^53, every partial sum of the reference's
+// sequential binary64 loop is exact, so each window sum is a difference of two
+// 64-bit integer prefix sums.  Other blocks (or a non-finite cell) keep the
+// sequential adds.  Columns up to dim_l, rows of W with that pitch; memory
+// bound (8 bytes written per cell).
+constexpr int kSumCols = 128;
+constexpr int kSumStage = kSumCols + kW;  // 192: windows of 65 around 128 columns
 
 __global__ void __launch_bounds__(kWarps * 32)
-    k_lradon(DevGeometry g, Batch b, const float* __restrict__ SI, float* __restrict__ SO, int64_t stride,
-             int tiles_j, const double* __restrict__ gauss_all, const double* __restrict__ taper,
-             const double* __restrict__ tw64) {
-    extern __shared__ double smem_d[];
-    Smem& sm = *reinterpret_cast<Smem*>(smem_d);
-    const int slot = blockIdx.y;
+    k_lradon_sums(DevGeometry g, Batch b, int slot0, const float* __restrict__ SI, int64_t stride,
+                  double* __restrict__ W, int64_t wstride, int col_blocks) {
+    __shared__ float cells[kWarps][kSumStage];
+    __shared__ long long prefix[kWarps][kSumStage + 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = slot0 + blockIdx.y;
+    const SectorDesc& d = g.desc[b.angle[slot]];
+    const int unit = blockIdx.x * kWarps + warp;
+    const int r = unit / col_blocks, j0 = (unit % col_blocks) * kSumCols;
+    if (r >= d.H || j0 >= d.diml) return;  // warp-uniform
+    const int f = g.first[d.row_off + r], l = g.last[d.row_off + r];
+    double* out = W + blockIdx.y * wstride + (int64_t)r * d.diml;
+    if (l <= f || j0 + kSumCols + kHalf <= f || j0 - kHalf >= l) {  // no valid cell in any window
+        for (int j = j0 + lane; j < min(j0 + kSumCols, d.diml); j += 32) out[j] = 0.0;
+        return;
+    }
+    const float* row = SI + slot * stride + (int64_t)r * d.dim_i;
+    float* s = cells[warp];
+#pragma unroll
+    for (int t = 0; t < kSumStage / 32; t++) {
+        const int c = j0 - kHalf + lane + 32 * t;
+        s[lane + 32 * t] = c >= f && c < l ? row[c] : 0.0f;
+    }
+    __syncwarp();
+    constexpr int kPer = kSumStage / 32;  // 6 consecutive cells per lane
+    unsigned u[kPer], m[kPer];
+    int ee[kPer], emin = INT_MAX, emax = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        u[k] = __float_as_uint(s[kPer * lane + k]);
+        const int e8 = (int)((u[k] >> 23) & 0xffu);
+        m[k] = (u[k] & 0x7fffffu) | (e8 ? 0x800000u : 0u);
+        ee[k] = m[k] ? max(e8, 1) : INT_MAX;
+        emin = min(emin, ee[k]);
+        emax = max(emax, e8);
+    }
+    emin = __reduce_min_sync(0xffffffffu, emin);
+    emax = __reduce_max_sync(0xffffffffu, emax);
+    bool exact = emax != 0xff && (emin == INT_MAX || emax - emin <= 28);
+    long long incl = 0;
+    if (exact && emin != INT_MAX) {
+        long long v[kPer], excl = 0;
+        unsigned long long mag = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            const long long x = m[k] ? (long long)m[k] << (ee[k] - emin) : 0;  // < 2^52
+            v[k] = (u[k] >> 31) ? -x : x;
+            mag += (unsigned long long)x;
+            incl += v[k];
+        }
+        excl = incl;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        excl = incl - excl;
+        for (int o = 16; o > 0; o >>= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
+        exact = mag < (1ull << 53);
+        if (exact) {
+            long long* pre = prefix[warp];
+#pragma unroll
+            for (int k = 0; k < kPer; k++) {
+                pre[kPer * lane + k] = excl;
+                excl += v[k];
+            }
+            if (lane == 31) pre[kSumStage] = excl;
+            __syncwarp();
+            const double scale = __longlong_as_double((long long)(emin - 150 + 1023) << 52);
+            for (int t = lane; t < kSumCols && j0 + t < d.diml; t += 32)
+                out[j0 + t] = __dmul_rn(__ll2double_rn(pre[t + kW + 1] - pre[t]), scale);
+        }
+    } else if (exact) {  // all cells zero
+        for (int t = lane; t < kSumCols && j0 + t < d.diml; t += 32) out[j0 + t] = 0.0;
+    }
+    if (!exact) {
+        for (int t = lane; t < kSumCols && j0 + t < d.diml; t += 32) {
+            double acc = 0.0;
+            for (int k = 0; k <= kW; k++) acc = __dadd_rn(acc, (double)s[t + k]);
+            out[j0 + t] = acc;
+        }
+    }
+}
+
+// ---- composed filters --------------------------------------------------------
+// F_m[q] = gauss[32-q] K_m[q] for m = kM0 .. 31, with
+// K_m[q] = 1/64 sum over k < 26 of (-1)^k taper[k] cos(2 pi k q / 64)
+// e^(-2 pi i k m / 64) from the host (lradon_init_tables).  Per slot: the float
+// pairs {re, re rest, im, im rest} in [q][m] order, the floats alone in [m][q]
+// order, and the two sums the error bounds take.
+constexpr int kM0 = 4;
+constexpr int kMn = kHalf - kM0;  // 28
+constexpr int kQn = kHalf + 1;    // 33
+constexpr int kQp = kQn + 1;      // row pitch of the float table (16-byte rows)
+
+struct LrTable {
+    float4 pair[kQn][kMn];
+    float2 one[kMn][kQp];
+    float sf[kMn];  // sum over q of (W terms of q) |F_m[q]|, rounded up
+    float sg;       // sum of the 64 weights, rounded up
+    float unused[3];
+};
+
+__device__ double2 g_lr_kernel[kQn * kMn];  // K_m[q] at [q][m]
+
+__global__ void __launch_bounds__(256)
+    k_lradon_tables(Batch b, int slot0, const double* __restrict__ gauss_all, LrTable* __restrict__ tab) {
+    const int slot = slot0 + blockIdx.x;
+    const double* gauss = gauss_all + (int64_t)b.angle[slot] * kW;
+    LrTable& t = tab[blockIdx.x];
+    for (int k = threadIdx.x; k < kQn * kMn; k += blockDim.x) {
+        const int q = k / kMn, m = k % kMn;
+        const double2 K = g_lr_kernel[k];
+        const double re = K.x * gauss[kHalf - q], im = K.y * gauss[kHalf - q];
+        const float rh = (float)re, ih = (float)im;
+        t.pair[q][m] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
+        t.one[m][q] = make_float2(rh, ih);
+        if (q == 0) t.one[m][kQn] = make_float2(0.0f, 0.0f);
+    }
+    if (threadIdx.x < kMn) {
+        double s = 0.0;
+        for (int q = 0; q < kQn; q++) {
+            const double2 K = g_lr_kernel[q * kMn + threadIdx.x];
+            s += (q == 0 || q == kHalf ? 1.0 : 2.0) * gauss[kHalf - q] * (fabs(K.x) + fabs(K.y));
+        }
+        t.sf[threadIdx.x] = (float)(s * 1.00001);
+    }
+    if (threadIdx.x == kMn) {
+        double s = 0.0;
+        for (int m = 0; m < kW; m++) s += gauss[m];
+        t.sg = (float)(s * 1.00001);
+    }
+}
+
+// ---- cells ---------------------------------------------------------------------
+constexpr int kTI = 64;               // cell rows per tile
+constexpr int kTJ = 32;               // cell columns per tile (one lane each)
+constexpr int kRows = kTI + kW - 1;   // rows of W a tile needs
+constexpr float kUndecided = -1.0f;   // left in SO for k_lradon_exact (no output is negative)
+
+struct CellSmem {
+    float hi[kRows][kTJ], lo[kRows][kTJ];  // W = hi + lo, hi truncated to 24 bits
+    LrTable tab;
+};
+
+// A binary64 value as hi (its top 24 significand bits) + lo (the other 29,
+// rounded to 24), by bit operations: conversions run on the FP64 pipe.  Values
+// outside [2^-60, 2^60) other than zero give NaN, which leaves their cells
+// undecided.
+__device__ __forceinline__ void split(double w, float* hi, float* lo) {
+    const long long bits = __double_as_longlong(w);
+    const int e = (int)((bits >> 52) & 0x7ff);
+    const unsigned sign = (unsigned)(bits >> 32) & 0x80000000u;
+    if (e == 0 && (bits & 0x7fffffffffffffffll) == 0) {
+        *hi = *lo = 0.0f;
+        return;
+    }
+    if (e < 1023 - 60 || e >= 1023 + 60) {
+        *hi = *lo = __int_as_float(0x7fc00000);
+        return;
+    }
+    const unsigned fe = (unsigned)(e - 1023 + 127);
+    *hi = __uint_as_float(sign | (fe << 23) | ((unsigned)(bits >> 29) & 0x7fffffu));
+    const float unit = __uint_as_float(sign | ((fe - 52) << 23));  // 2^(exponent - 52), signed
+    *lo = __fmul_rn(__uint2float_rn((unsigned)bits & 0x1fffffffu), unit);
+}
+
+// max(a, |b|), NaN if either is.
+__device__ __forceinline__ float max_abs(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(fabsf(b)));
+    return r;
+}
+
+// (s, t) with s = fl(a + b) and t the exact rest (Knuth's two-sum).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
+// (sh, sl) += v * (fh + fl) for a pair v = vh + vl.
+__device__ __forceinline__ void pair_mac(float vh, float vl, float fh, float fl, float& sh, float& sl) {
+    const float p = __fmul_rn(vh, fh);
+    float pe = __fmaf_rn(vh, fh, -p);
+    pe = __fmaf_rn(vh, fl, pe);
+    pe = __fmaf_rn(vl, fh, pe);
+    float s, t;
+    two_sum(sh, p, s, t);
+    sh = s;
+    sl = __fadd_rn(sl, __fadd_rn(t, pe));
+}
+
+__global__ void __launch_bounds__(kWarps * 32, 2)
+    k_lradon_cells(DevGeometry g, Batch b, int slot0, const double* __restrict__ W, int64_t wstride,
+                   const LrTable* __restrict__ tabs, float* __restrict__ SO, int64_t stride, int tiles_j) {
+    extern __shared__ __align__(16) unsigned char smem_lr[];
+    CellSmem& sm = *reinterpret_cast<CellSmem*>(smem_lr);
+    const int slot = slot0 + blockIdx.y;
     const SectorDesc& d = g.desc[b.angle[slot]];
     const int i0 = (blockIdx.x / tiles_j) * kTI, j0 = (blockIdx.x % tiles_j) * kTJ;
-    if (i0 >= d.H) return;
+    if (i0 >= d.H || j0 >= d.diml) return;
     const int32_t* first = g.first + d.row_off;
     const int32_t* last = g.last + d.row_off;
-    // Skip tiles without a valid cell.
     int any = 0;
     for (int r = threadIdx.x; r < kTI; r += blockDim.x) {
         const int i = i0 + r;
         if (i < d.H && first[i] < j0 + kTJ && last[i] > j0 && first[i] < last[i]) any = 1;
     }
     if (!__syncthreads_or(any)) return;
-
-    const float* in = SI + slot * stride;
-    int bad = 0;
-    for (int t = threadIdx.x; t < kRows * kCols; t += blockDim.x) {
-        const int r = t / kCols, c = t % kCols;
-        const int k = i0 - kHalf + r, l = j0 - kHalf + c;
-        float v = 0.0f;
-        if (k >= 0 && k < d.H && l >= first[k] && l < last[k]) v = in[(int64_t)k * d.dim_i + l];
-        sm.s[r][c] = v;
-        bad |= !isfinite(v);
-    }
-    // Finite tiles take the reduced-work FFT (warp_fft_real); any non-finite
-    // input keeps every operation of the reference.
-    const bool finite = !__syncthreads_or(bad);
-    for (int t = threadIdx.x; t < kW; t += blockDim.x) sm.gauss[t] = gauss_all[(int64_t)b.angle[slot] * kW + t];
-    for (int t = threadIdx.x; t < kLocalRadonKeep; t += blockDim.x) sm.taper[t] = taper[t];
-    for (int t = threadIdx.x; t < 2 * (kW - 1); t += blockDim.x) sm.tw[t] = tw64[t];
-    __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // Window sums, one warp per staged row.  Every float is an integer multiple
-    // of 2^(e - 150); when the row's exponents span at most 28 binades and the
-    // sum of its magnitudes in units of its smallest 2^e stays below 2^53, every
-    // partial sum of the reference's sequential binary64 loop is exact, so each
-    // window sum is the exact sum: a difference of two 64-bit integer prefix
-    // sums.  Other rows (or a non-finite value) keep the sequential adds.
-    static_assert(kCols == 3 * 32, "three staged cells per lane");
-    static_assert(sizeof(cd) * kW >= sizeof(long long) * (kCols + 1), "prefix sums fit the FFT buffer");
+    const int j = j0 + lane;
+    const double* wcol = W + blockIdx.y * wstride + j;
     for (int r = warp; r < kRows; r += kWarps) {
-        const float* row = sm.s[r];
-        unsigned u[3], m[3];
-        int ee[3], emin = INT_MAX, emax = 0;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            u[k] = __float_as_uint(row[3 * lane + k]);
-            const int e8 = (int)((u[k] >> 23) & 0xffu);
-            m[k] = (u[k] & 0x7fffffu) | (e8 ? 0x800000u : 0u);
-            ee[k] = m[k] ? max(e8, 1) : INT_MAX;
-            emin = min(emin, ee[k]);
-            emax = max(emax, e8);
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            emin = min(emin, __shfl_xor_sync(0xffffffffu, emin, o));
-            emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-        }
-        bool exact = emax != 0xff && (emin == INT_MAX || emax - emin <= 28);
-        if (exact && emin != INT_MAX) {
-            long long v[3];
-            unsigned long long mag = 0;
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                const long long x = m[k] ? (long long)m[k] << (ee[k] - emin) : 0;  // < 2^52
-                v[k] = (u[k] >> 31) ? -x : x;
-                mag += (unsigned long long)x;
-            }
-            long long incl = v[0] + v[1] + v[2];
-            for (int o = 1; o < 32; o <<= 1) {
-                const long long t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            for (int o = 16; o > 0; o >>= 1) mag += __shfl_xor_sync(0xffffffffu, mag, o);
-            exact = mag < (1ull << 53);
-            if (exact) {
-                long long* pre = reinterpret_cast<long long*>(sm.x[warp]);  // idle until the cell loop
-                const long long excl = incl - (v[0] + v[1] + v[2]);
-                pre[3 * lane] = excl;
-                pre[3 * lane + 1] = excl + v[0];
-                pre[3 * lane + 2] = excl + v[0] + v[1];
-                if (lane == 31) pre[kCols] = incl;
-                __syncwarp();
-                const double scale = __longlong_as_double((long long)(emin - 150 + 1023) << 52);
-                sm.w[r][lane] = __dmul_rn(__ll2double_rn(pre[lane + kW + 1] - pre[lane]), scale);
-                __syncwarp();
-            }
-        } else if (exact) {
-            sm.w[r][lane] = 0.0;  // all cells zero
-        }
-        if (!exact) {
-            double acc = 0.0;
-            for (int k = 0; k <= kW; k++) acc = __dadd_rn(acc, (double)row[lane + k]);
-            sm.w[r][lane] = acc;
-        }
+        const int k = i0 - kHalf + r;
+        float h = 0.0f, l = 0.0f;
+        if (k >= 0 && k < d.H && j < d.diml) split(wcol[(int64_t)k * d.diml], &h, &l);
+        sm.hi[r][lane] = h;
+        sm.lo[r][lane] = l;
+    }
+    {
+        const int4* src = reinterpret_cast<const int4*>(tabs + blockIdx.y);
+        int4* dst = reinterpret_cast<int4*>(&sm.tab);
+        for (int k = threadIdx.x; k < (int)(sizeof(LrTable) / sizeof(int4)); k += blockDim.x) dst[k] = src[k];
     }
     __syncthreads();
 
-    cd* x = sm.x[warp];
-    const cd scale{0.125, 0.0};  // 1/sqrt(64) (helper.h:102-104)
+    constexpr float u = 5.9604644775390625e-8f;  // 2^-24
+    const float sg = sm.tab.sg;
     float* out = SO + slot * stride;
-    for (int cell = warp; cell < kTI * kTJ; cell += kWarps) {
-        const int ci = cell / kTJ, cj = cell % kTJ;
-        const int i = i0 + ci, j = j0 + cj;
-        if (i >= d.H || j < first[i] || j >= last[i]) continue;  // warp-uniform
-        const int64_t p = (int64_t)i * d.dim_i + j;
-        if (j >= d.dim_i && owner_row(d, first, last, p) != i) continue;
-        for (int m = lane; m < kW; m += 32) x[m] = cd{__dmul_rn(sm.w[ci + m][cj], sm.gauss[m]), 0.0};
-        __syncwarp();
-        // Only Re X_k for k < 26 is read: the pruned FFT forms Re X_k, k < 32.
-        if (finite) warp_fft_real<kKeepLowRe>(x, kW, sm.tw, lane);
-        else warp_fft(x, kW, sm.tw, lane);
-        for (int m = lane; m < kW; m += 32) {
-            double y = 0.0;
-            if (m < kLocalRadonKeep) {
-                // Finite: x * (0.125, 0) is (re/8, im/8) up to the sign of zeros.
-                const double re = finite ? __dmul_rn(x[m].re, 0.125) : cmul(x[m], scale).re;
-                y = __dmul_rn(sm.taper[m], re);
-            }
-            x[m] = cd{y, 0.0};
+    for (int ca = 2 * warp; ca < kTI; ca += 2 * kWarps) {
+        // Cells (i, j) and (i + 1, j), i = i0 + ca.
+        bool valid[2];
+        int64_t p[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const int i = i0 + ca + c;
+            valid[c] = i < d.H && j >= first[i] && j < last[i];
+            p[c] = (int64_t)i * d.dim_i + j;
+            if (valid[c] && j >= d.dim_i && owner_row(d, first, last, p[c]) != i) valid[c] = false;
         }
-        __syncwarp();
-        // Y is zero from bin 26 on; only Z_m for m < 32 is read.
-        if (finite) warp_fft_real<kKeepLow, true>(x, kW, sm.tw, lane);
-        else warp_fft(x, kW, sm.tw, lane);
-        x[lane] = finite ? cd{__dmul_rn(x[lane].re, 0.125), __dmul_rn(x[lane].im, 0.125)} : cmul(x[lane], scale);
-        __syncwarp();
-        // getParameter: from m = 5 the first |Z_m|^2 > |Z_{m-1}|^2 gives
-        // |Z_{m-1}|^2 (none: 0).  Lane m forms |Z_m|^2 (the reference's
-        // products and sum); a ballot finds the first ascent.
-        const double nm = __dadd_rn(__dmul_rn(x[lane].re, x[lane].re), __dmul_rn(x[lane].im, x[lane].im));
-        const double prev = __shfl_up_sync(0xffffffffu, nm, 1);
-        const unsigned asc = __ballot_sync(0xffffffffu, lane >= 5 && lane < kHalf && nm > prev);
-        const int ia = asc ? __ffs(asc) - 1 : 1;
-        const double v = __shfl_sync(0xffffffffu, nm, ia - 1);
-        if (lane == 0) out[p] = __double2float_rn(asc ? v : 0.0);
-        __syncwarp();
+        if (!__any_sync(0xffffffffu, valid[0] || valid[1])) continue;
+        // V_q of both cells; rows of the tile: cell i is staged row ca + 32.
+        float V[2][kQn], top = 0.0f, top1 = 0.0f;
+        {
+            const int c0 = ca + kHalf;
+            float up = sm.hi[c0 + 1][lane], dn = sm.hi[c0][lane];
+            V[0][0] = dn;
+            V[1][0] = up;
+            top = fabsf(dn);
+            top1 = fabsf(up);
+            // Row c0 - q + 1 is cell i+1's lower row and cell i's previous one.
+#pragma unroll
+            for (int q = 1; q < kHalf; q++) {
+                const float a0 = sm.hi[c0 - q][lane], b1 = sm.hi[c0 + 1 + q][lane];
+                V[0][q] = __fadd_rn(a0, up);
+                V[1][q] = __fadd_rn(dn, b1);
+                top = max_abs(max_abs(top, a0), up);
+                top1 = max_abs(max_abs(top1, dn), b1);
+                up = b1;
+                dn = a0;
+            }
+            V[0][kHalf] = sm.hi[c0 - kHalf][lane];
+            V[1][kHalf] = dn;
+            top = max_abs(top, V[0][kHalf]);
+            top1 = max_abs(top1, dn);
+        }
+        // First ascent in float.  state: 0 searching, 1 found (at[c] = m - 1), 2 undecided.
+        const float mw[2] = {top, top1};
+        float prev[2] = {0.0f, 0.0f}, ptol[2] = {0.0f, 0.0f};
+        int state[2], at[2] = {kM0, kM0};
+#pragma unroll
+        for (int c = 0; c < 2; c++) state[c] = valid[c] && mw[c] != 0.0f ? 0 : 2;
+        for (int m = kM0; m < kHalf; m++) {
+            if (!__any_sync(0xffffffffu, state[0] == 0 || state[1] == 0)) break;
+            const float4* t4 = reinterpret_cast<const float4*>(sm.tab.one[m - kM0]);
+            float zr[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, zi[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll
+            for (int q = 0; q < kQn; q += 2) {
+                const float4 t = t4[q / 2];
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    zr[c][0] = __fmaf_rn(V[c][q], t.x, zr[c][0]);
+                    zi[c][0] = __fmaf_rn(V[c][q], t.y, zi[c][0]);
+                    if (q + 1 < kQn) {
+                        zr[c][1] = __fmaf_rn(V[c][q + 1], t.z, zr[c][1]);
+                        zi[c][1] = __fmaf_rn(V[c][q + 1], t.w, zi[c][1]);
+                    }
+                }
+            }
+            const float sf = 24.0f * u * sm.tab.sf[m - kM0];
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const float re = __fadd_rn(zr[c][0], zr[c][1]), im = __fadd_rn(zi[c][0], zi[c][1]);
+                const float nm = __fmaf_rn(re, re, __fmul_rn(im, im));
+                // |Z|^2 is off by at most 2 |Z| e + e^2 and its own rounding
+                // (1e-36: of subnormal squares).
+                const float e = sf * mw[c];
+                const float tol = e * (2.02f * (fabsf(re) + fabsf(im)) + e) + 4.0f * u * nm + 1e-36f;
+                const float diff = __fsub_rn(nm, prev[c]);
+                if (m > kM0 && state[c] == 0) {
+                    if (!(fabsf(diff) > 1.01f * (tol + ptol[c]))) state[c] = 2;
+                    else if (diff > 0.0f) {
+                        state[c] = 1;
+                        at[c] = m - 1;
+                    }
+                }
+                prev[c] = nm;
+                ptol[c] = tol;
+            }
+        }
+        // The one |Z_m|^2 the output is, in float pairs, rounded where its whole
+        // error interval rounds to the same float.
+#pragma unroll 1
+        for (int c = 0; c < 2; c++) {
+            float res = kUndecided;
+            if (mw[c] == 0.0f) res = 0.0f;        // every W is zero: no ascent
+            else if (state[c] == 0) res = 0.0f;  // no ascent up to m = 31
+            if (__any_sync(0xffffffffu, state[c] == 1)) {
+                const int c0 = ca + c + kHalf, mi = at[c] - kM0;
+                float rh[4], rl[4], ih[4], il[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) rh[k] = rl[k] = ih[k] = il[k] = 0.0f;
+                {
+                    const float4 F = sm.tab.pair[0][mi];
+                    pair_mac(sm.hi[c0][lane], sm.lo[c0][lane], F.x, F.y, rh[0], rl[0]);
+                    pair_mac(sm.hi[c0][lane], sm.lo[c0][lane], F.z, F.w, ih[0], il[0]);
+                    const float4 E = sm.tab.pair[kHalf][mi];
+                    pair_mac(sm.hi[c0 - kHalf][lane], sm.lo[c0 - kHalf][lane], E.x, E.y, rh[1], rl[1]);
+                    pair_mac(sm.hi[c0 - kHalf][lane], sm.lo[c0 - kHalf][lane], E.z, E.w, ih[1], il[1]);
+                }
+#pragma unroll 1
+                for (int q0 = 1; q0 < kHalf; q0 += 4) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int q = q0 + k;
+                        if (q >= kHalf) break;
+                        float vh, vl;
+                        two_sum(sm.hi[c0 - q][lane], sm.hi[c0 + q][lane], vh, vl);
+                        vl = __fadd_rn(vl, __fadd_rn(sm.lo[c0 - q][lane], sm.lo[c0 + q][lane]));
+                        const float4 F = sm.tab.pair[q][mi];
+                        pair_mac(vh, vl, F.x, F.y, rh[k], rl[k]);
+                        pair_mac(vh, vl, F.z, F.w, ih[k], il[k]);
+                    }
+                }
+                float zr = rh[0], zrl = rl[0], zi = ih[0], zil = il[0];
+#pragma unroll
+                for (int k = 1; k < 4; k++) {
+                    float s, t;
+                    two_sum(zr, rh[k], s, t);
+                    zr = s;
+                    zrl = __fadd_rn(zrl, __fadd_rn(t, rl[k]));
+                    two_sum(zi, ih[k], s, t);
+                    zi = s;
+                    zil = __fadd_rn(zil, __fadd_rn(t, il[k]));
+                }
+                // |Z|^2 = a + r, a the larger part.
+                const float p0 = __fmul_rn(zr, zr), p1 = __fmul_rn(zi, zi);
+                float r0 = __fmaf_rn(zr, zr, -p0), r1 = __fmaf_rn(zi, zi, -p1);
+                r0 = __fmaf_rn(2.0f * zr, zrl, r0);
+                r1 = __fmaf_rn(2.0f * zi, zil, r1);
+                float a, r;
+                two_sum(p0, p1, a, r);
+                r = __fadd_rn(r, __fadd_rn(r0, r1));
+                // 2^-39 of the products' sum, 2^-46 of the reference's own, and the squares' rounding.
+                const float e = mw[c] * (1.8189894035458565e-12f * sm.tab.sf[mi] + 1.4210854715202004e-14f * sg);
+                const float del = e * (2.02f * (fabsf(zr) + fabsf(zi)) + e) + 1.8189894035458565e-12f * a;
+                const float lo = __fadd_rn(a, __fsub_rd(r, del)), hi = __fadd_rn(a, __fadd_ru(r, del));
+                // Squares below 2^-90 would lose their rests to the subnormal range.
+                if (state[c] == 1 && lo == hi && a > 8.0779356694631609e-28f) res = lo;
+            }
+            if (valid[c]) out[p[c]] = res;
+        }
+    }
+}
+
+// ---- undecided cells -------------------------------------------------------------
+// The reference's operations: one warp per cell, both 64-point transforms with
+// one butterfly per lane per stage (warp_fft: the reference's DIF order and
+// twiddle sequence, binary64, no fused operations).  The 1/sqrt(64) scaling is
+// the reference's complex multiplication by (0.125, 0).  Cells whose W are all
+// finite use warp_fft_real and real scalings: the same values up to the sign of
+// zeros, so the squared magnitudes are bit-identical.  A warp looks over 32
+// cells of SO at a time for the mark k_lradon_cells left.
+__global__ void __launch_bounds__(kWarps * 32)
+    k_lradon_exact(DevGeometry g, Batch b, int slot0, const double* __restrict__ W, int64_t wstride,
+                   float* __restrict__ SO, int64_t stride, int64_t len, const double* __restrict__ gauss_all,
+                   const double* __restrict__ taper_all, const double* __restrict__ tw64) {
+    __shared__ cd xs[kWarps][kW];
+    __shared__ double tw[2 * (kW - 1)], gauss[kW], taper[kLocalRadonKeep];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = slot0 + blockIdx.y;
+    const SectorDesc& d = g.desc[b.angle[slot]];
+    for (int t = threadIdx.x; t < 2 * (kW - 1); t += blockDim.x) tw[t] = tw64[t];
+    for (int t = threadIdx.x; t < kW; t += blockDim.x) gauss[t] = gauss_all[(int64_t)b.angle[slot] * kW + t];
+    for (int t = threadIdx.x; t < kLocalRadonKeep; t += blockDim.x) taper[t] = taper_all[t];
+    __syncthreads();
+    const int32_t* first = g.first + d.row_off;
+    const int32_t* last = g.last + d.row_off;
+    const double* w = W + blockIdx.y * wstride;
+    float* out = SO + slot * stride;
+    cd* x = xs[warp];
+    const cd scale{0.125, 0.0};  // 1/sqrt(64) (helper.h:102-104)
+    const int64_t end = min((int64_t)len, (int64_t)(d.H - 1) * d.dim_i + d.diml);
+    const int64_t step = (int64_t)gridDim.x * kWarps * 32;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; q0 < end; q0 += step) {
+        unsigned todo = __ballot_sync(0xffffffffu, q0 + lane < end && out[q0 + lane] == kUndecided);
+        while (todo) {
+            const int64_t p = q0 + __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int i = owner_row(d, first, last, p);  // warp-uniform, >= 0: only valid cells are marked
+            const int j = (int)(p - (int64_t)i * d.dim_i);
+            bool fin = true;
+            for (int m = lane; m < kW; m += 32) {
+                const int k = i - kHalf + m;
+                const double v = k >= 0 && k < d.H ? w[(int64_t)k * d.diml + j] : 0.0;
+                fin = fin && isfinite(v);
+                x[m] = cd{__dmul_rn(v, gauss[m]), 0.0};
+            }
+            const bool finite = __all_sync(0xffffffffu, fin);
+            __syncwarp();
+            // Only Re X_k for k < 26 is read: the pruned FFT forms Re X_k, k < 32.
+            if (finite) warp_fft_real<kKeepLowRe>(x, kW, tw, lane);
+            else warp_fft(x, kW, tw, lane);
+            for (int m = lane; m < kW; m += 32) {
+                double y = 0.0;
+                if (m < kLocalRadonKeep) {
+                    // Finite: x * (0.125, 0) is (re/8, im/8) up to the sign of zeros.
+                    const double re = finite ? __dmul_rn(x[m].re, 0.125) : cmul(x[m], scale).re;
+                    y = __dmul_rn(taper[m], re);
+                }
+                x[m] = cd{y, 0.0};
+            }
+            __syncwarp();
+            // Y is zero from bin 26 on; only Z_m for m < 32 is read.
+            if (finite) warp_fft_real<kKeepLow, true>(x, kW, tw, lane);
+            else warp_fft(x, kW, tw, lane);
+            x[lane] = finite ? cd{__dmul_rn(x[lane].re, 0.125), __dmul_rn(x[lane].im, 0.125)} : cmul(x[lane], scale);
+            __syncwarp();
+            // getParameter: from m = 5 the first |Z_m|^2 > |Z_{m-1}|^2 gives
+            // |Z_{m-1}|^2 (none: 0).  Lane m forms |Z_m|^2 (the reference's
+            // products and sum); a ballot finds the first ascent.
+            const double nm = __dadd_rn(__dmul_rn(x[lane].re, x[lane].re), __dmul_rn(x[lane].im, x[lane].im));
+            const double prev = __shfl_up_sync(0xffffffffu, nm, 1);
+            const unsigned asc = __ballot_sync(0xffffffffu, lane >= 5 && lane < kHalf && nm > prev);
+            const int ia = asc ? __ffs(asc) - 1 : 1;
+            const double v = __shfl_sync(0xffffffffu, nm, ia - 1);
+            if (lane == 0) out[p] = __double2float_rn(asc ? v : 0.0);
+            __syncwarp();
+        }
     }
 }
 
 }  // namespace
 
-cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
-                               int max_H, int max_cols, const double* gauss, const double* taper, const double* tw64,
-                               cudaStream_t st) {
-    if (b.count == 0) return cudaSuccess;
-    const int tiles_i = (max_H + kTI - 1) / kTI, tiles_j = (max_cols + kTJ - 1) / kTJ;
-    const size_t smem = sizeof(Smem);
-    cudaError_t e = cudaFuncSetAttribute(k_lradon, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t lradon_init_tables() {
+    static double2 K[kQn * kMn];
+    for (int q = 0; q < kQn; q++)
+        for (int m = 0; m < kMn; m++) {
+            double re = 0.0, im = 0.0;
+            for (int k = 1; k < kLocalRadonKeep; k++) {
+                const double taper = std::sin((k / (0.4 * kW - 1)) * M_PI_2);  // kernelRADN.h:157-161
+                const double c = std::cos(2.0 * M_PI * ((k * q) % kW) / kW) * taper * (k & 1 ? -1.0 : 1.0);
+                const double a = 2.0 * M_PI * ((k * (m + kM0)) % kW) / kW;
+                re += c * std::cos(a);
+                im -= c * std::sin(a);
+            }
+            K[q * kMn + m] = make_double2(re / kW, im / kW);
+        }
+    return cudaMemcpyToSymbol(g_lr_kernel, K, sizeof(K));
+}
+
+size_t lradon_scratch_bytes(int64_t max_rows, int diml, int slots) {
+    const size_t w = ((size_t)max_rows * diml * sizeof(double) + 255) / 256 * 256;
+    return (w + sizeof(LrTable)) * (size_t)slots;
+}
+
+cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, int count, const float* SI, float* SO,
+                               int64_t stride, int64_t len, int max_H, int max_cols, const double* gauss,
+                               const double* taper, const double* tw64, void* scratch, cudaStream_t st) {
+    if (count <= 0) return cudaSuccess;
+    const int64_t wstride = (int64_t)(((size_t)max_H * max_cols * sizeof(double) + 255) / 256 * 256 / sizeof(double));
+    double* W = static_cast<double*>(scratch);
+    LrTable* tabs = reinterpret_cast<LrTable*>(W + wstride * count);
+    k_lradon_tables<<<count, 256, 0, st>>>(b, slot0, gauss, tabs);
+    const int col_blocks = (max_cols + kSumCols - 1) / kSumCols;
+    const int64_t units = (int64_t)max_H * col_blocks;
+    k_lradon_sums<<<dim3((unsigned)((units + kWarps - 1) / kWarps), count), kWarps * 32, 0, st>>>(
+        g, b, slot0, SI, stride, W, wstride, col_blocks);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_lradon<<<dim3((unsigned)(tiles_i * tiles_j), b.count), kWarps * 32, smem, st>>>(g, b, SI, SO, stride, tiles_j,
-                                                                                      gauss, taper, tw64);
+    const size_t smem = sizeof(CellSmem);
+    e = cudaFuncSetAttribute(k_lradon_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int tiles_i = (max_H + kTI - 1) / kTI, tiles_j = (max_cols + kTJ - 1) / kTJ;
+    k_lradon_cells<<<dim3((unsigned)(tiles_i * tiles_j), count), kWarps * 32, smem, st>>>(g, b, slot0, W, wstride, tabs,
+                                                                                        SO, stride, tiles_j);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const int64_t chunks = (len + kWarps * 32 - 1) / (kWarps * 32);
+    const unsigned blocks = (unsigned)(chunks < 256 ? (chunks < 1 ? 1 : chunks) : 256);
+    k_lradon_exact<<<dim3(blocks, count), kWarps * 32, 0, st>>>(g, b, slot0, W, wstride, SO, stride, len, gauss, taper,
+                                                               tw64);
     return cudaGetLastError();
 }
 

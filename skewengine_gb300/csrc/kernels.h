@@ -224,11 +224,17 @@ int radon_launches(bool rows_only, int max_H2, bool f32 = false);
 // separate sums and transform; -1 for another value.
 int radon_select(int path);
 
-// Local Radon transform (k_lradon.cu): tiles of every sector up to max_H rows
-// and max_cols columns; gauss: 180 x 64 weights, taper: the kept bins' factors.
-cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
-                               int max_H, int max_cols, const double* gauss, const double* taper, const double* tw64,
-                               cudaStream_t st);
+// Local Radon transform (k_lradon.cu) of slots slot0 .. slot0 + count - 1: tiles
+// of every sector up to max_H rows and max_cols = dim_l columns; gauss: 180 x 64
+// weights, taper: the kept bins' factors; len: cells of a slot.  SO holds zeros.
+// scratch: lradon_scratch_bytes(max_H, max_cols, count) bytes.
+cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, int count, const float* SI, float* SO,
+                               int64_t stride, int64_t len, int max_H, int max_cols, const double* gauss,
+                               const double* taper, const double* tw64, void* scratch, cudaStream_t st);
+constexpr int kLocalRadonLaunches = 4;  // kernels of one launch_local_radon
+// The window sums of `slots` sectors of up to max_rows rows, and their filters.
+size_t lradon_scratch_bytes(int64_t max_rows, int diml, int slots);
+cudaError_t lradon_init_tables();  // the composed filters' kernel, once per device
 
 // Cepstrum blur estimation in float32, fused over the sector loop, for a batch
 // of square images of side dim (k_cepstrum_f32.cu): orientations from

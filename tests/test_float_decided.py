@@ -1,6 +1,7 @@
 """Operators whose float stage decides a cell and leaves the rest to binary64:
-the cepstrum of a whole run (bins decided in float) against the same sectors
-through the per-sector calls (every value in binary64).  Equal bits on inputs that take each route: textures,
+the local Radon transform against the oracle, and the cepstrum of a whole run
+(bins decided in float) against the same sectors through the per-sector calls
+(every value in binary64).  Equal bits on inputs that take each route: textures,
 rows at the tiles' edges, flat and empty images (nothing decided), values far
 from one, infinities and NaN."""
 import numpy as np
@@ -54,6 +55,16 @@ KINDS = ["texture", "bytes", "zero", "flat", "half", "signed", "tiny", "huge", "
 def same(a, b):
     nan = np.isnan(a)
     return np.array_equal(nan, np.isnan(b)) and bits_equal(np.where(nan, 0, a), np.where(nan, 0, b))
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("dims", SIZES)
+def test_local_radon_equals_oracle(ske, oracle, dims, kind):
+    dimx, dimy = dims
+    x = image(kind, dimx, dimy)
+    with ske.SkewEngine(dimx, dimy) as eng:
+        got = eng.run("localradon", x, angles=ANGLES)
+    assert same(got, oracle.run_angles(5, x, ANGLES))
 
 
 @pytest.mark.parametrize("kind", KINDS)
