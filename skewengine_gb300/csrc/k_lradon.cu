@@ -15,7 +15,8 @@
 // per 512 x 512 image at all 180 angles, that pipe 83% busy).  Every value the
 // output depends on is a comparison or one rounding to float, so a cheaper
 // evaluation with a proven error decides it unless it falls within that error
-// of a tie (the whole run of that image: 278.7 ms before, 7.53 ms so):
+// of a tie (the whole run of that image: 278.7 ms before, 3.7 ms so, of it 0.25 ms
+// in step 1, 2.4 in step 2 and 0.6 in step 3):
 //  1. k_lradon_sums: W of every row, once per column (the tile-by-tile form
 //     recomputed each about three times), as exact 64-bit integer prefix sums
 //     where the reference's sequential binary64 sums make no rounding.
@@ -24,21 +25,27 @@
 //     (gauss and the kept bins' cosines are even around row i), so one Z_m is
 //     66 multiply-adds, and m runs from 4 only until the first ascent (m = 6 or
 //     7 on textures).  Float decides the ascent; the one Z_{m-1} the output
-//     needs is then formed in float pairs (about 2^-40) and rounded.
-//  3. k_lradon_exact: the cells neither step could decide (under 1% of a
-//     texture's) run the reference's transforms, one warp per cell.
+//     needs is then formed from 28-bit integers, whose products add up without
+//     rounding in 64 bits, and float corrections, and rounded.
+//  3. k_lradon_exact: the cells neither step could decide (about one in a
+//     thousand of a texture's) run the reference's transforms, one warp per cell.
 //
-// Error bounds (u = 2^-24, maxW = the largest |W| of the cell's column, SF_m =
-// sum over q of |F_m[q]| times the number of W it multiplies):
-//  * float Z_m: truncation of W to 24 bits 2u, the pair's sum u, F_m's rounding
-//    u, two chains of 17 multiply-adds 17u: within 24 u maxW SF_m.
-//  * float-pair Z_m: pairs of W, filters and products are good to a few u^2
-//    each; the four chains' rests (below 14 u maxW SF_m each) and their merge
-//    round at most 260 u^2 maxW SF_m away: 2^-39 maxW SF_m is used.
+// W of a column of a tile is hi + lo in units of g, the largest |W| of the column
+// being 2^26 .. 2^27 of them: hi an integer, |lo| <= 1/2.  F is an integer of
+// 2^-30 units plus a rest.  Error bounds in g (u = 2^-24, maxW = the largest |W|
+// of the cell's rows, SF_m = sum over q of |F_m[q]| times the W it multiplies):
+//  * float Z_m: lo left out, SF_m / 2; rounding of hi, of the pair's sum, of F_m
+//    and of the last sum, u each; and u for every addition from q's own to the
+//    end of its chain, q/2 + 1 of them since the chains run from q = 32 down to
+//    0, towards the large F: together u maxW SW_m, SW_m = sum of (q/2 + 5) times
+//    |F_m[q]|, formed per sector (LrTable).
+//  * integer Z_m: lo and the rest of F are good to 2^-24 and 2^-55; the two float
+//    chains of 33 corrections below 1 and 5 leave at most 33 u (1 + 5) = 1.2e-5;
+//    F_m itself is good to 2^-46 maxW.
 //  * the reference's own binary64 result differs from the exact one by the
 //    rounding of its 12 stages and its iterated twiddles (up to 15 * 2^-53 off
 //    the unit circle in a stage of 64 points, 61 over a transform's stages): at
-//    most 45 * 2^-53 S, S = sum of |W| gauss <= maxW sum gauss; 2^-46 maxW sum
+//    most 45 * 2^-53 S, S = sum of |W| gauss <= maxW sum gauss; 2^-47 maxW sum
 //    gauss is used.
 #include <climits>
 #include <cmath>
@@ -152,20 +159,19 @@ __global__ void __launch_bounds__(kWarps * 32)
 // ---- composed filters --------------------------------------------------------
 // F_m[q] = gauss[32-q] K_m[q] for m = kM0 .. 31, with
 // K_m[q] = 1/64 sum over k < 26 of (-1)^k taper[k] cos(2 pi k q / 64)
-// e^(-2 pi i k m / 64) from the host (lradon_init_tables).  Per slot: the float
-// pairs {re, re rest, im, im rest} in [q][m] order, the floats alone in [m][q]
-// order, and the two sums the error bounds take.
+// e^(-2 pi i k m / 64) from the host (lradon_init_tables).
 constexpr int kM0 = 4;
 constexpr int kMn = kHalf - kM0;  // 28
 constexpr int kQn = kHalf + 1;    // 33
 constexpr int kQp = kQn + 1;      // row pitch of the float table (16-byte rows)
 
 struct LrTable {
-    float4 pair[kQn][kMn];
-    float2 one[kMn][kQp];
-    float sf[kMn];  // sum over q of (W terms of q) |F_m[q]|, rounded up
-    float sg;       // sum of the 64 weights, rounded up
-    float unused[3];
+    int4 fix[kQn][kMn];    // {re, im} in 2^-30 units, {re, im} as float bits
+    float2 rest[kQn][kMn];  // what the integers leave of re and im
+    float2 one[kMn][kQp];  // {re, im}, rows for the float search
+    float sf[kMn], sw[kMn];  // SF_m and SW_m, rounded up
+    float sg;                // sum of the 64 weights, rounded up
+    float unused[7];
 };
 
 __device__ double2 g_lr_kernel[kQn * kMn];  // K_m[q] at [q][m]
@@ -179,64 +185,68 @@ __global__ void __launch_bounds__(256)
         const int q = k / kMn, m = k % kMn;
         const double2 K = g_lr_kernel[k];
         const double re = K.x * gauss[kHalf - q], im = K.y * gauss[kHalf - q];
-        const float rh = (float)re, ih = (float)im;
-        t.pair[q][m] = make_float4(rh, (float)(re - (double)rh), ih, (float)(im - (double)ih));
-        t.one[m][q] = make_float2(rh, ih);
+        const int ri = __double2int_rn(re * 1073741824.0), ii = __double2int_rn(im * 1073741824.0);
+        t.fix[q][m] = make_int4(ri, ii, __float_as_int((float)re), __float_as_int((float)im));
+        t.rest[q][m] = make_float2((float)(re - ri * 9.3132257461547852e-10), (float)(im - ii * 9.3132257461547852e-10));
+        t.one[m][q] = make_float2((float)re, (float)im);
         if (q == 0) t.one[m][kQn] = make_float2(0.0f, 0.0f);
     }
     if (threadIdx.x < kMn) {
-        double s = 0.0;
+        double s = 0.0, w = 0.0;
         for (int q = 0; q < kQn; q++) {
             const double2 K = g_lr_kernel[q * kMn + threadIdx.x];
-            s += (q == 0 || q == kHalf ? 1.0 : 2.0) * gauss[kHalf - q] * (fabs(K.x) + fabs(K.y));
+            const double v = (q == 0 || q == kHalf ? 1.0 : 2.0) * gauss[kHalf - q] * sqrt(K.x * K.x + K.y * K.y);
+            s += v;
+            w += v * (q / 2 + 5);
         }
-        t.sf[threadIdx.x] = (float)(s * 1.00001);
+        t.sf[threadIdx.x] = (float)(s * 1.001);
+        t.sw[threadIdx.x] = (float)(w * 1.001);
     }
     if (threadIdx.x == kMn) {
         double s = 0.0;
         for (int m = 0; m < kW; m++) s += gauss[m];
-        t.sg = (float)(s * 1.00001);
+        t.sg = (float)(s * 1.001);
     }
 }
 
 // ---- cells ---------------------------------------------------------------------
-constexpr int kTI = 64;               // cell rows per tile
+constexpr int kTI = 128;              // cell rows per tile: 191 rows of W and one copy of the filters serve them (64
+                                      // rows: 2.68 ms against 2.42 at 512 x 512)
 constexpr int kTJ = 32;               // cell columns per tile (one lane each)
 constexpr int kRows = kTI + kW - 1;   // rows of W a tile needs
+constexpr int kPerWarp = (kRows + kWarps - 1) / kWarps;
 constexpr float kUndecided = -1.0f;   // left in SO for k_lradon_exact (no output is negative)
 
 struct CellSmem {
-    float hi[kRows][kTJ], lo[kRows][kTJ];  // W = hi + lo, hi truncated to 24 bits
+    int2 w[kRows][kTJ];      // W = hi + lo in units of the column's g: {hi, lo as float bits}
+    float hif[kRows][kTJ];   // hi as float
+    int top[kWarps][kTJ];    // largest exponent field of the column, per warp's rows
+    int2 range[kTI];         // {first, last} of the tile's cell rows ({0, 0} past the last)
     LrTable tab;
 };
 
-// A binary64 value as hi (its top 24 significand bits) + lo (the other 29,
-// rounded to 24), by bit operations: conversions run on the FP64 pipe.  Values
-// outside [2^-60, 2^60) other than zero give NaN, which leaves their cells
-// undecided.
-__device__ __forceinline__ void split(double w, float* hi, float* lo) {
+// Binary64 w in units of 2^(emax - 1023 - 26), emax at least w's exponent field:
+// hi the nearest integer, lo the rest to 2^-25 (bit operations: conversions run
+// on the FP64 pipe).
+__device__ __forceinline__ void split(double w, int emax, int* hi, float* lo) {
     const long long bits = __double_as_longlong(w);
     const int e = (int)((bits >> 52) & 0x7ff);
-    const unsigned sign = (unsigned)(bits >> 32) & 0x80000000u;
-    if (e == 0 && (bits & 0x7fffffffffffffffll) == 0) {
-        *hi = *lo = 0.0f;
-        return;
+    const long long s = (bits & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
+    const int t = min(26 + emax - e, 88);  // w = s 2^-t units
+    long long h = 0, rem = s;
+    if (t <= 60) {
+        h = (s + (1ll << (t - 1))) >> t;
+        rem = s - (h << t);
     }
-    if (e < 1023 - 60 || e >= 1023 + 60) {
-        *hi = *lo = __int_as_float(0x7fc00000);
-        return;
-    }
-    const unsigned fe = (unsigned)(e - 1023 + 127);
-    *hi = __uint_as_float(sign | (fe << 23) | ((unsigned)(bits >> 29) & 0x7fffffu));
-    const float unit = __uint_as_float(sign | ((fe - 52) << 23));  // 2^(exponent - 52), signed
-    *lo = __fmul_rn(__uint2float_rn((unsigned)bits & 0x1fffffffu), unit);
+    const float l = __fmul_rn(__int2float_rn((int)(rem >> min(t - 26, 63))), 1.4901161193847656e-8f);  // 2^-26
+    *hi = bits < 0 ? -(int)h : (int)h;
+    *lo = bits < 0 ? -l : l;
 }
 
-// max(a, |b|), NaN if either is.
-__device__ __forceinline__ float max_abs(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(fabsf(b)));
-    return r;
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 // (s, t) with s = fl(a + b) and t the exact rest (Knuth's two-sum).
@@ -246,16 +256,13 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
     t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
-// (sh, sl) += v * (fh + fl) for a pair v = vh + vl.
-__device__ __forceinline__ void pair_mac(float vh, float vl, float fh, float fl, float& sh, float& sl) {
-    const float p = __fmul_rn(vh, fh);
-    float pe = __fmaf_rn(vh, fh, -p);
-    pe = __fmaf_rn(vh, fl, pe);
-    pe = __fmaf_rn(vl, fh, pe);
-    float s, t;
-    two_sum(sh, p, s, t);
-    sh = s;
-    sl = __fadd_rn(sl, __fadd_rn(t, pe));
+// acc 2^-30 + c as a normalised float pair (|acc 2^-30| < 2^30, |c| small).
+__device__ __forceinline__ void to_pair(long long acc, float c, float& h, float& l) {
+    const int ah = (int)(acc >> 30);
+    const float fh = __int2float_rn(ah);
+    const float rest = __int2float_rn(ah - __float2int_rn(fh));
+    const float low = __fmaf_rn(__int2float_rn((int)(acc & 0x3fffffff)), 9.3132257461547852e-10f, rest);
+    two_sum(fh, __fadd_rn(low, c), h, l);
 }
 
 __global__ void __launch_bounds__(kWarps * 32, 2)
@@ -272,78 +279,101 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     int any = 0;
     for (int r = threadIdx.x; r < kTI; r += blockDim.x) {
         const int i = i0 + r;
-        if (i < d.H && first[i] < j0 + kTJ && last[i] > j0 && first[i] < last[i]) any = 1;
+        const int2 fl = i < d.H ? make_int2(first[i], last[i]) : make_int2(0, 0);
+        sm.range[r] = fl;
+        if (fl.x < j0 + kTJ && fl.y > j0 && fl.x < fl.y) any = 1;
     }
     if (!__syncthreads_or(any)) return;
+    // The sector's filters, while the window sums are fetched and split.
+    for (int k = threadIdx.x; k < (int)(sizeof(LrTable) / 16); k += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(reinterpret_cast<int4*>(&sm.tab) + k)),
+                     "l"(reinterpret_cast<const int4*>(tabs + blockIdx.y) + k));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = j0 + lane;
-    const double* wcol = W + blockIdx.y * wstride + j;
-    for (int r = warp; r < kRows; r += kWarps) {
-        const int k = i0 - kHalf + r;
-        float h = 0.0f, l = 0.0f;
-        if (k >= 0 && k < d.H && j < d.diml) split(wcol[(int64_t)k * d.diml], &h, &l);
-        sm.hi[r][lane] = h;
-        sm.lo[r][lane] = l;
-    }
+    int emax = 0;  // largest exponent field of the column's W
     {
-        const int4* src = reinterpret_cast<const int4*>(tabs + blockIdx.y);
-        int4* dst = reinterpret_cast<int4*>(&sm.tab);
-        for (int k = threadIdx.x; k < (int)(sizeof(LrTable) / sizeof(int4)); k += blockDim.x) dst[k] = src[k];
+        const double* wcol = W + blockIdx.y * wstride + j;
+        double w[kPerWarp];
+#pragma unroll
+        for (int t = 0; t < kPerWarp; t++) {
+            const int r = warp + t * kWarps, k = i0 - kHalf + r;
+            w[t] = r < kRows && k >= 0 && k < d.H && j < d.diml ? wcol[(int64_t)k * d.diml] : 0.0;
+            emax = max(emax, (int)((__double_as_longlong(w[t]) >> 52) & 0x7ff));
+        }
+        sm.top[warp][lane] = emax;
+        __syncthreads();
+        for (int t = 0; t < kWarps; t++) emax = max(emax, sm.top[t][lane]);
+#pragma unroll
+        for (int t = 0; t < kPerWarp; t++) {
+            const int r = warp + t * kWarps;
+            if (r >= kRows) continue;
+            int h;
+            float l;
+            split(w[t], emax, &h, &l);
+            sm.w[r][lane] = make_int2(h, __float_as_int(l));
+            sm.hif[r][lane] = __int2float_rn(h);
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     constexpr float u = 5.9604644775390625e-8f;  // 2^-24
     const float sg = sm.tab.sg;
+    // g as a float; columns with a non-finite W or one outside the range where g
+    // and the squares stay normal floats are left undecided.
+    const bool col_ok = emax == 0 || (emax > 1023 - 30 && emax < 1023 + 80);
+    const float unit = __uint_as_float((unsigned)min(max(emax - 1023 - 26 + 127, 1), 254) << 23);
     float* out = SO + slot * stride;
     for (int ca = 2 * warp; ca < kTI; ca += 2 * kWarps) {
-        // Cells (i, j) and (i + 1, j), i = i0 + ca.
+        // Cells (i, j) and (i + 1, j), i = i0 + ca; cell i is staged row ca + 32.
         bool valid[2];
         int64_t p[2];
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const int i = i0 + ca + c;
-            valid[c] = i < d.H && j >= first[i] && j < last[i];
+            valid[c] = j >= sm.range[ca + c].x && j < sm.range[ca + c].y;
             p[c] = (int64_t)i * d.dim_i + j;
             if (valid[c] && j >= d.dim_i && owner_row(d, first, last, p[c]) != i) valid[c] = false;
         }
         if (!__any_sync(0xffffffffu, valid[0] || valid[1])) continue;
-        // V_q of both cells; rows of the tile: cell i is staged row ca + 32.
-        float V[2][kQn], top = 0.0f, top1 = 0.0f;
+        // V_q of both cells.
+        const int c0 = ca + kHalf;
+        float V[2][kQn], mw[2];
         {
-            const int c0 = ca + kHalf;
-            float up = sm.hi[c0 + 1][lane], dn = sm.hi[c0][lane];
+            float up = sm.hif[c0 + 1][lane], dn = sm.hif[c0][lane];
             V[0][0] = dn;
             V[1][0] = up;
-            top = fabsf(dn);
-            top1 = fabsf(up);
+            mw[0] = fabsf(dn);
+            mw[1] = fabsf(up);
             // Row c0 - q + 1 is cell i+1's lower row and cell i's previous one.
 #pragma unroll
             for (int q = 1; q < kHalf; q++) {
-                const float a0 = sm.hi[c0 - q][lane], b1 = sm.hi[c0 + 1 + q][lane];
+                const float a0 = sm.hif[c0 - q][lane], b1 = sm.hif[c0 + 1 + q][lane];
                 V[0][q] = __fadd_rn(a0, up);
                 V[1][q] = __fadd_rn(dn, b1);
-                top = max_abs(max_abs(top, a0), up);
-                top1 = max_abs(max_abs(top1, dn), b1);
+                mw[0] = fmaxf(fmaxf(mw[0], fabsf(a0)), fabsf(up));
+                mw[1] = fmaxf(fmaxf(mw[1], fabsf(dn)), fabsf(b1));
                 up = b1;
                 dn = a0;
             }
-            V[0][kHalf] = sm.hi[c0 - kHalf][lane];
+            V[0][kHalf] = sm.hif[c0 - kHalf][lane];
             V[1][kHalf] = dn;
-            top = max_abs(top, V[0][kHalf]);
-            top1 = max_abs(top1, dn);
+            mw[0] = fmaxf(mw[0], fabsf(V[0][kHalf]));
+            mw[1] = fmaxf(mw[1], fabsf(dn));
         }
-        // First ascent in float.  state: 0 searching, 1 found (at[c] = m - 1), 2 undecided.
-        const float mw[2] = {top, top1};
+        // First ascent in float.  state: 0 searching, 1 found (at[c] = m - 1), 2
+        // undecided, 3 too close between at[c] = m - 1 and m.
         float prev[2] = {0.0f, 0.0f}, ptol[2] = {0.0f, 0.0f};
         int state[2], at[2] = {kM0, kM0};
 #pragma unroll
-        for (int c = 0; c < 2; c++) state[c] = valid[c] && mw[c] != 0.0f ? 0 : 2;
+        for (int c = 0; c < 2; c++) state[c] = valid[c] && col_ok && mw[c] != 0.0f ? 0 : 2;
         for (int m = kM0; m < kHalf; m++) {
             if (!__any_sync(0xffffffffu, state[0] == 0 || state[1] == 0)) break;
             const float4* t4 = reinterpret_cast<const float4*>(sm.tab.one[m - kM0]);
             float zr[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, zi[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
 #pragma unroll
-            for (int q = 0; q < kQn; q += 2) {
+            for (int q = kHalf; q >= 0; q -= 2) {
                 const float4 t = t4[q / 2];
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
@@ -355,20 +385,19 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                     }
                 }
             }
-            const float sf = 24.0f * u * sm.tab.sf[m - kM0];
+            const float sf = 0.51f * sm.tab.sf[m - kM0], sw = u * sm.tab.sw[m - kM0];
 #pragma unroll
             for (int c = 0; c < 2; c++) {
                 const float re = __fadd_rn(zr[c][0], zr[c][1]), im = __fadd_rn(zi[c][0], zi[c][1]);
                 const float nm = __fmaf_rn(re, re, __fmul_rn(im, im));
-                // |Z|^2 is off by at most 2 |Z| e + e^2 and its own rounding
-                // (1e-36: of subnormal squares).
-                const float e = sf * mw[c];
-                const float tol = e * (2.02f * (fabsf(re) + fabsf(im)) + e) + 4.0f * u * nm + 1e-36f;
+                // |Z|^2 is off by at most 2 |Z| e + e^2 and its own rounding.
+                const float e = __fmaf_rn(sw, mw[c] + 1.0f, sf);
+                const float tol = __fmaf_rn(e, __fmaf_rn(2.01f, sqrt_approx(nm), e), 4.0f * u * nm);
                 const float diff = __fsub_rn(nm, prev[c]);
                 if (m > kM0 && state[c] == 0) {
-                    if (!(fabsf(diff) > 1.01f * (tol + ptol[c]))) state[c] = 2;
-                    else if (diff > 0.0f) {
-                        state[c] = 1;
+                    const bool sure = fabsf(diff) > 1.01f * (tol + ptol[c]);
+                    if (!sure || diff > 0.0f) {
+                        state[c] = sure ? 1 : 3;
                         at[c] = m - 1;
                     }
                 }
@@ -376,51 +405,47 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 ptol[c] = tol;
             }
         }
-        // The one |Z_m|^2 the output is, in float pairs, rounded where its whole
-        // error interval rounds to the same float.
-#pragma unroll 1
+        // The one |Z_m|^2 the output is in integers, rounded where its whole error
+        // interval rounds to the same float.  Cells float left too close go on
+        // from there, one m at a time.
+#pragma unroll
         for (int c = 0; c < 2; c++) {
+            const int cc = c0 + c;
             float res = kUndecided;
-            if (mw[c] == 0.0f) res = 0.0f;        // every W is zero: no ascent
-            else if (state[c] == 0) res = 0.0f;  // no ascent up to m = 31
-            if (__any_sync(0xffffffffu, state[c] == 1)) {
-                const int c0 = ca + c + kHalf, mi = at[c] - kM0;
-                float rh[4], rl[4], ih[4], il[4];
+            if (state[c] == 0) res = 0.0f;  // no ascent up to m = 31
+            if (mw[c] == 0.0f && col_ok) {
+                // Every hi is zero: where every W is (no lo either), there is no ascent.
+                float l = 0.0f;
+                for (int k = -kHalf; k < kHalf; k++) l = fmaxf(l, fabsf(__int_as_float(sm.w[cc + k][lane].y)));
+                if (l == 0.0f) res = 0.0f;
+            }
+            float pa = 0.0f, pr = 0.0f, pd = 0.0f;  // |Z|^2 of the last m: pa + pr, off by at most pd
+            int mi = at[c] - kM0;
+            for (int step = 0; __any_sync(0xffffffffu, step == 0 ? (state[c] & 1) : state[c] == 3); step++) {
+                long long ar = 0, ai = 0;
+                float lr = 0.0f, li = 0.0f, fr = 0.0f, fi = 0.0f;
+                auto tap = [&](int q, int vi, float vl) {
+                    const float vf = __int2float_rn(vi);
+                    const int4 F = sm.tab.fix[q][mi];
+                    const float2 R = sm.tab.rest[q][mi];
+                    ar += (long long)vi * F.x;
+                    ai += (long long)vi * F.y;
+                    lr = __fmaf_rn(vl, __int_as_float(F.z), lr);
+                    li = __fmaf_rn(vl, __int_as_float(F.w), li);
+                    fr = __fmaf_rn(vf, R.x, fr);
+                    fi = __fmaf_rn(vf, R.y, fi);
+                };
+                const int2 wc = sm.w[cc][lane], we = sm.w[cc - kHalf][lane];
+                tap(0, wc.x, __int_as_float(wc.y));
+                tap(kHalf, we.x, __int_as_float(we.y));
 #pragma unroll
-                for (int k = 0; k < 4; k++) rh[k] = rl[k] = ih[k] = il[k] = 0.0f;
-                {
-                    const float4 F = sm.tab.pair[0][mi];
-                    pair_mac(sm.hi[c0][lane], sm.lo[c0][lane], F.x, F.y, rh[0], rl[0]);
-                    pair_mac(sm.hi[c0][lane], sm.lo[c0][lane], F.z, F.w, ih[0], il[0]);
-                    const float4 E = sm.tab.pair[kHalf][mi];
-                    pair_mac(sm.hi[c0 - kHalf][lane], sm.lo[c0 - kHalf][lane], E.x, E.y, rh[1], rl[1]);
-                    pair_mac(sm.hi[c0 - kHalf][lane], sm.lo[c0 - kHalf][lane], E.z, E.w, ih[1], il[1]);
+                for (int q = 1; q < kHalf; q++) {
+                    const int2 wa = sm.w[cc - q][lane], wb = sm.w[cc + q][lane];
+                    tap(q, wa.x + wb.x, __fadd_rn(__int_as_float(wa.y), __int_as_float(wb.y)));
                 }
-#pragma unroll 1
-                for (int q0 = 1; q0 < kHalf; q0 += 4) {
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const int q = q0 + k;
-                        if (q >= kHalf) break;
-                        float vh, vl;
-                        two_sum(sm.hi[c0 - q][lane], sm.hi[c0 + q][lane], vh, vl);
-                        vl = __fadd_rn(vl, __fadd_rn(sm.lo[c0 - q][lane], sm.lo[c0 + q][lane]));
-                        const float4 F = sm.tab.pair[q][mi];
-                        pair_mac(vh, vl, F.x, F.y, rh[k], rl[k]);
-                        pair_mac(vh, vl, F.z, F.w, ih[k], il[k]);
-                    }
-                }
-                float zr = rh[0], zrl = rl[0], zi = ih[0], zil = il[0];
-#pragma unroll
-                for (int k = 1; k < 4; k++) {
-                    float s, t;
-                    two_sum(zr, rh[k], s, t);
-                    zr = s;
-                    zrl = __fadd_rn(zrl, __fadd_rn(t, rl[k]));
-                    two_sum(zi, ih[k], s, t);
-                    zi = s;
-                    zil = __fadd_rn(zil, __fadd_rn(t, il[k]));
-                }
+                float zr, zrl, zi, zil;
+                to_pair(ar, __fadd_rn(lr, fr), zr, zrl);
+                to_pair(ai, __fadd_rn(li, fi), zi, zil);
                 // |Z|^2 = a + r, a the larger part.
                 const float p0 = __fmul_rn(zr, zr), p1 = __fmul_rn(zi, zi);
                 float r0 = __fmaf_rn(zr, zr, -p0), r1 = __fmaf_rn(zi, zi, -p1);
@@ -429,13 +454,26 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 float a, r;
                 two_sum(p0, p1, a, r);
                 r = __fadd_rn(r, __fadd_rn(r0, r1));
-                // 2^-39 of the products' sum, 2^-46 of the reference's own, and the squares' rounding.
-                const float e = mw[c] * (1.8189894035458565e-12f * sm.tab.sf[mi] + 1.4210854715202004e-14f * sg);
-                const float del = e * (2.02f * (fabsf(zr) + fabsf(zi)) + e) + 1.8189894035458565e-12f * a;
-                const float lo = __fadd_rn(a, __fsub_rd(r, del)), hi = __fadd_rn(a, __fadd_ru(r, del));
-                // Squares below 2^-90 would lose their rests to the subnormal range.
-                if (state[c] == 1 && lo == hi && a > 8.0779356694631609e-28f) res = lo;
+                // 2^-46 of F, 2^-47 sum gauss of the reference; 2^-42 a of the squares.
+                const float e = __fmaf_rn(mw[c] + 1.0f, 1.4210854715202004e-14f + 7.1054273576010019e-15f * sg, 1.6e-5f);
+                const float del = __fmaf_rn(e, __fmaf_rn(2.01f, sqrt_approx(a), e), 2.2737367544323206e-13f * a);
+                bool next = true;  // this m becomes the last one
+                if (step > 0) {
+                    const float diff = __fadd_rn(__fsub_rn(a, pa), __fsub_rn(r, pr));
+                    const bool sure = fabsf(diff) > 1.01f * (del + pd) + 2.0f * u * fabsf(diff);
+                    next = state[c] == 3 && sure && diff < 0.0f;
+                    if (state[c] == 3 && !next) state[c] = sure ? 1 : 2;
+                }
+                if (next) pa = a, pr = r, pd = del;
+                if (state[c] == 3 && ++mi == kMn) {
+                    state[c] = 2;
+                    res = 0.0f;  // no ascent up to m = 31
+                }
             }
+            const float lo = __fadd_rn(pa, __fsub_rd(pr, pd)), hi = __fadd_rn(pa, __fadd_ru(pr, pd));
+            // In the input's units, where that loses nothing.
+            const float v = __fmul_rn(__fmul_rn(lo, unit), unit);
+            if (state[c] == 1 && lo == hi && v > 1e-35f && v < 1e38f) res = v;
             if (valid[c]) out[p[c]] = res;
         }
     }
