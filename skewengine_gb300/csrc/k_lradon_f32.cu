@@ -50,14 +50,28 @@ __constant__ float c_tx[kW * kKP];
 __constant__ float c_tzc[kZn * kKP];
 __constant__ float c_tzs[kZn * kKP];
 
+// Packed pairs of floats (f32x2): two independent IEEE operations, round to
+// nearest, so the bits of the scalar ones.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0,%1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 struct SmemF {
     float s[kRows][kCols];
     float w[kRows][kTJ];
     float gauss[kW];
     float taper[kKP];
     float tx[kW][kKP];
-    float tzc[kZn][kKP];
-    float tzs[kZn][kKP];
+    float2 tz[kZn][kKeep];  // {cos, sin}
 };
 
 __global__ void __launch_bounds__(kThreads)
@@ -89,9 +103,9 @@ __global__ void __launch_bounds__(kThreads)
     for (int t = threadIdx.x; t < kW; t += blockDim.x) sm.gauss[t] = (float)gauss_all[(int64_t)b.angle[slot] * kW + t];
     for (int t = threadIdx.x; t < kKeep; t += blockDim.x) sm.taper[t] = (float)taper[t];
     for (int t = threadIdx.x; t < kW * kKP; t += blockDim.x) (&sm.tx[0][0])[t] = c_tx[t];
-    for (int t = threadIdx.x; t < kZn * kKP; t += blockDim.x) {
-        (&sm.tzc[0][0])[t] = c_tzc[t];
-        (&sm.tzs[0][0])[t] = c_tzs[t];
+    for (int t = threadIdx.x; t < kZn * kKeep; t += blockDim.x) {
+        const int m = t / kKeep, k = t % kKeep;
+        sm.tz[m][k] = make_float2(c_tzc[m * kKP + k], c_tzs[m * kKP + k]);
     }
     __syncthreads();
     // Window sums: warp per row, lane per column, 65 sequential adds.
@@ -118,58 +132,65 @@ __global__ void __launch_bounds__(kThreads)
             p[u] = (int64_t)i * d.dim_i + j;
             if (valid[u] && j >= d.dim_i && owner_row(d, first, last, p[u]) != i) valid[u] = false;
         }
+        const unsigned act = __ballot_sync(0xffffffffu, valid[0] || valid[1]);
         if (!valid[0] && !valid[1]) continue;
-        float re[2][kKeep];
+        // Bins k and k + 1 of a cell in one pair.
+        f2 acc[2][kKeep / 2];
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
-            for (int k = 0; k < kKeep; k++) re[u][k] = 0.0f;
+            for (int k = 0; k < kKeep / 2; k++) acc[u][k] = 0;
 #pragma unroll 2
         for (int m = 0; m < kW; m++) {
             const float gm = sm.gauss[m];
             const float x0 = __fmul_rn(sm.w[ca + m][cj], gm);
             const float x1 = __fmul_rn(sm.w[ca + kTI / 2 + m][cj], gm);
+            const f2 x0p = pk(x0, x0), x1p = pk(x1, x1);
             const float4* t4 = reinterpret_cast<const float4*>(sm.tx[m]);
 #pragma unroll
             for (int q = 0; q < kKP / 4; q++) {
                 const float4 t = t4[q];
-                const float tv[4] = {t.x, t.y, t.z, t.w};
+                const f2 tv[2] = {pk(t.x, t.y), pk(t.z, t.w)};
 #pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (4 * q + e < kKeep) {
-                        re[0][4 * q + e] = __fmaf_rn(x0, tv[e], re[0][4 * q + e]);
-                        re[1][4 * q + e] = __fmaf_rn(x1, tv[e], re[1][4 * q + e]);
+                for (int e = 0; e < 2; e++)
+                    if (2 * q + e < kKeep / 2) {
+                        acc[0][2 * q + e] = fma2(x0p, tv[e], acc[0][2 * q + e]);
+                        acc[1][2 * q + e] = fma2(x1p, tv[e], acc[1][2 * q + e]);
                     }
             }
         }
+        float re[2][kKeep];
 #pragma unroll
         for (int u = 0; u < 2; u++)
 #pragma unroll
-            for (int k = 0; k < kKeep; k++) re[u][k] = __fmul_rn(sm.taper[k], __fmul_rn(re[u][k], 0.125f));
+            for (int k = 0; k < kKeep; k += 2) {
+                upk(acc[u][k / 2], re[u][k], re[u][k + 1]);
+                re[u][k] = __fmul_rn(sm.taper[k], __fmul_rn(re[u][k], 0.125f));
+                re[u][k + 1] = __fmul_rn(sm.taper[k + 1], __fmul_rn(re[u][k + 1], 0.125f));
+            }
+        // m goes on only while a cell of the warp has seen no ascent: m = 6 or 7
+        // on textures, not 31.
         float prev[2] = {0.0f, 0.0f}, found[2] = {0.0f, 0.0f};
-        bool done[2] = {false, false};
-#pragma unroll 2
+        bool done[2] = {!valid[0], !valid[1]};
         for (int m = kZ0; m < kZ1; m++) {
-            float zr[2] = {0.0f, 0.0f}, zi[2] = {0.0f, 0.0f};
-            const float4* tc4 = reinterpret_cast<const float4*>(sm.tzc[m - kZ0]);
-            const float4* ts4 = reinterpret_cast<const float4*>(sm.tzs[m - kZ0]);
+            if (__all_sync(act, done[0] && done[1])) break;
+            f2 z[2] = {0, 0};  // {re, im}
+            const float4* t4 = reinterpret_cast<const float4*>(sm.tz[m - kZ0]);
 #pragma unroll
-            for (int q = 0; q < kKP / 4; q++) {
-                const float4 c = tc4[q], sn = ts4[q];
-                const float cv[4] = {c.x, c.y, c.z, c.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+            for (int q = 0; q < kKeep / 2; q++) {
+                const float4 t = t4[q];
+                const f2 ta = pk(t.x, t.y), tb = pk(t.z, t.w);
 #pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (4 * q + e < kKeep) {
-#pragma unroll
-                        for (int u = 0; u < 2; u++) {
-                            zr[u] = __fmaf_rn(re[u][4 * q + e], cv[e], zr[u]);
-                            zi[u] = __fmaf_rn(re[u][4 * q + e], sv[e], zi[u]);
-                        }
-                    }
+                for (int u = 0; u < 2; u++) {
+                    z[u] = fma2(pk(re[u][2 * q], re[u][2 * q]), ta, z[u]);
+                    z[u] = fma2(pk(re[u][2 * q + 1], re[u][2 * q + 1]), tb, z[u]);
+                }
             }
 #pragma unroll
             for (int u = 0; u < 2; u++) {
-                const float a = __fmul_rn(zr[u], 0.125f), bq = __fmul_rn(zi[u], 0.125f);
+                float zr, zi;
+                upk(z[u], zr, zi);
+                const float a = __fmul_rn(zr, 0.125f), bq = __fmul_rn(zi, 0.125f);
                 const float nm = __fadd_rn(__fmul_rn(a, a), __fmul_rn(bq, bq));
                 if (m > kZ0 && !done[u] && nm > prev[u]) {
                     found[u] = prev[u];
