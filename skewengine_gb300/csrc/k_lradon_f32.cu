@@ -16,9 +16,12 @@
 // twiddles (cosines and sines of 2 pi (k m mod 64) / 64, rounded to float on
 // the host) sit in shared memory as one row per m, read by every thread at the
 // same address (broadcast, 16 bytes per load), with the 26 bins unrolled in
-// registers.  Two cells per thread (a twiddle row serves both); a CTA of 256
-// threads owns a 32 x 32 tile of cells, stages the skewed rows it needs (95
-// rows x 96 columns) and forms each W once.
+// registers.  Two cells per thread (a twiddle row serves both), their bins in
+// packed f32x2 operations; the second transform stops at the bin where both have
+// ascended.  A CTA of 256 threads owns a 128 x 32 tile of cells, stages the
+// skewed rows it needs (191 rows x 96 columns) and forms each W once.  Bound by
+// the FP32 pipe: 1.4e9 packed multiply-adds per 512 x 512 image (32-row tiles
+// formed every W three times, and all 28 bins of every cell: 9.4 ms).
 // The order of the float32 sums differs from the reference's binary64 FFT, so
 // values differ in their last bits, and where two successive |Z|^2 nearly tie
 // the first ascent can fall on another bin: the rate of output cells that
@@ -36,8 +39,8 @@ namespace {
 constexpr int kW = kLocalRadonWindow;  // 64
 constexpr int kHalf = kW / 2;          // 32
 constexpr int kKeep = kLocalRadonKeep;  // 26
-constexpr int kTI = 32, kTJ = 32;
-constexpr int kRows = kTI + kW - 1;  // 95 W rows a tile needs
+constexpr int kTI = 128, kTJ = 32;   // cells of a tile
+constexpr int kRows = kTI + kW - 1;  // 191 W rows a tile needs
 constexpr int kCols = kTJ + kW;      // 96 staged columns
 constexpr int kThreads = 256;
 constexpr int kZ0 = 4, kZ1 = 32;  // |Z_m|^2 formed for m = kZ0 .. kZ1 - 1
@@ -46,9 +49,10 @@ constexpr int kKP = 28;  // twiddle row pitch (kKeep padded to 16 bytes)
 
 // Row m of the first transform: cos(2 pi k m / 64); rows m = kZ0.. of the
 // second: cos and sin of 2 pi k m / 64; k < kKeep, zero padding.
-__constant__ float c_tx[kW * kKP];
-__constant__ float c_tzc[kZn * kKP];
-__constant__ float c_tzs[kZn * kKP];
+// (Global arrays: the lanes of a warp copy different entries to shared memory,
+// which a constant bank would serve one at a time.)
+__device__ float g_tx[kW * kKP];
+__device__ float2 g_tz[kZn * kKeep];  // {cos, sin}
 
 // Packed pairs of floats (f32x2): two independent IEEE operations, round to
 // nearest, so the bits of the scalar ones.
@@ -66,6 +70,8 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
 }
 
 struct SmemF {
+    int2 range[kRows];  // {first, last} of the staged rows ({0, 0} outside the grid)
+    int2 pad;
     float s[kRows][kCols];
     float w[kRows][kTJ];
     float gauss[kW];
@@ -85,50 +91,65 @@ __global__ void __launch_bounds__(kThreads)
     if (i0 >= d.H) return;
     const int32_t* first = g.first + d.row_off;
     const int32_t* last = g.last + d.row_off;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int any = 0;
-    for (int r = threadIdx.x; r < kTI; r += blockDim.x) {
-        const int i = i0 + r;
-        if (i < d.H && first[i] < j0 + kTJ && last[i] > j0 && first[i] < last[i]) any = 1;
+    for (int r = threadIdx.x; r < kRows; r += blockDim.x) {
+        const int k = i0 - kHalf + r;
+        const int2 fl = k >= 0 && k < d.H ? make_int2(first[k], last[k]) : make_int2(0, 0);
+        sm.range[r] = fl;
+        if (r >= kHalf && r < kHalf + kTI && fl.x < j0 + kTJ && fl.y > j0 && fl.x < fl.y) any = 1;
     }
     if (!__syncthreads_or(any)) return;
 
+    // Staged rows: a warp per row, three columns per lane, four rows in flight.
     const float* in = SI + slot * stride;
-    for (int t = threadIdx.x; t < kRows * kCols; t += blockDim.x) {
-        const int r = t / kCols, c = t % kCols;
-        const int k = i0 - kHalf + r, l = j0 - kHalf + c;
-        float v = 0.0f;
-        if (k >= 0 && k < d.H && l >= first[k] && l < last[k]) v = in[(int64_t)k * d.dim_i + l];
-        sm.s[r][c] = v;
+#pragma unroll 4
+    for (int r = warp; r < kRows; r += kThreads / 32) {
+        const int2 fl = sm.range[r];
+        const float* row = in + (int64_t)(i0 - kHalf + r) * d.dim_i;
+#pragma unroll
+        for (int t = 0; t < kCols / 32; t++) {
+            const int l = j0 - kHalf + lane + 32 * t;
+            sm.s[r][lane + 32 * t] = l >= fl.x && l < fl.y ? row[l] : 0.0f;
+        }
     }
     for (int t = threadIdx.x; t < kW; t += blockDim.x) sm.gauss[t] = (float)gauss_all[(int64_t)b.angle[slot] * kW + t];
     for (int t = threadIdx.x; t < kKeep; t += blockDim.x) sm.taper[t] = (float)taper[t];
-    for (int t = threadIdx.x; t < kW * kKP; t += blockDim.x) (&sm.tx[0][0])[t] = c_tx[t];
-    for (int t = threadIdx.x; t < kZn * kKeep; t += blockDim.x) {
-        const int m = t / kKeep, k = t % kKeep;
-        sm.tz[m][k] = make_float2(c_tzc[m * kKP + k], c_tzs[m * kKP + k]);
-    }
+    for (int t = threadIdx.x; t < kW * kKP; t += blockDim.x) (&sm.tx[0][0])[t] = g_tx[t];
+    for (int t = threadIdx.x; t < kZn * kKeep; t += blockDim.x) (&sm.tz[0][0])[t] = g_tz[t];
     __syncthreads();
-    // Window sums: warp per row, lane per column, 65 sequential adds.
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = warp; r < kRows; r += kThreads / 32) {
-        float acc = 0.0f;
-#pragma unroll 5
-        for (int l = 0; l <= kW; l++) acc = __fadd_rn(acc, sm.s[r][lane + l]);
-        sm.w[r][lane] = acc;
+    // Window sums, 65 sequential adds each: four columns of a row per thread, so
+    // a 16-byte load serves up to 16 of them.
+    for (int t = threadIdx.x; t < kRows * (kTJ / 4); t += kThreads) {
+        const int r = t / (kTJ / 4), c = 4 * (t % (kTJ / 4));
+        const float4* src = reinterpret_cast<const float4*>(&sm.s[r][c]);
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i <= kW / 4; i++) {
+            const float4 v4 = src[i];
+            const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (4 * i + e >= k && 4 * i + e - k <= kW) acc[k] = __fadd_rn(acc[k], v[e]);
+        }
+        *reinterpret_cast<float4*>(&sm.w[r][c]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     }
     __syncthreads();
 
-    // Two cells per thread, rows ci and ci + kTI/2 of the tile: every twiddle
-    // row and window weight read from shared memory serves both.
+    // Two cells per thread, rows ca and ca + 1 of the tile: every twiddle row and
+    // window weight read from shared memory serves both.
     float* out = SO + slot * stride;
-    for (int ca = warp; ca < kTI / 2; ca += kThreads / 32) {
+    for (int ca = 2 * warp; ca < kTI; ca += 2 * (kThreads / 32)) {
         const int cj = lane, j = j0 + cj;
         int64_t p[2];
         bool valid[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const int i = i0 + ca + u * (kTI / 2);
-            valid[u] = i < d.H && j >= first[i] && j < last[i];
+            const int i = i0 + ca + u;
+            const int2 fl = sm.range[kHalf + ca + u];
+            valid[u] = j >= fl.x && j < fl.y;
             p[u] = (int64_t)i * d.dim_i + j;
             if (valid[u] && j >= d.dim_i && owner_row(d, first, last, p[u]) != i) valid[u] = false;
         }
@@ -140,11 +161,11 @@ __global__ void __launch_bounds__(kThreads)
         for (int u = 0; u < 2; u++)
 #pragma unroll
             for (int k = 0; k < kKeep / 2; k++) acc[u][k] = 0;
-#pragma unroll 2
+#pragma unroll 16  // fewer moves of the accumulators: 4.4 ms at 2, 3.7 at 8, 3.56 at 16
         for (int m = 0; m < kW; m++) {
             const float gm = sm.gauss[m];
             const float x0 = __fmul_rn(sm.w[ca + m][cj], gm);
-            const float x1 = __fmul_rn(sm.w[ca + kTI / 2 + m][cj], gm);
+            const float x1 = __fmul_rn(sm.w[ca + 1 + m][cj], gm);
             const f2 x0p = pk(x0, x0), x1p = pk(x1, x1);
             const float4* t4 = reinterpret_cast<const float4*>(sm.tx[m]);
 #pragma unroll
@@ -208,19 +229,18 @@ __global__ void __launch_bounds__(kThreads)
 }  // namespace
 
 int lradon_f32_init_tables() {
-    static float tx[kW * kKP], tzc[kZn * kKP], tzs[kZn * kKP];
+    static float tx[kW * kKP];
+    static float2 tz[kZn * kKeep];
     for (int m = 0; m < kW; m++)
         for (int k = 0; k < kKP; k++)
             tx[m * kKP + k] = k < kKeep ? (float)std::cos(2.0 * M_PI * ((k * m) % kW) / kW) : 0.0f;
     for (int m = kZ0; m < kZ1; m++)
-        for (int k = 0; k < kKP; k++) {
+        for (int k = 0; k < kKeep; k++) {
             const double a = 2.0 * M_PI * ((k * m) % kW) / kW;
-            tzc[(m - kZ0) * kKP + k] = k < kKeep ? (float)std::cos(a) : 0.0f;
-            tzs[(m - kZ0) * kKP + k] = k < kKeep ? (float)std::sin(a) : 0.0f;
+            tz[(m - kZ0) * kKeep + k] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
-    if (cudaMemcpyToSymbol(c_tx, tx, sizeof(tx)) != cudaSuccess) return -1;
-    if (cudaMemcpyToSymbol(c_tzc, tzc, sizeof(tzc)) != cudaSuccess) return -1;
-    if (cudaMemcpyToSymbol(c_tzs, tzs, sizeof(tzs)) != cudaSuccess) return -1;
+    if (cudaMemcpyToSymbol(g_tx, tx, sizeof(tx)) != cudaSuccess) return -1;
+    if (cudaMemcpyToSymbol(g_tz, tz, sizeof(tz)) != cudaSuccess) return -1;
     return 0;
 }
 
