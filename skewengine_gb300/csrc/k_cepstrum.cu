@@ -22,15 +22,19 @@
 // pipe 84% busy).  So the cepstrum is formed in float with a bound on its error
 // (one thread per cell, the window in registers), and only the cells whose bin
 // that leaves open run the exact kernel.  The whole run of a 512 x 512 texture
-// (180 angles): 353.3 ms with every cell in binary64, 3.96 ms so.
+// (180 angles): 353.3 ms with every cell in binary64, 3.20 ms so (the float
+// kernel 2.2, the open cells 0.6).
 //  * Windows with all 64 cells inside the row lose their centre cell's value
-//    first: only X_0 depends on the mean, and a smaller window sum makes every
-//    bound smaller.
-//  * X is off by at most 52 u L1 (u = 2^-24, L1 = sum of |window| after that
-//    subtraction): five stages of fused butterflies at 6 u, the real-input split
-//    (1.42 times their sum), its own 6 u and the subtraction's u.
-//  * log |X_n|^2 is off by at most 2.2 |dX| / |X_n| while that is below 0.05,
-//    plus the logarithm's 2^-22 (max(1, |log2|)); log |X_n|^2 + log |X_{32-n}|^2
+//    first: only X_0 depends on the mean, and a smaller window makes every bound
+//    smaller.
+//  * X is off, as a vector, by at most 240 u |window| (u = 2^-24, Euclidean
+//    norms): the transform is sqrt(32) times a unitary one, and its stages are
+//    off by u (two stages of plain additions), 5.8 u (three of fused
+//    butterflies), 8 u (the real-input split) and u (the subtraction) of their
+//    norm, 29 u together; X_0 takes another sqrt(2).
+//  * log |X_n|^2 is off by at most 2.2 |dX_n| / |X_n| while that is below 0.05,
+//    the sum over n by Cauchy's inequality by 2.2 |dX| (sum of 1 / |X_n|^2)^1/2;
+//    the logarithm itself by 2^-22 max(1, |log2|); log |X_n|^2 + log |X_{32-n}|^2
 //    is the logarithm of the product, 17 logarithms instead of 32.
 //  * Scaling X by a constant only moves c_0, which nothing reads.
 //  * c_4 .. c_15 are cosine sums folded over n, 16 - n and 8 - n: 62
@@ -187,9 +191,9 @@ __device__ __forceinline__ float lg2(float x) {
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float rsq(float x) {
+__device__ __forceinline__ float rcp(float x) {
     float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -197,19 +201,19 @@ __device__ __forceinline__ float rsq(float x) {
 // full: every sample lies inside the row (mean: the window's centre sample).
 __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float mean) {
     constexpr float u = 5.9604644775390625e-8f;  // 2^-24
-    float re[32], im[32], l1 = 0.0f;
+    float re[32], im[32], l2 = 0.0f;
 #pragma unroll
     for (int n = 0; n < 32; n++) {  // z_n = w[2n] + i w[2n+1], stored bit-reversed
         const float a = __fsub_rn(w[2 * n], mean), c = __fsub_rn(w[2 * n + 1], mean);
         re[brev5(n)] = a;
         im[brev5(n)] = c;
-        l1 += fabsf(a);
-        l1 += fabsf(c);
+        l2 = __fmaf_rn(a, a, l2);
+        l2 = __fmaf_rn(c, c, l2);
     }
     fft32_fused(re, im);
     // 2 X_k = E + W64^k O, E = Z_k + conj Z_{32-k}, O = -i (Z_k - conj Z_{32-k});
     // 2 X_{32-k} = conj(E - W64^k O).  e[n] = log2 |2 X_n|^2 |2 X_{32-n}|^2, inv =
-    // sum of 1 / |2 X_n|, all of it: of the logs' magnitudes.
+    // sum of 1 / |2 X_n|^2, all: of the logs' magnitudes.
     float e[17], inv = 0.0f, all = 0.0f;
     {
         const float x0 = __fmaf_rn(128.0f, mean, __fmul_rn(2.0f, __fadd_rn(re[0], im[0])));
@@ -217,7 +221,7 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
         const float p16 = __fmul_rn(4.0f, __fmaf_rn(re[16], re[16], __fmul_rn(im[16], im[16])));
         e[0] = lg2(p0);
         e[16] = lg2(p16);
-        inv = rsq(p0) + rsq(p16);
+        inv = rcp(p0) + rcp(p16);
         all = fabsf(e[0]) + fabsf(e[16]);
     }
 #pragma unroll
@@ -230,8 +234,8 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
         const float vr = __fmaf_rn(2.0f, er, -ur), vi = __fmaf_rn(2.0f, ei, -ui);
         const float pk = __fmaf_rn(ur, ur, __fmul_rn(ui, ui)), pm = __fmaf_rn(vr, vr, __fmul_rn(vi, vi));
         e[k] = lg2(__fmul_rn(pk, pm));
-        inv += rsq(pk);
-        inv += rsq(pm);
+        inv += rcp(pk);
+        inv += rcp(pm);
         all += fabsf(e[k]);
     }
     // T_k = e_0 + (-1)^k e_16 + sum over 0 < n < 16 of e_n cos(2 pi k n / 32); c_k = T_k ln 2 / sqrt(32).
@@ -272,8 +276,8 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
         for (int n = 1; n < 4; n++) acc = __fmaf_rn(g[n], cos64(2 * k * n), acc);
         c[k] = acc;
     }
-    // The bound of every c_k: 0.17678 = 1 / sqrt(32); 2 X is off by 104 u L1.
-    const float dx = 104.0f * u * l1 * inv;
+    // The bound of every c_k: 0.17678 = 1 / sqrt(32); 2 X is off by 480 u |window|.
+    const float dx = 481.0f * u * sqrtf(l2 * inv);
     const float err = 0.17678f * (2.2f * dx + 0.7f * (4.0f * u * (17.0f + all) + 14.0f * u * all)) + 100.0f * u;
     float s[16], top = 0.0f;
 #pragma unroll
@@ -296,7 +300,7 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
     }
     const float slack = err + 8.0f * u * hi;
     const float b0 = floorf(10.0f * fmaxf(lo - slack, 0.0f)), b1 = floorf(10.0f * (hi + slack));
-    const bool sure = b0 == b1 && dx < 0.05f && all < 1e4f && l1 > 1e-10f && l1 < 1e12f;
+    const bool sure = b0 == b1 && dx < 0.05f && all < 1e4f && l2 > 1e-20f && l2 < 1e24f;
     return sure ? b0 : -1.0f;
 }
 
