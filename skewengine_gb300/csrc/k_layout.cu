@@ -19,7 +19,9 @@ constexpr int kTile = 32;
 // prepare (skewEngine.cuh:925-951): o0 = input, o1 = transpose + flip both,
 // o2 = transpose + flip y, o3 = flip x.  32x32 tiles staged through shared
 // memory so the transposed stores stay coalesced.
-__global__ void k_prepare(const float* __restrict__ in, float* __restrict__ orient, int dimx, int dimy) {
+// xmax: the bits of the largest finite magnitude (zeroed by the caller).
+__global__ void k_prepare(const float* __restrict__ in, float* __restrict__ orient, int dimx, int dimy,
+                          unsigned* __restrict__ xmax) {
     __shared__ float tile[kTile][kTile + 1];
     const int64_t n = (int64_t)dimx * dimy;
     float* o0 = orient;
@@ -27,15 +29,20 @@ __global__ void k_prepare(const float* __restrict__ in, float* __restrict__ orie
     float* o2 = orient + 2 * n;
     float* o3 = orient + 3 * n;
     const int j0 = blockIdx.x * kTile, i0 = blockIdx.y * kTile;
+    unsigned top = 0;
     for (int ty = threadIdx.y; ty < kTile; ty += blockDim.y) {
         const int i = i0 + ty, j = j0 + threadIdx.x;
         if (i < dimy && j < dimx) {
             const float v = in[(int64_t)i * dimx + j];
             tile[ty][threadIdx.x] = v;
+            const unsigned m = __float_as_uint(v) & 0x7fffffffu;
+            top = m < 0x7f800000u ? max(top, m) : top;
             o0[(int64_t)i * dimx + j] = v;
             o3[(int64_t)i * dimx + (dimx - 1 - j)] = v;
         }
     }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (threadIdx.x == 0 && top > 0) atomicMax(xmax, top);
     __syncthreads();
     // Transposed writes: thread x walks input rows (output columns).
     for (int ty = threadIdx.y; ty < kTile; ty += blockDim.y) {
@@ -121,13 +128,29 @@ constexpr int kDeskewBand = kDeskewRows + 34;  // rows + 1 + max column drift ov
 enum { kDeskewAdd = 0, kDeskewKahan = 1, kDeskewMax = 2 };
 
 // Skewed output cell (r, c), c < dim_i, of a Radon sector read from its
-// filtered row values q instead of SO: the back-projection writes
-// 0.0f + q[r] (in binary64, then rounded) on every valid cell of row r
-// (kernelRADN.h:251-257), and zero elsewhere.  Only for sectors whose rows stay
-// within dim_i, where no two rows share a cell.
+// filtered row values q instead of SO.  The back-projection starts from 0.0f and
+// adds q[r] (in binary64, then rounded) on every valid cell of row r, in row
+// order (kernelRADN.h:251-257): a cell of row r takes q[r - 1] first where that
+// row overruns its width by at least c + 1 cells (kOver; dim_l <= 2 dim_i, so no
+// earlier row reaches it).
+__device__ __forceinline__ float row_add(float v, const cd* __restrict__ q, int r) {
+    return __double2float_rn(__dadd_rn((double)v, q[r].re));
+}
+template <bool kOver>
 __device__ __forceinline__ float row_cell(const SectorDesc& d, const int32_t* __restrict__ first,
                                           const int32_t* __restrict__ last, const cd* __restrict__ q, int r, int c) {
-    return (r < d.H && c >= first[r] && c < last[r]) ? __double2float_rn(__dadd_rn(0.0, q[r].re)) : 0.0f;
+    float v = 0.0f;
+    if (kOver && r >= 1 && r <= d.H && c + d.dim_i >= first[r - 1] && c + d.dim_i < last[r - 1])
+        v = row_add(v, q, r - 1);
+    return (r < d.H && c >= first[r] && c < last[r]) ? row_add(v, q, r) : v;
+}
+
+// The 32 columns from j0 that lie in [lo, hi), as a mask.
+__device__ __forceinline__ unsigned column_mask(int lo, int hi, int j0) {
+    lo = max(lo - j0, 0);
+    hi = min(hi - j0, kTile);
+    if (hi <= lo) return 0u;
+    return (hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);
 }
 
 // kRows: the batch's skewed outputs are Radon sectors given as per-row values
@@ -135,7 +158,8 @@ __device__ __forceinline__ float row_cell(const SectorDesc& d, const int32_t* __
 // kMasked: SO is defined only on its sectors' valid cells (rows within dim_i,
 // not zeroed first): a staged row carries the mask of the tile's columns in
 // its valid range and other cells read as zero.
-template <int kMode, bool kRows = false, bool kMasked = false>
+// kOver (with kRows): rows may overrun their width into the next one.
+template <int kMode, bool kRows = false, bool kMasked = false, bool kOver = false>
 __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(DevGeometry g, TypeLists tl, const float* __restrict__ SO,
                                                 int64_t stride, float* __restrict__ acc, float* __restrict__ comp,
                                                 int dimx, int dimy, const cd* __restrict__ Q = nullptr,
@@ -145,6 +169,9 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
     // kRows: the band's rows as (value, mask of the tile's columns inside the
     // row's valid range); a cell is its row's value inside the range, else zero.
     __shared__ float2 rqm[kRows ? kDeskewBand : 1];
+    // kOver: (mask of the columns the previous row reaches, its value alone, its
+    // value with this row's).
+    __shared__ float3 rqo[kOver ? kDeskewBand : 1];
     // Thread (tx, ty) owns rows ty*kPer .. ty*kPer+kPer-1 of the tile in column
     // j0+tx: consecutive rows share a skewed cell (row k's upper cell is row
     // k+1's lower one), so kPer+1 cells per sector serve its kPer rows.
@@ -197,11 +224,22 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
                 float v = 0.0f;
                 unsigned m = 0;
                 if (r < d.H) {
-                    v = __double2float_rn(__dadd_rn(0.0, qv[r].re));
-                    const int lo_c = max(rfirst[r] - j0, 0), hi_c = min(rlast[r] - j0, kTile);
-                    if (hi_c > lo_c) m = (hi_c >= 32 ? 0xffffffffu : (1u << hi_c) - 1u) & ~((1u << lo_c) - 1u);
+                    v = row_add(0.0f, qv, r);
+                    m = column_mask(rfirst[r], rlast[r], j0);
                 }
                 rqm[tid] = make_float2(v, __uint_as_float(m));
+                if (kOver) {
+                    float3 o = make_float3(0.0f, 0.0f, 0.0f);
+                    if (r >= 1 && r <= d.H) {
+                        const unsigned mo = column_mask(rfirst[r - 1] - dim_i, rlast[r - 1] - dim_i, j0);
+                        if (mo) {
+                            o.x = __uint_as_float(mo);
+                            o.y = row_add(0.0f, qv, r - 1);
+                            o.z = r < d.H ? row_add(o.y, qv, r) : 0.0f;
+                        }
+                    }
+                    rqo[tid] = o;
+                }
             }
             __syncthreads();
         } else if (staged) {
@@ -246,9 +284,14 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
             const int r = i0 + ib + kk + tj;
             if (kRows && staged) {
                 const float2 e = rqm[br];
-                cell[kk] = ((__float_as_uint(e.y) >> tx) & 1u) ? e.x : 0.0f;
+                const bool in = (__float_as_uint(e.y) >> tx) & 1u;
+                cell[kk] = in ? e.x : 0.0f;
+                if (kOver) {
+                    const float3 o = rqo[br];
+                    if ((__float_as_uint(o.x) >> tx) & 1u) cell[kk] = in ? o.z : o.y;
+                }
             } else if (kRows) {
-                cell[kk] = row_cell(d, rfirst, rlast, qv, r, j);
+                cell[kk] = row_cell<kOver>(d, rfirst, rlast, qv, r, j);
             } else if (kMasked && !full) {
                 const bool ok = staged ? ((bmask[br] >> tx) & 1u) != 0
                                        : (r < d.H && j >= rfirst[r] && j < rlast[r]);
@@ -620,9 +663,9 @@ inline int blocks_for(int64_t work, int threads, int cap = 65535) {
 
 }  // namespace
 
-cudaError_t launch_prepare(const float* in, float* orient, int dimx, int dimy, cudaStream_t st) {
+cudaError_t launch_prepare(const float* in, float* orient, int dimx, int dimy, unsigned* xmax, cudaStream_t st) {
     dim3 grid((dimx + kTile - 1) / kTile, (dimy + kTile - 1) / kTile);
-    k_prepare<<<grid, dim3(kTile, 8), 0, st>>>(in, orient, dimx, dimy);
+    k_prepare<<<grid, dim3(kTile, 8), 0, st>>>(in, orient, dimx, dimy, xmax);
     return cudaGetLastError();
 }
 
@@ -732,7 +775,8 @@ bool encode_skew_maps(SkewMaps* m, const float* orient, int dimx, int dimy) {
 
 cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const float* SO, int64_t stride,
                               float* acc, float* comp, int dimx, int dimy, int accum_mode, cudaStream_t st,
-                              const cd* Q, int64_t pstride, bool masked, const DeskewMaps* maps, int* status) {
+                              const cd* Q, int64_t pstride, bool masked, const DeskewMaps* maps, int* status,
+                              bool rows_over) {
     const dim3 grid = deskew_grid(dimx, dimy), block(kTile, 8);
     if (!Q && maps && maps->ok && status) {
         if (accum_mode == kAccumKahan) {
@@ -759,7 +803,14 @@ cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const f
             k_deskew<kDeskewAdd, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx, dimy);
         return cudaGetLastError();
     }
-    if (Q) {
+    if (Q && rows_over) {
+        if (accum_mode == kAccumKahan)
+            k_deskew<kDeskewKahan, true, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy,
+                                                                            Q, pstride);
+        else
+            k_deskew<kDeskewAdd, true, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx,
+                                                                          dimy, Q, pstride);
+    } else if (Q) {
         if (accum_mode == kAccumKahan)
             k_deskew<kDeskewKahan, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy, Q, pstride);
         else

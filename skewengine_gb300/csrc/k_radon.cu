@@ -9,11 +9,12 @@
 // no fused operations, so the result is bit-identical to the reference.
 //
 // Three launches per batch: row sums (one warp per row), transform (one CTA per
-// sector), back-projection (one thread per cell).  For sectors whose rows stay
-// within their width the engine skips the back-projection (its deskew reads the
-// filtered row values) and the skew (the row sums gather the skewed cells from
-// the oriented input themselves), and runs sums and transform as one fused
-// sector kernel (k_radon_sector, a thread-block cluster per sector).
+// sector), back-projection (one thread per cell).  Where no row is longer than
+// twice its width (every grid up to 2:1) the engine skips the back-projection
+// (its deskew reads the filtered row values) and the skew (the row sums gather
+// the skewed cells from the oriented input themselves).  Selectable for sectors
+// whose rows stay within their width: sums and transform as one fused sector
+// kernel (k_radon_sector, a thread-block cluster per sector).
 #include <climits>
 
 #include <cooperative_groups.h>
@@ -41,9 +42,6 @@ __device__ __forceinline__ int pow2_at_least(int h) {
 // overflow) and returns sum * 2^emin.  Rows with a non-finite value or failing
 // these conditions are added in binary64, left to right, by one lane.
 //
-// kGather: the cells are formed from the oriented input as the skew forms them
-// (skew_gather), instead of read from the skewed grid; only for sectors whose
-// rows stay within dim_i, where cell (r, j) is the skew's value at r*dim_i + j.
 constexpr int kSumWarps = 8;
 constexpr int kMaxSpread = 28;
 constexpr int kMaxExactRow = 2048;
@@ -88,18 +86,14 @@ struct ExactPart {
     }
 };
 
-template <bool kGather>
 __global__ void __launch_bounds__(kSumWarps * 32)
-    k_radon_sums(DevGeometry g, Batch b, const float* __restrict__ SI, int64_t stride, const float* __restrict__ orient,
-                 int64_t n_cells, cd* __restrict__ P, int64_t pstride) {
+    k_radon_sums(DevGeometry g, Batch b, const float* __restrict__ SI, int64_t stride, cd* __restrict__ P,
+                 int64_t pstride) {
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.y;
     const SectorDesc d = g.desc[b.angle[slot]];
     const int H2 = pow2_at_least(d.H);
     const float* in = SI + slot * stride;
-    const float* src = orient + (int64_t)d.type * n_cells;
-    const int32_t* tgt = g.target + d.col_off;
-    const float* wgt = g.weight + d.col_off;
     cd* p = P + slot * pstride;
     const int nwarps = gridDim.x * kSumWarps;
     for (int r = blockIdx.x * kSumWarps + (threadIdx.x >> 5); r < H2; r += nwarps) {
@@ -109,10 +103,9 @@ __global__ void __launch_bounds__(kSumWarps * 32)
         }
         const int f = g.first[d.row_off + r], l = g.last[d.row_off + r];
         const float* row = in + (int64_t)r * d.dim_i;
-        auto cell = [&](int j) { return kGather ? skew_gather(d, tgt, wgt, src, r, j) : row[j]; };
         ExactPart a;
 #pragma unroll 2
-        for (int j = f + lane; j < l; j += 32) a.add(cell(j));
+        for (int j = f + lane; j < l; j += 32) a.add(row[j]);
         const bool lane_bad = a.bad();
         int gmin = a.emin, gmax = a.emax;
         for (int o = 16; o > 0; o >>= 1) {
@@ -139,9 +132,231 @@ __global__ void __launch_bounds__(kSumWarps * 32)
             }
         }
         if (bad && lane == 0)
-            for (int j = f; j < l; j++) s = __dadd_rn(s, (double)cell(j));
+            for (int j = f; j < l; j++) s = __dadd_rn(s, (double)row[j]);
         if (lane == 0) p[r] = {s, 0.0};
     }
+}
+
+// Row sums formed from the oriented input, without a skewed grid (every sector
+// with dim_l <= 2 dim_i).  A lane owns a row: 32 rows per CTA, each of its four
+// warps a quarter of their columns.  All lanes are at the same column, so its
+// shift, weight and address are one broadcast, and its 32 (or 33) source cells
+// are consecutive: read from the transposed orientation (plain and mirrored
+// sectors from orientation 2, transposed ones from the plain grid), where a
+// column of the sector's own orientation is a row.  A warp per row, lanes along
+// its columns, touched up to 32 lines a load at 45 degrees, took 15 integer
+// operations a cell to add it up exactly and reduced every row over the lanes:
+// 137 us per 512 x 512 image at 180 angles, this form 69 us (bound by issue:
+// 36 instructions a cell, 13 of them the cuts).
+// A cell is the skew's, w x[r-t-1] + (1-w) x[r-t], up to the sign of a zero.
+//
+// Exact sums in float.  With |cell| <= 2^E (E from the grid's largest finite
+// magnitude) a cell is cut into multiples of q1 = 2^(E+1-B), q2 = q1 2^-B and
+// q3, B = 24 - ceil(log2 n) for n columns: each part is added without rounding,
+// its sum staying below 2^24 of its units.  q3 is at least 2^(E-53) n, so where
+// nothing is left below it every partial sum of the reference's left-to-right
+// binary64 loop is exact too: its result is the parts' sum.  Rows with a rest
+// (exponents too far apart, a non-finite cell) are summed in 64-bit integers
+// (RowPart), and where those do not fit either, left to right in binary64.
+//
+// kOver: rows may overrun their width into the next row's cells (and past the
+// last row into zeros).  kF32: float sums in blocks of kRowStep columns.
+constexpr int kRowWarps = 4;
+constexpr int kRowStep = 8;  // columns in flight
+
+// Exact integer sum of one row's cells in units of 2^(emin - 150).
+struct RowPart {
+    long long sum = 0;
+    unsigned long long mag = 0;  // of the magnitudes
+    int emin = INT_MAX, emax = 0;
+    __device__ __forceinline__ void add(float v) {
+        const unsigned u = __float_as_uint(v);
+        const int e8 = (int)((u >> 23) & 0xffu);
+        const unsigned m = (u & 0x7fffffu) | (e8 ? 0x800000u : 0u);
+        const int ee = max(e8, 1);
+        if (m && ee < emin) {
+            const int sh = emin == INT_MAX ? 0 : emin - ee;
+            sum = (long long)shl64((unsigned long long)sum, sh);
+            mag = shl64(mag, sh);
+            emin = ee;
+        }
+        emax = max(emax, e8);
+        const unsigned long long x = shl64(m, ee - emin);  // m = 0: x = 0 whatever the shift
+        mag += x;
+        sum += (u >> 31) ? -(long long)x : (long long)x;
+    }
+    // Joins another part of the row.
+    __device__ __forceinline__ void join(const RowPart& o) {
+        const int e = min(emin, o.emin);
+        const int sa = emin == INT_MAX ? 0 : emin - e, sb = o.emin == INT_MAX ? 0 : o.emin - e;
+        sum = (long long)(shl64((unsigned long long)sum, sa) + shl64((unsigned long long)o.sum, sb));
+        mag = shl64(mag, sa) + shl64(o.mag, sb);
+        emin = e;
+        emax = max(emax, o.emax);
+    }
+};
+
+// Two floats at a time (f32x2): plain IEEE additions of both halves.
+__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
+    float2 r;
+    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2,%3}; mov.b64 y, {%4,%5}; add.rn.f32x2 z, x, y; mov.b64 {%0,%1}, z; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 sub_pair(float2 a, float2 b) {
+    float2 r;
+    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2,%3}; mov.b64 y, {%4,%5}; sub.rn.f32x2 z, x, y; mov.b64 {%0,%1}, z; }"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+template <bool kF32, bool kOver>
+__global__ void __launch_bounds__(kRowWarps * 32)
+    k_radon_rows(DevGeometry g, Batch b, const float* __restrict__ orient, int64_t n_cells, int dimx, int dimy,
+                 const unsigned* __restrict__ xmax, cd* __restrict__ P, int64_t pstride) {
+    struct Column {
+        float w;
+        int t;
+        int64_t off;  // of the w term's source cell from the lane's row
+    };
+    __shared__ Column meta[kRowWarps][32];
+    __shared__ RowPart parts[kF32 ? 1 : kRowWarps][32];
+    __shared__ float sums[3][kRowWarps][32];
+    __shared__ int marks[kRowWarps][32];  // the warp's part of the row has a rest
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slot = blockIdx.y;
+    const SectorDesc& d = g.desc[b.angle[slot]];
+    const int H = d.H, H2 = pow2_at_least(H), dim_i = d.dim_i, dim_o = d.dim_o;
+    const int r = blockIdx.x * 32 + lane;
+    if (blockIdx.x * 32 >= H2) return;
+    cd* p = P + slot * pstride;
+    const int f = r < H ? g.first[d.row_off + r] : 0, l = r < H ? g.last[d.row_off + r] : 0;
+    const int lo = __reduce_min_sync(0xffffffffu, f < l ? f : INT_MAX), hi = __reduce_max_sync(0xffffffffu, f < l ? l : 0);
+    if (hi == 0) {  // no valid cell in these rows
+        if (warp == 0 && r < H2) p[r] = {0.0, 0.0};
+        return;
+    }
+    // Cell (i, c) of the sector's orientation is base[c * cs + i * is].
+    const bool tr = d.type == 1 || d.type == 2;
+    const float* base = orient + (tr ? 0 : 2 * n_cells);
+    int64_t cs = tr ? -dimx : dimy;
+    int is = -1;
+    if (d.type == 0) base += dimy - 1;
+    if (d.type == 3) base += n_cells - 1, cs = -dimy;
+    if (d.type == 1) base += n_cells - 1;
+    if (d.type == 2) base += n_cells - dimx, is = 1;
+    const float* mine = base + (int64_t)r * is;
+    const unsigned width = (unsigned)max(l - f, 0);
+    auto column = [&](int j) {
+        const int over = kOver && j >= dim_i ? 1 : 0, c = j - (over ? dim_i : 0);
+        Column m;
+        const bool in = c < dim_i;
+        m.w = in ? g.weight[d.col_off + c] : 0.0f;
+        m.t = (in ? g.target[d.col_off + c] : 0) - over;
+        m.off = c * cs - (int64_t)(m.t + 1) * is;
+        return m;
+    };
+    // Cell j of the lane's row (0 outside its valid range).
+    auto cell = [&](int j, const Column& m) {
+        bool ok = (unsigned)(j - f) < width;
+        if (kOver) ok = ok && (j < dim_i || r + 1 < H);
+        const unsigned i0 = (unsigned)(r - m.t - 1);
+        const float* q = mine + m.off;
+        const float a = ok && i0 < (unsigned)dim_o ? q[0] : 0.0f;
+        const float e = ok && i0 + 1u < (unsigned)dim_o ? q[is] : 0.0f;
+        return __fadd_rn(__fmul_rn(m.w, a), __fmul_rn(__fsub_rn(1.0f, m.w), e));
+    };
+    const int each = ((hi - lo + kRowWarps - 1) / kRowWarps + kRowStep - 1) / kRowStep * kRowStep;
+    const int j0 = lo + warp * each, j1 = min(j0 + each, hi);
+    // add(v): kRowStep cells of consecutive columns.
+    auto walk = [&](auto add) {
+        for (int jb = j0; jb < j1; jb += 32) {
+            __syncwarp();
+            meta[warp][lane] = column(jb + lane);
+            __syncwarp();
+            const int n = min(32, j1 - jb);
+            for (int k = 0; k < n; k += kRowStep) {
+                float v[kRowStep];
+#pragma unroll
+                for (int q = 0; q < kRowStep; q++) v[q] = cell(jb + k + q, meta[warp][k + q]);
+                add(v);
+            }
+        }
+    };
+    if (kF32) {
+        float acc = 0.0f;
+        walk([&](const float* v) { acc += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])); });
+        sums[0][warp][lane] = acc;
+        __syncthreads();
+        if (warp != 0 || r >= H2) return;
+        const float s = (sums[0][0][lane] + sums[0][1][lane]) + (sums[0][2][lane] + sums[0][3][lane]);
+        p[r] = {(double)s, 0.0};
+        return;
+    }
+    // Exponents of the cuts; 1.5 * 2^23 units of q added and taken away leave the
+    // nearest multiple of q.
+    const int ln = 32 - __clz(hi - lo - 1);  // n <= 2^ln
+    const int E = (int)(xmax[0] >> 23) - 127 + 1, B = 24 - ln;
+    const int e1 = E + 1 - B, e2 = E + 1 - 2 * B, e3 = max(E + 1 - 3 * B, E - 53 + ln);
+    bool rest = hi - lo > kMaxExactRow || E < -70 || E > 100;
+    if (!rest) {
+        const float c1 = __uint_as_float((unsigned)(e1 + 23 + 127) << 23 | 0x400000u);
+        const float c2 = __uint_as_float((unsigned)(e2 + 23 + 127) << 23 | 0x400000u);
+        const float c3 = __uint_as_float((unsigned)(e3 + 23 + 127) << 23 | 0x400000u);
+        const float2 C1 = make_float2(c1, c1), C2 = make_float2(c2, c2), C3 = make_float2(c3, c3);
+        float2 s1 = make_float2(0.0f, 0.0f), s2 = s1, s3 = s1, left = s1;
+        walk([&](const float* v) {
+#pragma unroll
+            for (int q = 0; q < kRowStep; q += 2) {
+                const float2 x = make_float2(v[q], v[q + 1]);
+                const float2 h1 = sub_pair(add_pair(x, C1), C1), x1 = sub_pair(x, h1);
+                const float2 h2 = sub_pair(add_pair(x1, C2), C2), x2 = sub_pair(x1, h2);
+                const float2 h3 = sub_pair(add_pair(x2, C3), C3), x3 = sub_pair(x2, h3);
+                s1 = add_pair(s1, h1);
+                s2 = add_pair(s2, h2);
+                s3 = add_pair(s3, h3);
+                left.x += fabsf(x3.x);  // not zero, or NaN: something is left
+                left.y += fabsf(x3.y);
+            }
+        });
+        rest = !(left.x + left.y == 0.0f);
+        sums[0][warp][lane] = s1.x + s1.y;
+        sums[1][warp][lane] = s2.x + s2.y;
+        sums[2][warp][lane] = s3.x + s3.y;
+    }
+    marks[warp][lane] = rest;
+    const bool again = __syncthreads_or(rest);
+    double s = 0.0;
+    if (warp == 0 && !(marks[0][lane] | marks[1][lane] | marks[2][lane] | marks[3][lane])) {
+        float t[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) t[k] = (sums[k][0][lane] + sums[k][1][lane]) + (sums[k][2][lane] + sums[k][3][lane]);
+        s = __dadd_rn(__dadd_rn((double)t[0], (double)t[1]), (double)t[2]);
+    }
+    if (again) {
+        // All rows of the CTA are summed again, the marked ones take the result.
+        RowPart part;
+        walk([&](const float* v) {
+#pragma unroll
+            for (int q = 0; q < kRowStep; q++) part.add(v[q]);
+        });
+        parts[warp][lane] = part;
+        __syncthreads();
+        if (warp == 0 && (marks[0][lane] | marks[1][lane] | marks[2][lane] | marks[3][lane])) {
+#pragma unroll
+            for (int k = 1; k < kRowWarps; k++) part.join(parts[k][lane]);
+            const bool bad = l - f > kMaxExactRow || part.emax == 0xff ||
+                             (part.emin != INT_MAX && (part.emax - part.emin > kMaxSpread || part.mag >= (1ull << 53)));
+            s = 0.0;
+            if (!bad && part.emin != INT_MAX)
+                s = __dmul_rn(__ll2double_rn(part.sum), __longlong_as_double((long long)(part.emin - 150 + 1023) << 52));
+            if (bad)
+                for (int j = f; j < l; j++) s = __dadd_rn(s, (double)cell(j, column(j)));
+        }
+    }
+    if (warp == 0 && r < H2) p[r] = {s, 0.0};
 }
 
 // In-place reference DIF FFT of x[0..n) by one CTA, then bit reversal.
@@ -332,18 +547,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kTransfor
 // deskew or back-projection.  Values differ from the reference's binary64 in
 // their low bits (the sums' order and float rounding); the relative error of
 // the output is measured and stated (tests/test_gpu_parity.py).
-template <bool kGather>
 __global__ void __launch_bounds__(kSumWarps * 32)
-    k_radon_sums_f32(DevGeometry g, Batch b, const float* __restrict__ SI, int64_t stride,
-                     const float* __restrict__ orient, int64_t n_cells, cd* __restrict__ P, int64_t pstride) {
+    k_radon_sums_f32(DevGeometry g, Batch b, const float* __restrict__ SI, int64_t stride, cd* __restrict__ P,
+                     int64_t pstride) {
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.y;
     const SectorDesc d = g.desc[b.angle[slot]];
     const int H2 = pow2_at_least(d.H);
     const float* in = SI + slot * stride;
-    const float* src = orient + (int64_t)d.type * n_cells;
-    const int32_t* tgt = g.target + d.col_off;
-    const float* wgt = g.weight + d.col_off;
     cd* p = P + slot * pstride;
     const int nwarps = gridDim.x * kSumWarps;
     for (int r = blockIdx.x * kSumWarps + (threadIdx.x >> 5); r < H2; r += nwarps) {
@@ -354,7 +565,7 @@ __global__ void __launch_bounds__(kSumWarps * 32)
         const int f = g.first[d.row_off + r], l = g.last[d.row_off + r];
         const float* row = in + (int64_t)r * d.dim_i;
         float acc = 0.0f;
-        for (int j = f + lane; j < l; j += 32) acc += kGather ? skew_gather(d, tgt, wgt, src, r, j) : row[j];
+        for (int j = f + lane; j < l; j += 32) acc += row[j];
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (lane == 0) p[r] = {(double)acc, 0.0};
     }
@@ -445,9 +656,9 @@ __global__ void k_radon_backproject(DevGeometry g, Batch b, const cd* __restrict
 // transform as two launches, measured faster (radon_select).
 int g_radon_path = 1;
 
-int radon_launches(bool rows_only, int max_H2, bool f32) {
+int radon_launches(bool rows_only, int max_H2, bool f32, bool in_width) {
     if (f32 && max_H2 <= kSmemH2) return rows_only ? 2 : 3;
-    return rows_only ? (max_H2 <= kSmemH2 && g_radon_path == 0 ? 1 : 2) : 3;
+    return rows_only ? (in_width && max_H2 <= kSmemH2 && g_radon_path == 0 ? 1 : 2) : 3;
 }
 
 int radon_select(int path) {
@@ -459,15 +670,17 @@ int radon_select(int path) {
 cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
                          int64_t len, double* P, int64_t pstride, const double* twiddles, const int64_t* tw_off,
                          int max_H2, cudaStream_t st, bool backproject, const float* orient, int64_t n_cells,
-                         bool f32) {
+                         int dimx, int dimy, const unsigned* xmax, bool f32, bool in_width) {
     if (orient && backproject) return cudaErrorInvalidValue;  // the gathered cells are not kept for SO
     cd* Pc = reinterpret_cast<cd*>(P);
     if (f32 && max_H2 <= kSmemH2) {
-        dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count);
-        if (orient)
-            k_radon_sums_f32<true><<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, orient, n_cells, Pc, pstride);
+        dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count), gr((max_H2 + 31) / 32, b.count);
+        if (orient && in_width)
+            k_radon_rows<true, false><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
+        else if (orient)
+            k_radon_rows<true, true><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
         else
-            k_radon_sums_f32<false><<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, orient, n_cells, Pc, pstride);
+            k_radon_sums_f32<<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, Pc, pstride);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         const int smem = max_H2 * (int)sizeof(float2);
@@ -483,7 +696,7 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
         k_radon_backproject<<<dim3((unsigned)blocks, b.count), 256, 0, st>>>(g, b, Pc, pstride, SO, stride, len);
         return cudaGetLastError();
     }
-    if (orient && max_H2 <= kSmemH2 && g_radon_path == 0) {  // one fused launch: a cluster per sector
+    if (orient && in_width && max_H2 <= kSmemH2 && g_radon_path == 0) {  // one fused launch: a cluster per sector
         const int smem = max_H2 * (int)sizeof(cd);
         cudaError_t e = cudaSuccess;
         if (smem > 48 * 1024) e = cudaFuncSetAttribute(k_radon_sector, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -492,11 +705,13 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
                                                                                    twiddles, tw_off);
         return cudaGetLastError();
     }
-    dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count);
-    if (orient)
-        k_radon_sums<true><<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, orient, n_cells, Pc, pstride);
+    dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count), gr((max_H2 + 31) / 32, b.count);
+    if (orient && in_width)
+        k_radon_rows<false, false><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
+    else if (orient)
+        k_radon_rows<false, true><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
     else
-        k_radon_sums<false><<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, orient, n_cells, Pc, pstride);
+        k_radon_sums<<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, Pc, pstride);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int smem = max_H2 <= kSmemH2 ? max_H2 * (int)sizeof(cd) : 0;

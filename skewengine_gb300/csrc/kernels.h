@@ -23,8 +23,9 @@ enum AccumMode { kAccumReference = 0, kAccumKahan = 1 };
 
 // --- layout (k_layout.cu) -------------------------------------------------
 // The four orientations of a dimy x dimx input (skewEngine.cuh:925-951):
-// orient[t*N ...], t = 0..3.
-cudaError_t launch_prepare(const float* in, float* orient, int dimx, int dimy, cudaStream_t st);
+// orient[t*N ...], t = 0..3.  *xmax (zeroed before): bits of the largest finite
+// magnitude of the input.
+cudaError_t launch_prepare(const float* in, float* orient, int dimx, int dimy, unsigned* xmax, cudaStream_t st);
 
 // Skewed input of every sector of the batch into slot s of SI (stride floats per
 // slot, `len` = 2N + dim_l cells each, zero past H*dim_i).
@@ -60,9 +61,10 @@ cudaError_t launch_identity(const DevGeometry& g, const Batch& b, const float* S
 
 // Deskew + accumulate (skewEngine.cuh:772-792) of every slot of the batch into
 // the per-type accumulators acc[t*N ...] (and comp[] in Kahan mode).
-// With Q set, the slots are Radon sectors whose rows stay within dim_i, read
-// from their filtered row values (Q: pstride complex doubles per slot) instead
-// of SO: what the back-projection would write, without writing it.
+// With Q set, the slots are Radon sectors with dim_l <= 2 dim_i, read from their
+// filtered row values (Q: pstride complex doubles per slot) instead of SO: what
+// the back-projection would write, without writing it.  rows_over: some of their
+// rows overrun dim_i into the next row.
 // Tensor maps of the skewed-output buffer for the TMA-staged deskew: 3-D
 // (columns, rows, slots) float32 views with rows of dimx (x) and dimy (y) cells.
 struct DeskewMaps {
@@ -80,7 +82,8 @@ bool encode_band_maps(DeskewMaps* m, const float* SO, int64_t stride, int slots,
 cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const float* SO,
                               int64_t stride, float* acc, float* comp, int dimx, int dimy,
                               int accum_mode, cudaStream_t st, const cd* Q = nullptr, int64_t pstride = 0,
-                              bool masked = false, const DeskewMaps* maps = nullptr, int* status = nullptr);
+                              bool masked = false, const DeskewMaps* maps = nullptr, int* status = nullptr,
+                              bool rows_over = false);
 // Max mode with angle encoding (skewEngine.cuh:774-785).
 cudaError_t launch_deskew_max(const DevGeometry& g, const TypeLists& tl, const float* SO,
                               int64_t stride, float* acc, int dimx, int dimy, cudaStream_t st);
@@ -209,17 +212,19 @@ int sdem_chunk();
 // Radon / filtered back-projection (k_radon.cu).  P: per-slot complex scratch
 // of pstride complex doubles; re: per-slot max_H doubles.
 // backproject = false leaves SO untouched (the deskew reads P instead).  With
-// orient set (only with backproject = false, for sectors whose rows stay within
-// dim_i) the row sums gather the skewed cells from the oriented input (n_cells
-// per orientation) and SI is not read: the batch needs no skew launch.
+// orient set (only with backproject = false, for sectors with dim_l <= 2 dim_i)
+// the row sums gather the skewed cells from the oriented input (n_cells per
+// orientation) and SI is not read: the batch needs no skew launch.  xmax: as
+// launch_prepare leaves it.  in_width: every sector's rows stay within dim_i.
 cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, float* SO,
                          int64_t stride, int64_t len, double* P, int64_t pstride, const double* twiddles,
                          const int64_t* tw_off, int max_H2, cudaStream_t st, bool backproject = true,
-                         const float* orient = nullptr, int64_t n_cells = 0, bool f32 = false);
+                         const float* orient = nullptr, int64_t n_cells = 0, int dimx = 0, int dimy = 0,
+                         const unsigned* xmax = nullptr, bool f32 = false, bool in_width = true);
 
 // Kernel launches launch_radon makes (rows_only: gathered sums, no back-projection;
 // f32: the float32 mode).
-int radon_launches(bool rows_only, int max_H2, bool f32 = false);
+int radon_launches(bool rows_only, int max_H2, bool f32 = false, bool in_width = true);
 // Radon path for later launches: 0 = fused sector kernel where it applies, 1 =
 // separate sums and transform; -1 for another value.
 int radon_select(int path);
