@@ -601,7 +601,7 @@ int run_deskew(ske_engine e, const Batch& b, int is_max, int accum, bool rows_fr
     LaunchScope ls(e, "deskew", 1);
     if (is_max) return ls.done(launch_deskew_max(e->dg, tl, e->d_SO, e->stride, e->d_acc, e->dimx, e->dimy, e->stream));
     return ls.done(launch_deskew_add(e->dg, tl, e->d_SO, e->stride, e->d_acc, e->d_comp, e->dimx, e->dimy, accum,
-                                     e->stream, rows_from_p ? reinterpret_cast<const cd*>(e->d_P) : nullptr,
+                                     e->stream, rows_from_p ? reinterpret_cast<const RowValue*>(e->d_P) : nullptr,
                                      e->pstride, so_masked, &e->maps, e->d_status, rows_over));
 }
 

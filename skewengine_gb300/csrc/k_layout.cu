@@ -127,24 +127,6 @@ constexpr int kDeskewRows = 64;
 constexpr int kDeskewBand = kDeskewRows + 34;  // rows + 1 + max column drift over 32 columns (+1)
 enum { kDeskewAdd = 0, kDeskewKahan = 1, kDeskewMax = 2 };
 
-// Skewed output cell (r, c), c < dim_i, of a Radon sector read from its
-// filtered row values q instead of SO.  The back-projection starts from 0.0f and
-// adds q[r] (in binary64, then rounded) on every valid cell of row r, in row
-// order (kernelRADN.h:251-257): a cell of row r takes q[r - 1] first where that
-// row overruns its width by at least c + 1 cells (kOver; dim_l <= 2 dim_i, so no
-// earlier row reaches it).
-__device__ __forceinline__ float row_add(float v, const cd* __restrict__ q, int r) {
-    return __double2float_rn(__dadd_rn((double)v, q[r].re));
-}
-template <bool kOver>
-__device__ __forceinline__ float row_cell(const SectorDesc& d, const int32_t* __restrict__ first,
-                                          const int32_t* __restrict__ last, const cd* __restrict__ q, int r, int c) {
-    float v = 0.0f;
-    if (kOver && r >= 1 && r <= d.H && c + d.dim_i >= first[r - 1] && c + d.dim_i < last[r - 1])
-        v = row_add(v, q, r - 1);
-    return (r < d.H && c >= first[r] && c < last[r]) ? row_add(v, q, r) : v;
-}
-
 // The 32 columns from j0 that lie in [lo, hi), as a mask.
 __device__ __forceinline__ unsigned column_mask(int lo, int hi, int j0) {
     lo = max(lo - j0, 0);
@@ -153,25 +135,15 @@ __device__ __forceinline__ unsigned column_mask(int lo, int hi, int j0) {
     return (hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u);
 }
 
-// kRows: the batch's skewed outputs are Radon sectors given as per-row values
-// (Q: pstride complex doubles per slot, real part) rather than SO.
 // kMasked: SO is defined only on its sectors' valid cells (rows within dim_i,
 // not zeroed first): a staged row carries the mask of the tile's columns in
 // its valid range and other cells read as zero.
-// kOver (with kRows): rows may overrun their width into the next one.
-template <int kMode, bool kRows = false, bool kMasked = false, bool kOver = false>
+template <int kMode, bool kMasked = false>
 __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(DevGeometry g, TypeLists tl, const float* __restrict__ SO,
                                                 int64_t stride, float* __restrict__ acc, float* __restrict__ comp,
-                                                int dimx, int dimy, const cd* __restrict__ Q = nullptr,
-                                                int64_t pstride = 0) {
-    __shared__ float band[kRows ? 1 : kDeskewBand][kTile];
+                                                int dimx, int dimy) {
+    __shared__ float band[kDeskewBand][kTile];
     __shared__ unsigned bmask[kMasked ? kDeskewBand : 1];
-    // kRows: the band's rows as (value, mask of the tile's columns inside the
-    // row's valid range); a cell is its row's value inside the range, else zero.
-    __shared__ float2 rqm[kRows ? kDeskewBand : 1];
-    // kOver: (mask of the columns the previous row reaches, its value alone, its
-    // value with this row's).
-    __shared__ float3 rqo[kOver ? kDeskewBand : 1];
     // Thread (tx, ty) owns rows ty*kPer .. ty*kPer+kPer-1 of the tile in column
     // j0+tx: consecutive rows share a skewed cell (row k's upper cell is row
     // k+1's lower one), so kPer+1 cells per sector serve its kPer rows.
@@ -209,40 +181,13 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
         const int r0 = i0 + tmin;
         const int nrows = (i_end - i0) + 1 + (tmax - tmin);
         const float* so = SO + tl.slot[t][q] * stride;
-        const cd* qv = kRows ? Q + tl.slot[t][q] * pstride : nullptr;
         const int32_t* rfirst = g.first + d.row_off;
         const int32_t* rlast = g.last + d.row_off;
         // Steep sectors of elongated grids (tan > 1) can drift more than the band
         // holds; those tiles read the skewed cells directly.
         const bool staged = nrows <= kDeskewBand;
         bool full = false;  // kMasked: every staged cell of the tile is valid
-        if (staged && kRows) {
-            __syncthreads();  // previous sector's rows fully consumed
-            const int tid = ty * kTile + tx;
-            if (tid < nrows) {
-                const int r = r0 + tid;
-                float v = 0.0f;
-                unsigned m = 0;
-                if (r < d.H) {
-                    v = row_add(0.0f, qv, r);
-                    m = column_mask(rfirst[r], rlast[r], j0);
-                }
-                rqm[tid] = make_float2(v, __uint_as_float(m));
-                if (kOver) {
-                    float3 o = make_float3(0.0f, 0.0f, 0.0f);
-                    if (r >= 1 && r <= d.H) {
-                        const unsigned mo = column_mask(rfirst[r - 1] - dim_i, rlast[r - 1] - dim_i, j0);
-                        if (mo) {
-                            o.x = __uint_as_float(mo);
-                            o.y = row_add(0.0f, qv, r - 1);
-                            o.z = r < d.H ? row_add(o.y, qv, r) : 0.0f;
-                        }
-                    }
-                    rqo[tid] = o;
-                }
-            }
-            __syncthreads();
-        } else if (staged) {
+        if (staged) {
             // All of this thread's band loads are issued before any store.
             constexpr int kLoads = (kDeskewBand + 7) / 8;
             float v[kLoads];
@@ -255,10 +200,7 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
             const int tid = ty * kTile + tx;
             if (kMasked && tid < nrows) {
                 const int r = r0 + tid;
-                if (r < d.H) {
-                    const int lo_c = max(rfirst[r] - j0, 0), hi_c = min(rlast[r] - j0, kTile);
-                    if (hi_c > lo_c) m = (hi_c >= 32 ? 0xffffffffu : (1u << hi_c) - 1u) & ~((1u << lo_c) - 1u);
-                }
+                if (r < d.H) m = column_mask(rfirst[r], rlast[r], j0);
             }
             __syncthreads();  // previous sector's band fully consumed
 #pragma unroll
@@ -282,17 +224,7 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
             if (kk > nv) continue;
             const int br = ib + kk + off;
             const int r = i0 + ib + kk + tj;
-            if (kRows && staged) {
-                const float2 e = rqm[br];
-                const bool in = (__float_as_uint(e.y) >> tx) & 1u;
-                cell[kk] = in ? e.x : 0.0f;
-                if (kOver) {
-                    const float3 o = rqo[br];
-                    if ((__float_as_uint(o.x) >> tx) & 1u) cell[kk] = in ? o.z : o.y;
-                }
-            } else if (kRows) {
-                cell[kk] = row_cell<kOver>(d, rfirst, rlast, qv, r, j);
-            } else if (kMasked && !full) {
+            if (kMasked && !full) {
                 const bool ok = staged ? ((bmask[br] >> tx) & 1u) != 0
                                        : (r < d.H && j >= rfirst[r] && j < rlast[r]);
                 cell[kk] = ok ? (staged ? band[br][tx] : so[(int64_t)r * dim_i + j]) : 0.0f;
@@ -330,6 +262,165 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
         if (i >= i_end) continue;
         A[(int64_t)i * dim_i + j] = s[k];
         if (kMode == kDeskewKahan) comp[t * n + (int64_t)i * dim_i + j] = c[k];
+    }
+}
+
+// ---- Radon deskew -----------------------------------------------------------
+// The additive deskew of Radon sectors whose back-projection is not formed: a
+// skewed output cell (r, c), c < dim_i, is read from the filtered row values Q
+// (RowValue, pstride per slot).  The back-projection starts from 0.0f and adds
+// q[r] (in binary64, then rounded) on every valid cell of row r, in row order
+// (kernelRADN.h:251-257): a cell of row r takes q[r - 1] first where that row
+// overruns its width by at least c + 1 cells (kOver; dim_l <= 2 dim_i, so no
+// earlier row reaches it).
+//
+// A tile as in k_deskew.  Each of the eight warps stages one sector of the next
+// eight - its band's rows as (value, mask of the tile's columns in the row's
+// range) and the columns' shifts and weights - while the CTA accumulates the
+// eight before: one barrier for eight sectors, and no global load in the loop
+// over them.  With a sector staged at a time, two barriers and dependent loads
+// of the column tables each, the kernel waited: 100 us per 512 x 512 image at
+// 180 angles, so 39 us.
+constexpr int kRowSectors = 8;
+
+template <bool kOver>
+struct RowStage {
+    float2 row[kRowSectors][kDeskewBand];  // (value, mask bits)
+    // kOver: (mask of the columns the previous row reaches, its value alone, its
+    // value with this row's).
+    float3 over[kOver ? kRowSectors : 1][kOver ? kDeskewBand : 1];
+    float2 col[kRowSectors][kTile];        // (weight, row of the band its cells start at, or -1)
+};
+
+__device__ __forceinline__ float row_add(float v, double q) { return __double2float_rn(__dadd_rn((double)v, q)); }
+
+// Cell (r, c) where the band does not hold the tile's rows.
+template <bool kOver>
+__device__ __forceinline__ float row_cell(const SectorDesc& d, const int32_t* __restrict__ first,
+                                          const int32_t* __restrict__ last, const RowValue* __restrict__ q, int r,
+                                          int c) {
+    float v = 0.0f;
+    if (kOver && r >= 1 && r <= d.H && c + d.dim_i >= first[r - 1] && c + d.dim_i < last[r - 1]) v = q[r - 1].alone;
+    return (r < d.H && c >= first[r] && c < last[r]) ? row_add(v, q[r].q) : v;
+}
+
+template <bool kKahan, bool kOver>
+__global__ void __launch_bounds__(256, kKahan ? 2 : 4)
+    k_deskew_rows(DevGeometry g, TypeLists tl, const RowValue* __restrict__ Q, int64_t pstride, float* __restrict__ acc,
+                  float* __restrict__ comp, int dimx, int dimy) {
+    __shared__ RowStage<kOver> stage[2];
+    constexpr int kPer = kDeskewRows / 8;
+    const int t = blockIdx.z;
+    const int cnt = tl.count[t];
+    if (cnt == 0) return;
+    const int64_t n = (int64_t)dimx * dimy;
+    const int dim_i = (t == 1 || t == 2) ? dimy : dimx;
+    const int dim_o = (t == 1 || t == 2) ? dimx : dimy;
+    const int j0 = blockIdx.x * kTile, i0 = blockIdx.y * kDeskewRows;
+    if (j0 >= dim_i || i0 >= dim_o) return;
+    const int tx = threadIdx.x, ty = threadIdx.y, j = j0 + tx;
+    const bool col_ok = j < dim_i;
+    const int jlast = min(j0 + kTile, dim_i) - 1;
+    const int i_end = min(i0 + kDeskewRows, dim_o);
+    const int ib = ty * kPer;
+    const int nv = col_ok ? min(kPer, i_end - i0 - ib) : 0;  // this thread's rows inside the grid
+    float* A = acc + t * n;
+    float s[kPer], c[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        const int64_t at = (int64_t)(i0 + ib + k) * dim_i + j;
+        s[k] = k < nv ? A[at] : 0.0f;
+        c[k] = kKahan && k < nv ? comp[t * n + at] : 0.0f;
+    }
+    // Warp ty stages sector q0 + ty: lanes over the band's rows, then its columns.
+    auto fill = [&](RowStage<kOver>& st, int q0) {
+        const int q = q0 + ty;
+        if (q >= cnt) return;
+        const SectorDesc& d = g.desc[tl.angle[t][q]];
+        const int32_t* tg = g.target + d.col_off;
+        const int tmin = tg[j0], nrows = (i_end - i0) + 1 + (tg[jlast] - tmin);
+        const bool staged = nrows <= kDeskewBand;
+        const int jc = min(j, jlast);
+        st.col[ty][tx] = make_float2(g.weight[d.col_off + jc], __int_as_float(staged ? tg[jc] - tmin : -1));
+        if (!staged) return;
+        const int r0 = i0 + tmin;
+        const int32_t* rfirst = g.first + d.row_off;
+        const int32_t* rlast = g.last + d.row_off;
+        const RowValue* qv = Q + tl.slot[t][q] * pstride;
+        for (int k = tx; k < nrows; k += 32) {
+            const int r = r0 + k;
+            float2 e = make_float2(0.0f, 0.0f);
+            if (r < d.H) e = make_float2(qv[r].alone, __uint_as_float(column_mask(rfirst[r], rlast[r], j0)));
+            st.row[ty][k] = e;
+            if (kOver) {
+                float3 o = make_float3(0.0f, 0.0f, 0.0f);
+                if (r >= 1 && r <= d.H) {
+                    const unsigned mo = column_mask(rfirst[r - 1] - dim_i, rlast[r - 1] - dim_i, j0);
+                    if (mo) {
+                        const float before = qv[r - 1].alone;
+                        o = make_float3(__uint_as_float(mo), before, r < d.H ? row_add(before, qv[r].q) : 0.0f);
+                    }
+                }
+                st.over[ty][k] = o;
+            }
+        }
+    };
+    fill(stage[0], 0);
+    __syncthreads();
+    for (int q0 = 0, buf = 0; q0 < cnt; q0 += kRowSectors, buf ^= 1) {
+        fill(stage[buf ^ 1], q0 + kRowSectors);
+        const RowStage<kOver>& st = stage[buf];
+        const int m = min(kRowSectors, cnt - q0);
+        for (int u = 0; u < m && nv > 0; u++) {
+            const float2 col = st.col[u][tx];
+            const float w = col.x, w1 = __fsub_rn(1.0f, w);
+            const int off = __float_as_int(col.y);
+            // Cells of the skewed rows this thread's accumulator rows need.
+            float cell[kPer + 1];
+            if (off >= 0) {
+                const float2* row = st.row[u] + ib + off;
+#pragma unroll
+                for (int kk = 0; kk <= kPer; kk++) {
+                    cell[kk] = 0.0f;
+                    if (kk > nv) continue;
+                    const float2 e = row[kk];
+                    const bool in = (__float_as_uint(e.y) >> tx) & 1u;
+                    cell[kk] = in ? e.x : 0.0f;
+                    if (kOver) {
+                        const float3 o = st.over[u][ib + off + kk];
+                        if ((__float_as_uint(o.x) >> tx) & 1u) cell[kk] = in ? o.z : o.y;
+                    }
+                }
+            } else {
+                const SectorDesc& d = g.desc[tl.angle[t][q0 + u]];
+                const int tj = g.target[d.col_off + j];
+#pragma unroll
+                for (int kk = 0; kk <= kPer; kk++)
+                    cell[kk] = kk <= nv ? row_cell<kOver>(d, g.first + d.row_off, g.last + d.row_off,
+                                                          Q + tl.slot[t][q0 + u] * pstride, i0 + ib + kk + tj, j)
+                                        : 0.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < kPer; k++) {
+                const float v = __fadd_rn(__fmul_rn(w1, cell[k]), __fmul_rn(w, cell[k + 1]));
+                if (kKahan) {
+                    const float y = __fsub_rn(v, c[k]);
+                    const float ts = __fadd_rn(s[k], y);
+                    c[k] = __fsub_rn(__fsub_rn(ts, s[k]), y);
+                    s[k] = ts;
+                } else {
+                    s[k] = __fadd_rn(s[k], v);
+                }
+            }
+        }
+        __syncthreads();  // the next eight are staged, these are free
+    }
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+        if (k >= nv) continue;
+        const int64_t at = (int64_t)(i0 + ib + k) * dim_i + j;
+        A[at] = s[k];
+        if (kKahan) comp[t * n + at] = c[k];
     }
 }
 
@@ -466,10 +557,7 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4)
             unsigned m = 0;
             if (kMasked && tid < nrows) {
                 const int r = r0 + tid;
-                if (r < d.H) {
-                    const int lo_c = max(rfirst[r] - j0, 0), hi_c = min(rlast[r] - j0, kTile);
-                    if (hi_c > lo_c) m = (hi_c >= 32 ? 0xffffffffu : (1u << hi_c) - 1u) & ~((1u << lo_c) - 1u);
-                }
+                if (r < d.H) m = column_mask(rfirst[r], rlast[r], j0);
                 bmask[tid] = m;
             }
             if (mbar_wait(&bar[buf], uses[buf] & 1)) uses[buf]++;
@@ -775,7 +863,7 @@ bool encode_skew_maps(SkewMaps* m, const float* orient, int dimx, int dimy) {
 
 cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const float* SO, int64_t stride,
                               float* acc, float* comp, int dimx, int dimy, int accum_mode, cudaStream_t st,
-                              const cd* Q, int64_t pstride, bool masked, const DeskewMaps* maps, int* status,
+                              const RowValue* Q, int64_t pstride, bool masked, const DeskewMaps* maps, int* status,
                               bool rows_over) {
     const dim3 grid = deskew_grid(dimx, dimy), block(kTile, 8);
     if (!Q && maps && maps->ok && status) {
@@ -798,24 +886,16 @@ cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const f
     }
     if (masked && !Q) {
         if (accum_mode == kAccumKahan)
-            k_deskew<kDeskewKahan, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy);
+            k_deskew<kDeskewKahan, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy);
         else
-            k_deskew<kDeskewAdd, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx, dimy);
+            k_deskew<kDeskewAdd, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx, dimy);
         return cudaGetLastError();
     }
-    if (Q && rows_over) {
-        if (accum_mode == kAccumKahan)
-            k_deskew<kDeskewKahan, true, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy,
-                                                                            Q, pstride);
-        else
-            k_deskew<kDeskewAdd, true, false, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx,
-                                                                          dimy, Q, pstride);
-    } else if (Q) {
-        if (accum_mode == kAccumKahan)
-            k_deskew<kDeskewKahan, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy, Q, pstride);
-        else
-            k_deskew<kDeskewAdd, true><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx, dimy, Q,
-                                                              pstride);
+    if (Q) {
+        const bool kahan = accum_mode == kAccumKahan;
+        auto kern = rows_over ? (kahan ? k_deskew_rows<true, true> : k_deskew_rows<false, true>)
+                              : (kahan ? k_deskew_rows<true, false> : k_deskew_rows<false, false>);
+        kern<<<grid, block, 0, st>>>(g, tl, Q, pstride, acc, kahan ? comp : nullptr, dimx, dimy);
     } else if (accum_mode == kAccumKahan) {
         k_deskew<kDeskewKahan><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy);
     } else {

@@ -417,6 +417,11 @@ __device__ void ramp_filter(cd* x, int H, int H2) {
     __syncthreads();
 }
 
+// Filtered row value i of a sector, as the deskew reads it.
+__device__ __forceinline__ void store_row(cd* p, int i, double q) {
+    reinterpret_cast<RowValue*>(p)[i] = RowValue{q, __double2float_rn(__dadd_rn(0.0, q))};
+}
+
 // One CTA per sector.  Sectors with H2 <= kSmemH2 transform a copy of their
 // row sums in shared memory (smem > 0), larger ones work in place in P.  The
 // final division by H2 (kernelRADN.h:255) is a multiplication by the exact
@@ -452,7 +457,7 @@ __global__ void __launch_bounds__(kTransformThreads)
     }
     // conj, then divide by H2: only the real part is used (kernelRADN.h:255).
     const double inv = 1.0 / (double)H2;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) p[i].re = __dmul_rn(x[i].re, inv);
+    for (int i = threadIdx.x; i < H; i += blockDim.x) store_row(p, i, __dmul_rn(x[i].re, inv));
 }
 
 // The whole Radon operator of a sector whose rows stay within its width, in
@@ -536,7 +541,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kTransfor
     }
     cd* p = P + slot * pstride;
     const double inv = 1.0 / (double)H2;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) p[i].re = __dmul_rn(xs[i].re, inv);
+    for (int i = threadIdx.x; i < H; i += blockDim.x) store_row(p, i, __dmul_rn(xs[i].re, inv));
 }
 
 // ---- float32 mode (SKE_FLAG_RADON_F32) -------------------------------------
@@ -624,7 +629,7 @@ __global__ void __launch_bounds__(kTransformThreads)
     __syncthreads();
     cta_fft_f32(xf, H2, tw);
     const float inv = 1.0f / (float)H2;
-    for (int i = threadIdx.x; i < H; i += blockDim.x) p[i].re = (double)(xf[i].x * inv);
+    for (int i = threadIdx.x; i < H; i += blockDim.x) store_row(p, i, (double)(xf[i].x * inv));
 }
 
 __global__ void k_radon_backproject(DevGeometry g, Batch b, const cd* __restrict__ P, int64_t pstride,

@@ -18,6 +18,15 @@ struct TypeLists {
     int angle[4][kMaxBatch];
 };
 
+// A Radon sector's filtered row value as the transform leaves it in its complex
+// scratch: q, and (float)(0.0 + q), what the back-projection writes on a cell no
+// other row covers.
+struct RowValue {
+    double q;
+    float alone;
+};
+static_assert(sizeof(RowValue) == sizeof(cd), "row values replace the transform's complex values");
+
 // Kahan mode keeps a compensation buffer beside every accumulator.
 enum AccumMode { kAccumReference = 0, kAccumKahan = 1 };
 
@@ -62,7 +71,7 @@ cudaError_t launch_identity(const DevGeometry& g, const Batch& b, const float* S
 // Deskew + accumulate (skewEngine.cuh:772-792) of every slot of the batch into
 // the per-type accumulators acc[t*N ...] (and comp[] in Kahan mode).
 // With Q set, the slots are Radon sectors with dim_l <= 2 dim_i, read from their
-// filtered row values (Q: pstride complex doubles per slot) instead of SO: what
+// filtered row values (Q: pstride entries per slot) instead of SO: what
 // the back-projection would write, without writing it.  rows_over: some of their
 // rows overrun dim_i into the next row.
 // Tensor maps of the skewed-output buffer for the TMA-staged deskew: 3-D
@@ -81,7 +90,7 @@ bool encode_band_maps(DeskewMaps* m, const float* SO, int64_t stride, int slots,
 // that never completes sets *status.
 cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const float* SO,
                               int64_t stride, float* acc, float* comp, int dimx, int dimy,
-                              int accum_mode, cudaStream_t st, const cd* Q = nullptr, int64_t pstride = 0,
+                              int accum_mode, cudaStream_t st, const RowValue* Q = nullptr, int64_t pstride = 0,
                               bool masked = false, const DeskewMaps* maps = nullptr, int* status = nullptr,
                               bool rows_over = false);
 // Max mode with angle encoding (skewEngine.cuh:774-785).
