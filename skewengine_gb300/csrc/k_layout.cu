@@ -265,6 +265,96 @@ __global__ void __launch_bounds__(256, kMode == kDeskewKahan ? 2 : 4) k_deskew(D
     }
 }
 
+// ---- deskew of small grids ----------------------------------------------------
+// The same deskew with one accumulator cell per thread and no staging: the tiles
+// of k_deskew and k_deskew_tma are too few to fill the machine on small grids, and
+// each walks its type's sectors one after another, a staged band and a barrier
+// each (a 64 x 64 run at 180 angles has 8 such tiles, 107 us).  Here a thread
+// reads its column's shift and weight in kSmallStep sectors at once, then the two
+// skewed cells of each, then accumulates them in order: two rounds of latency for
+// kSmallStep sectors, no barrier, and a thread per cell (64 x 64: 19 us).
+// kMasked: cells outside their row's valid range read as zero (SO not zeroed).
+constexpr int kSmallStep = 8;
+
+template <int kMode, bool kMasked>
+__global__ void __launch_bounds__(128) k_deskew_small(DevGeometry g, TypeLists tl, const float* __restrict__ SO,
+                                                      int64_t stride, float* __restrict__ acc,
+                                                      float* __restrict__ comp, int dimx, int dimy) {
+    struct Sec {
+        int64_t cells, col_off, row_off;  // start in SO, in target/weight, in first/last
+        int H, angle;
+    };
+    __shared__ Sec sec[kMaxBatch];
+    const int t = blockIdx.y;
+    const int cnt = tl.count[t];
+    if (cnt == 0) return;
+    for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+        const SectorDesc& d = g.desc[tl.angle[t][q]];
+        sec[q] = Sec{tl.slot[t][q] * stride, d.col_off, d.row_off, d.H, d.angle};
+    }
+    __syncthreads();
+    const int64_t n = (int64_t)dimx * dimy;
+    const int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (cell >= n) return;
+    const int dim_i = (t == 1 || t == 2) ? dimy : dimx;
+    const int i = (int)(cell / dim_i), j = (int)(cell - (int64_t)i * dim_i);
+    float s = acc[t * n + cell], c = kMode == kDeskewKahan ? comp[t * n + cell] : 0.0f;
+    for (int q0 = 0; q0 < cnt; q0 += kSmallStep) {
+        int r[kSmallStep];
+        float w[kSmallStep], lo[kSmallStep], hi[kSmallStep];
+        // (Past the last sector the last one is read again: no load waits for a
+        // branch.)
+#pragma unroll
+        for (int u = 0; u < kSmallStep; u++) {
+            const int64_t col = sec[min(q0 + u, cnt - 1)].col_off + j;
+            r[u] = i + g.target[col];
+            w[u] = g.weight[col];
+        }
+        int f0[kSmallStep], l0[kSmallStep], f1[kSmallStep], l1[kSmallStep];
+        if (kMasked) {
+#pragma unroll
+            for (int u = 0; u < kSmallStep; u++) {
+                const Sec& d = sec[min(q0 + u, cnt - 1)];
+                const int ra = min(r[u], d.H - 1), rb = min(r[u] + 1, d.H - 1);
+                f0[u] = g.first[d.row_off + ra];
+                l0[u] = r[u] < d.H ? g.last[d.row_off + ra] : 0;
+                f1[u] = g.first[d.row_off + rb];
+                l1[u] = r[u] + 1 < d.H ? g.last[d.row_off + rb] : 0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kSmallStep; u++) {
+            const float* so = SO + (sec[min(q0 + u, cnt - 1)].cells + (int64_t)r[u] * dim_i + j);
+            const bool lo_ok = !kMasked || (j >= f0[u] && j < l0[u]), hi_ok = !kMasked || (j >= f1[u] && j < l1[u]);
+            lo[u] = lo_ok ? so[0] : 0.0f;
+            hi[u] = hi_ok ? so[dim_i] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kSmallStep; u++) {
+            if (q0 + u >= cnt) continue;
+            if (kMode == kDeskewMax) {
+                const float m = (lo[u] < hi[u]) ? hi[u] : lo[u];  // std::max(lo, hi)
+                const float v = (s < m) ? m : s;                  // std::max(acc, m)
+                // a + 1000*(int)(v/1000): the low decimal digits carry the angle.
+                const int qq = __float2int_rz(__fdiv_rn(v, 1000.0f));
+                s = __int2float_rn(sec[q0 + u].angle + 1000 * qq);
+            } else {
+                const float v = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, w[u]), lo[u]), __fmul_rn(w[u], hi[u]));
+                if (kMode == kDeskewKahan) {
+                    const float y = __fsub_rn(v, c);
+                    const float ts = __fadd_rn(s, y);
+                    c = __fsub_rn(__fsub_rn(ts, s), y);
+                    s = ts;
+                } else {
+                    s = __fadd_rn(s, v);
+                }
+            }
+        }
+    }
+    acc[t * n + cell] = s;
+    if (kMode == kDeskewKahan) comp[t * n + cell] = c;
+}
+
 // ---- Radon deskew -----------------------------------------------------------
 // The additive deskew of Radon sectors whose back-projection is not formed: a
 // skewed output cell (r, c), c < dim_i, is read from the filtered row values Q
@@ -794,6 +884,15 @@ static dim3 deskew_grid(int dimx, int dimy) {
     return dim3((dl + kTile - 1) / kTile, (dl + kDeskewRows - 1) / kDeskewRows, 4);
 }
 
+// Grids the small kernel deskews, by the cells of its threads: up to here they
+// are short of the tiled kernels' band reuse by less than the tiles are short of
+// filling the machine (us at 180 angles, small against tiled: masked sums 19 / 82
+// at 64 x 64, 55 / 86 at 256, 84 / 91 at 320, 113 / 94 at 384; maximum 41 / 110 at
+// 256, 128 / 139 at 512, 281 / 255 at 768).
+constexpr int64_t kSmallAddCells = 320 * 320, kSmallMaxCells = 512 * 512;
+
+static dim3 small_grid(int dimx, int dimy) { return dim3((unsigned)(((int64_t)dimx * dimy + 127) / 128), 4); }
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // against the driver library).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -866,6 +965,13 @@ cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const f
                               const RowValue* Q, int64_t pstride, bool masked, const DeskewMaps* maps, int* status,
                               bool rows_over) {
     const dim3 grid = deskew_grid(dimx, dimy), block(kTile, 8);
+    if (!Q && (int64_t)dimx * dimy <= kSmallAddCells) {
+        const bool kahan = accum_mode == kAccumKahan;
+        auto kern = masked ? (kahan ? k_deskew_small<kDeskewKahan, true> : k_deskew_small<kDeskewAdd, true>)
+                           : (kahan ? k_deskew_small<kDeskewKahan, false> : k_deskew_small<kDeskewAdd, false>);
+        kern<<<small_grid(dimx, dimy), 128, 0, st>>>(g, tl, SO, stride, acc, kahan ? comp : nullptr, dimx, dimy);
+        return cudaGetLastError();
+    }
     if (!Q && maps && maps->ok && status) {
         if (accum_mode == kAccumKahan) {
             if (masked)
@@ -906,6 +1012,11 @@ cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const f
 
 cudaError_t launch_deskew_max(const DevGeometry& g, const TypeLists& tl, const float* SO, int64_t stride,
                               float* acc, int dimx, int dimy, cudaStream_t st) {
+    if ((int64_t)dimx * dimy <= kSmallMaxCells) {
+        k_deskew_small<kDeskewMax, false><<<small_grid(dimx, dimy), 128, 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx,
+                                                                                 dimy);
+        return cudaGetLastError();
+    }
     k_deskew<kDeskewMax><<<deskew_grid(dimx, dimy), dim3(kTile, 8), 0, st>>>(g, tl, SO, stride, acc, nullptr, dimx,
                                                                             dimy);
     return cudaGetLastError();
