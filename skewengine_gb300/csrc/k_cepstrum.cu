@@ -87,11 +87,19 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
             const int64_t base = (int64_t)r * d.dim_i;
             const int j = (int)(p - base);
             const int f = first[r], l = last[r];
-            bool fin = true;
+            bool fin = true, empty = true;
             for (int m = lane; m < kWin; m += 32) {
                 const int idx = j - kWin / 2 + m;
                 x[m] = (idx < f || idx >= l) ? cd{0.0, 0.0} : cd{(double)in[base + idx], 0.0};
                 fin = fin && isfinite(x[m].re);
+                empty = empty && x[m].re == 0.0;
+            }
+            // An empty window (image borders, cells of overrunning rows: float always
+            // leaves it open): every log is -inf, so every c_k but the first is NaN
+            // and no sample ascends: 0.
+            if (kMarked && __all_sync(0xffffffffu, empty)) {
+                if (lane == 0) out[p] = 0.0f;
+                continue;
             }
             __syncwarp();
             // Finite real input: the reduced-work FFT gives the same values up to the
