@@ -452,6 +452,26 @@ int ske_conv3x3_upcat_bf16(const void* xlow, const void* xskip, const void* w, c
  * they are).  cin and cout multiples of 8. */
 int ske_conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int n, int h, int w_, int cin,
                            int cout, void* stream);
+/* Gradient through the convolution's ReLU and of its bias, for `pixels` x c
+ * bfloat16 tensors: dz = dy where y > 0, dy * 0 elsewhere, db[c] = the float32
+ * sum of dz over the pixels (the same order on every call).  y null: no ReLU,
+ * dz is not written and db sums dy.  c a multiple of 8 up to 2048 with c / 8 a
+ * power of two up to 256. */
+int ske_relu_grad_bf16(const void* y, const void* dy, void* dz, float* db, int64_t pixels, int c, void* stream);
+/* Weights of the data gradient (ske_conv3x3_bf16 of the output gradient):
+ * out (cin x kpad(cout)) entry [ci][tap*cout + co] = w[co][(8 - tap)*cin + ci]
+ * of w (cout x kpad(cin)), zero in the padding columns; kpad as above. */
+int ske_flip_weights_bf16(const void* w, void* out, int cin, int cout, void* stream);
+/* The whole backward pass of ske_conv3x3_bf16 (+ ReLU when y, its output, is
+ * given): db and the gradient through the ReLU as ske_relu_grad_bf16, dx (null:
+ * not formed) as ske_conv3x3_bf16 of it with the flipped weights, dw (cout x
+ * kpad(cin), written whole) as ske_conv3x3_wgrad_bf16.  scratch: device memory on
+ * a 256-byte boundary, at least ske_conv3x3_backward_scratch bytes.  The limits
+ * of those three calls apply. */
+int ske_conv3x3_backward_bf16(const void* x, const void* w, const void* y, const void* dy, void* dx, float* dw,
+                              float* db, void* scratch, size_t scratch_bytes, int n, int h, int w_, int cin, int cout,
+                              void* stream);
+size_t ske_conv3x3_backward_scratch(int n, int h, int w_, int cin, int cout, int relu);
 /* The same 3x3 convolution (+ bias, ReLU when relu != 0) followed by a 1x1
  * convolution to one channel, fused: y[pixel] = head_b + sum over c in order of
  * bf16(act[pixel][c]) * head_w[c] in float32, y float32 (n x h x w), head_w

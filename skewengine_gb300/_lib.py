@@ -94,6 +94,10 @@ SIGNATURES = [
                                    C.c_int, C.c_int, C.c_int, C.c_void_p]),
     ("ske_conv3x3_upcat_bf16", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                          C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]),
+    ("ske_conv3x3_backward_bf16", C.c_int, [C.c_void_p] * 8 + [C.c_size_t] + [C.c_int] * 5 + [C.c_void_p]),
+    ("ske_conv3x3_backward_scratch", C.c_size_t, [C.c_int] * 6),
+    ("ske_relu_grad_bf16", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int, C.c_void_p]),
+    ("ske_flip_weights_bf16", C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p]),
     ("ske_conv3x3_wgrad_bf16", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                          C.c_int, C.c_void_p]),
     ("ske_conv_select", C.c_int, [C.c_int]),

@@ -696,6 +696,240 @@ __global__ void __launch_bounds__(kThreads) k_conv3x3_wgrad(const bf16* __restri
         }
 }
 
+// An 8-byte aligned float32 array takes paired atomics.
+int aligned8(const void* p) { return ((uintptr_t)p & 7) == 0; }
+
+// Weight gradient by image rows, the default for 32 input channels and more
+// (k_conv3x3_wgrad keeps the others: its tile is 64 of the 9 Cin columns, which
+// few channels fill better).  A CTA owns 32*kWco output x 16*kWci input channels
+// of all nine taps and walks down the rows of one column segment of kSeg pixels:
+// per row it stages dY (kSeg pixels) and one new row of X (kSeg + 2 pixels, a ring
+// of four rows), so X and dY leave L2 once per channel block instead of once per
+// tap, and nine taps share every dY fragment: 11 ldmatrix for 36 MMAs of a warp,
+// against 4 for 8.  Bound by the mma.sync rate.  At 64 -> 64 channels, 16 images
+// of 128 x 128: 139 us by 64-column tiles, WGRAD_US so.
+template <int kWco, int kWci, int kSeg>
+struct WgRows {
+    static constexpr int kThr = 32 * kWco * kWci;
+    static constexpr int kCo = 32 * kWco, kCi = 16 * kWci;
+    static constexpr int kPitchD = kCo + 8, kPitchX = kCi + 8;  // 16 bytes past a multiple of 32: conflict-free
+    bf16 d[2][kSeg][kPitchD];
+    bf16 x[4][kSeg + 2][kPitchX];
+};
+
+template <int kWco, int kWci, int kSeg>
+__global__ void __launch_bounds__(32 * kWco * kWci)
+    k_conv3x3_wgrad_rows(const bf16* __restrict__ X, const bf16* __restrict__ dY, float* __restrict__ dW, int H, int W,
+                         int Cin, int Cout, int Kpad, int segs, int64_t total, int share, int pairs) {
+    typedef WgRows<kWco, kWci, kSeg> Sm;
+    extern __shared__ __align__(16) unsigned char wg_smem[];
+    Sm& sm = *reinterpret_cast<Sm*>(wg_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ci0 = blockIdx.y * Sm::kCi, co0 = blockIdx.z * Sm::kCo;
+    // Row segments of (image, column segment) one below the other, `share` of all
+    // `total` of them per CTA.
+    int64_t u0 = (int64_t)blockIdx.x * share;
+    const int64_t u1 = min(u0 + share, total);
+    int x0 = 0, y0 = 0, y1 = 0;  // the piece of one column segment at hand
+    int64_t img = 0;
+    auto load_d = [&](int y) {
+        bf16(*dst)[Sm::kPitchD] = sm.d[y & 1];
+        for (int c = tid; c < kSeg * (Sm::kCo / 8); c += Sm::kThr) {
+            const int p = c / (Sm::kCo / 8), off = c % (Sm::kCo / 8) * 8;
+            const bool ok = y < y1 && x0 + p < W && co0 + off < Cout;
+            cp_async16(&dst[p][off], ok ? dY + (img + (int64_t)y * W + x0 + p) * Cout + co0 + off : dY, ok ? 16 : 0);
+        }
+    };
+    auto load_x = [&](int y) {  // image row y (may lie outside: zeros) into ring slot y & 3
+        bf16(*dst)[Sm::kPitchX] = sm.x[y & 3];
+        for (int c = tid; c < (kSeg + 2) * (Sm::kCi / 8); c += Sm::kThr) {
+            const int p = c / (Sm::kCi / 8), off = c % (Sm::kCi / 8) * 8;
+            const int xx = x0 + p - 1;
+            const bool ok = y >= 0 && y < H && xx >= 0 && xx < W && ci0 + off < Cin;
+            cp_async16(&dst[p][off], ok ? X + (img + (int64_t)y * W + xx) * Cin + ci0 + off : X, ok ? 16 : 0);
+        }
+    };
+    float acc[9][2][2][4];
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[t][i][j][e] = 0.0f;
+    const int wc = (warp / kWci) * 32, wk = (warp % kWci) * 16;
+    while (u0 < u1) {
+        const int64_t col = u0 / H;
+        y0 = (int)(u0 - col * H);
+        y1 = (int)min((int64_t)H, y0 + (u1 - u0));
+        x0 = (int)(col % segs) * kSeg;
+        img = col / segs * H * W;
+        u0 += y1 - y0;
+        load_x(y0 - 1);
+        load_x(y0);
+        load_x(y0 + 1);
+        load_d(y0);
+        cp_commit();
+        for (int y = y0; y < y1; y++) {
+            if (y + 1 < y1) {  // slot (y + 2) & 3 held row y - 2, read before the last barrier
+                load_x(y + 2);
+                load_d(y + 1);
+            }
+            cp_commit();
+            cp_wait<1>();
+            __syncthreads();
+            const bf16(*D)[Sm::kPitchD] = sm.d[y & 1];
+#pragma unroll
+            for (int kk = 0; kk < kSeg; kk += 16) {
+                unsigned af[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    ldsm_x4_t(af[i][0], af[i][1], af[i][2], af[i][3],
+                              &D[kk + (lane & 7) + ((lane >> 4) << 3)][wc + i * 16 + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+                for (int t = 0; t < 9; t++) {
+                    unsigned b[2][2];
+                    ldsm_x4_t(b[0][0], b[0][1], b[1][0], b[1][1],
+                              &sm.x[(y + t / 3 - 1) & 3][kk + t % 3 + (lane & 7) + ((lane >> 3) & 1) * 8]
+                                   [wk + (lane >> 4) * 8]);
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+#pragma unroll
+                        for (int j = 0; j < 2; j++) mma_bf16(acc[t][i][j], af[i], b[j]);
+                }
+            }
+            __syncthreads();
+        }
+        cp_wait<0>();
+    }
+#pragma unroll
+    for (int t = 0; t < 9; t++)
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int ci = ci0 + wk + j * 8 + (lane & 3) * 2;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int co = co0 + wc + i * 16 + (lane >> 2) + h * 8;
+                    if (co >= Cout || ci >= Cin) continue;
+                    float* p = dW + (int64_t)co * Kpad + t * Cin + ci;  // ci and Cin even: 8-byte aligned pairs
+                    const float v0 = acc[t][i][j][2 * h], v1 = acc[t][i][j][2 * h + 1];
+                    if (pairs) {
+                        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(v0), "f"(v1) : "memory");
+                    } else {
+                        atomicAdd(p, v0);
+                        atomicAdd(p + 1, v1);
+                    }
+                }
+            }
+}
+
+template <int kWco, int kWci, int kSeg>
+cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* dw, int n, int h, int w_, int cin, int cout,
+                              int kpad, int sms, cudaStream_t st) {
+    typedef WgRows<kWco, kWci, kSeg> Sm;
+    const int smem = (int)sizeof(Sm);
+    auto kern = k_conv3x3_wgrad_rows<kWco, kWci, kSeg>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int segs = (w_ + kSeg - 1) / kSeg, bi = (cin + Sm::kCi - 1) / Sm::kCi, bo = (cout + Sm::kCo - 1) / Sm::kCo;
+    int per_sm = 1;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Sm::kThr, smem);
+    if (e != cudaSuccess) return e;
+    // One wave of CTAs, at least 4 row segments each (a piece reads two rows of X
+    // more than it covers, a CTA ends in 9 * kCo * kCi atomics).
+    const int64_t total = (int64_t)n * segs * h, wave = (int64_t)sms * (per_sm < 1 ? 1 : per_sm);
+    int64_t workers = wave / ((int64_t)bi * bo);
+    workers = std::max<int64_t>(1, std::min(workers, (total + 3) / 4));
+    const int64_t share = (total + workers - 1) / workers;
+    workers = (total + share - 1) / share;
+    if (share > 0x7fffffff || bi > 65535 || bo > 65535) return cudaErrorInvalidValue;
+    kern<<<dim3((unsigned)workers, bi, bo), Sm::kThr, smem, st>>>(x, dy, dw, h, w_, cin, cout, kpad, segs, total,
+                                                                 (int)share, aligned8(dw));
+    return cudaGetLastError();
+}
+
+// ---- gradient through the ReLU, and of the bias -------------------------------
+// dZ = dY where y > 0, dY * 0 elsewhere (bfloat16, the tensor expression
+// dY * (y > 0)), and the sums of dZ over the pixels in float32.  A thread owns 8
+// channels of every 256 / (C / 8)-th pixel of its block's share; the block's sums
+// go to a row of `part`, which k_bias_sum adds up in block order.  Memory bound
+// (6 bytes a value): 100 MB at 16 x 128 x 128 x 64, RELU_US against 195 us for the
+// comparison, product, conversion and reduction one after another.
+constexpr int kReluBlocks = 608;   // 4 per SM
+constexpr int kReluMaxC = 2048;    // channels: C / 8 divides 256
+
+__global__ void __launch_bounds__(256) k_relu_grad(const uint4* __restrict__ y, const uint4* __restrict__ dy,
+                                                   uint4* __restrict__ dz, float* __restrict__ part, int64_t pixels,
+                                                   int groups) {
+    __shared__ float sums[256][9];
+    const int g = threadIdx.x % groups;
+    const int64_t step = (int64_t)gridDim.x * (256 / groups);
+    float s[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) s[k] = 0.0f;
+    for (int64_t p = (int64_t)blockIdx.x * (256 / groups) + threadIdx.x / groups; p < pixels; p += step) {
+        uint4 v = dy[p * groups + g];
+        const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&v);
+        float f[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 t = __bfloat1622float2(a2[k]);
+            f[2 * k] = t.x;
+            f[2 * k + 1] = t.y;
+        }
+        if (y) {
+            const uint4 u = y[p * groups + g];
+            const __nv_bfloat162* y2 = reinterpret_cast<const __nv_bfloat162*>(&u);
+            __nv_bfloat162 o[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float2 t = __bfloat1622float2(y2[k]);
+                f[2 * k] = t.x > 0.0f ? f[2 * k] : f[2 * k] * 0.0f;
+                f[2 * k + 1] = t.y > 0.0f ? f[2 * k + 1] : f[2 * k + 1] * 0.0f;
+                o[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+            }
+            dz[p * groups + g] = *reinterpret_cast<const uint4*>(o);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) s[k] += f[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) sums[threadIdx.x][k] = s[k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < 8 * groups; c += 256) {
+        float t = 0.0f;
+        for (int r = c / 8; r < 256; r += groups) t += sums[r][c & 7];
+        part[(int64_t)blockIdx.x * 8 * groups + c] = t;
+    }
+}
+
+__global__ void __launch_bounds__(1024) k_bias_sum(const float* __restrict__ part, float* __restrict__ db, int blocks,
+                                                   int C) {
+    __shared__ float sums[32][33];
+    const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, w = threadIdx.x >> 5;
+    float t = 0.0f;
+#pragma unroll 8
+    for (int b = w; b < blocks; b += 32) t += c < C ? part[(int64_t)b * C + c] : 0.0f;
+    sums[w][lane] = t;
+    __syncthreads();
+    if (w == 0 && c < C) {
+        for (int k = 1; k < 32; k++) t += sums[k][lane];
+        db[c] = t;
+    }
+}
+
+// Weights of the data gradient: out[ci][tap*Cout + co] = w[co][(8 - tap)*Cin + ci],
+// zero in the padding columns.
+__global__ void k_flip_weights(const bf16* __restrict__ w, bf16* __restrict__ out, int Cin, int Cout, int kin, int kout) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (int64_t)Cin * kout) return;
+    const int ci = (int)(e / kout), k = (int)(e - (int64_t)ci * kout), tap = k / Cout, co = k - tap * Cout;
+    out[e] = tap < 9 ? w[(int64_t)co * kin + (8 - tap) * Cin + ci] : __float2bfloat16(0.0f);
+}
+
 // cp.async copies 16 bytes: tensors must start on 16-byte boundaries (outputs:
 // 4 bytes, for the bf16 pairs of the epilogue).
 bool aligned(const void* p, uintptr_t a) { return ((uintptr_t)p & (a - 1)) == 0; }
@@ -1696,6 +1930,16 @@ static int ske_conv3x3_wgrad_bf16_impl(const void* x, const void* dy, float* dw,
         k_conv3x3_wgrad_tc<<<g3, kThreads, smem, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)dy, dw, wg);
         return cudaGetLastError() == cudaSuccess ? SKE_OK : SKE_ERR_CUDA;
     }
+    if (g_wgrad_path == 1 && cin >= 32 && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0) {
+        const bool wide = cout > 32, longer = w_ > 32;
+        auto fn = wide ? (longer ? launch_wgrad_rows<2, 4, 64> : launch_wgrad_rows<2, 4, 32>)
+                       : (longer ? launch_wgrad_rows<1, 2, 64> : launch_wgrad_rows<1, 2, 32>);
+        return fn((const bf16*)x, (const bf16*)dy, dw, n, h, w_, cin, cout, kpad, sms, (cudaStream_t)stream) ==
+                       cudaSuccess
+                   ? SKE_OK
+                   : SKE_ERR_CUDA;
+    }
     const dim3 grid((unsigned)((kpad + 63) / 64), (unsigned)((cout + 63) / 64),
                     (unsigned)((m + kWgChunk - 1) / kWgChunk));
     k_conv3x3_wgrad<<<grid, kThreads, 0, (cudaStream_t)stream>>>((const bf16*)x, (const bf16*)dy, dw, (int)m, h, w_,
@@ -1706,4 +1950,106 @@ static int ske_conv3x3_wgrad_bf16_impl(const void* x, const void* dy, float* dw,
 extern "C" int ske_conv3x3_wgrad_bf16(const void* x, const void* dy, float* dw, int n, int h, int w_, int cin,
                                       int cout, void* stream) {
     return conv_result(ske_conv3x3_wgrad_bf16_impl(x, dy, dw, n, h, w_, cin, cout, stream), "conv3x3_wgrad_bf16");
+}
+
+static bool relu_grad_ok(const void* y, const void* dy, const void* dz, const float* db, int64_t pixels, int c) {
+    return dy && db && (!y || dz) && pixels >= 1 && c >= 8 && c <= kReluMaxC && c % 8 == 0 && 256 % (c / 8) == 0 &&
+           aligned(y, 16) && aligned(dy, 16) && aligned(dz, 16) && aligned(db, 4);
+}
+
+// part: kReluBlocks * c floats.
+static cudaError_t launch_relu_grad(const void* y, const void* dy, void* dz, float* db, float* part, int64_t pixels,
+                                    int c, cudaStream_t st) {
+    const int groups = c / 8;
+    const int64_t want = (pixels + 256 / groups - 1) / (256 / groups);
+    const int blocks = (int)std::min<int64_t>(kReluBlocks, want);
+    k_relu_grad<<<blocks, 256, 0, st>>>((const uint4*)y, (const uint4*)dy, (uint4*)dz, part, pixels, groups);
+    k_bias_sum<<<(c + 31) / 32, 1024, 0, st>>>(part, db, blocks, c);
+    return cudaGetLastError();
+}
+
+static int ske_relu_grad_bf16_impl(const void* y, const void* dy, void* dz, float* db, int64_t pixels, int c,
+                                  void* stream) {
+    if (!relu_grad_ok(y, dy, dz, db, pixels, c)) return SKE_ERR_INVALID;
+    const cudaStream_t st = (cudaStream_t)stream;
+    float* part = nullptr;
+    if (cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(float) * (size_t)kReluBlocks * c, st) != cudaSuccess) {
+        cudaGetLastError();
+        return SKE_ERR_CUDA;
+    }
+    const cudaError_t e = launch_relu_grad(y, dy, dz, db, part, pixels, c, st);
+    cudaFreeAsync(part, st);
+    return e == cudaSuccess ? SKE_OK : SKE_ERR_CUDA;
+}
+
+extern "C" int ske_relu_grad_bf16(const void* y, const void* dy, void* dz, float* db, int64_t pixels, int c,
+                                  void* stream) {
+    return conv_result(ske_relu_grad_bf16_impl(y, dy, dz, db, pixels, c, stream), "relu_grad_bf16");
+}
+
+static int ske_flip_weights_bf16_impl(const void* w, void* out, int cin, int cout, void* stream) {
+    if (!w || !out || cin < 1 || cout < 1 || !aligned(w, 2) || !aligned(out, 2)) return SKE_ERR_INVALID;
+    if ((int64_t)cin * 9 > 0x7fffffff / 2 || (int64_t)cout * 9 > 0x7fffffff / 2) return SKE_ERR_INVALID;
+    const int kin = (9 * cin + kBK - 1) / kBK * kBK, kout = (9 * cout + kBK - 1) / kBK * kBK;
+    const int64_t total = (int64_t)cin * kout;
+    if ((total + 255) / 256 > 0x7fffffff) return SKE_ERR_INVALID;
+    k_flip_weights<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)w, (bf16*)out, cin,
+                                                                                     cout, kin, kout);
+    return cudaGetLastError() == cudaSuccess ? SKE_OK : SKE_ERR_CUDA;
+}
+
+extern "C" int ske_flip_weights_bf16(const void* w, void* out, int cin, int cout, void* stream) {
+    return conv_result(ske_flip_weights_bf16_impl(w, out, cin, cout, stream), "flip_weights_bf16");
+}
+
+// Scratch of a backward pass: dZ (with a ReLU and more than the bias gradient to
+// form), the flipped weights (with dx) and the bias sums.
+struct BackwardScratch {
+    size_t dz, flip, part, total;
+    BackwardScratch(int64_t pixels, int cin, int cout, bool relu) {
+        const size_t kout = (size_t)(9 * cout + kBK - 1) / kBK * kBK;
+        dz = 0;
+        flip = relu ? ((size_t)pixels * cout * 2 + 255) / 256 * 256 : 0;
+        part = flip + (cin * kout * 2 + 255) / 256 * 256;
+        total = part + sizeof(float) * kReluBlocks * (size_t)cout;
+    }
+};
+
+static int ske_conv3x3_backward_bf16_impl(const void* x, const void* w, const void* y, const void* dy, void* dx,
+                                         float* dw, float* db, void* scratch, size_t scratch_bytes, int n, int h,
+                                         int w_, int cin, int cout, void* stream) {
+    if (n < 1 || h < 1 || w_ < 1 || cin < 8 || cin % 8 || cout < 8 || cout % 8 || !scratch || !aligned(scratch, 256) ||
+        !dw)
+        return SKE_ERR_INVALID;
+    const int64_t pixels = (int64_t)n * h * w_;
+    const BackwardScratch at(pixels, cin, cout, y != nullptr);
+    unsigned char* base = static_cast<unsigned char*>(scratch);
+    void* dz = y ? base + at.dz : nullptr;
+    if (scratch_bytes < at.total || !relu_grad_ok(y, dy, dz, db, pixels, cout)) return SKE_ERR_INVALID;
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (launch_relu_grad(y, dy, dz, db, reinterpret_cast<float*>(base + at.part), pixels, cout, st) != cudaSuccess)
+        return SKE_ERR_CUDA;
+    const void* g = y ? dz : dy;
+    if (dx) {
+        void* flip = base + at.flip;
+        int rc = ske_flip_weights_bf16_impl(w, flip, cin, cout, stream);
+        if (rc == SKE_OK)
+            rc = ske_conv3x3_bf16_impl(g, flip, nullptr, dx, n, h, w_, cout, cin, 0, stream);
+        if (rc != SKE_OK) return rc;
+    }
+    const size_t kin = (size_t)(9 * cin + kBK - 1) / kBK * kBK;
+    if (cudaMemsetAsync(dw, 0, sizeof(float) * kin * cout, st) != cudaSuccess) return SKE_ERR_CUDA;
+    return ske_conv3x3_wgrad_bf16_impl(x, g, dw, n, h, w_, cin, cout, stream);
+}
+
+extern "C" int ske_conv3x3_backward_bf16(const void* x, const void* w, const void* y, const void* dy, void* dx,
+                                         float* dw, float* db, void* scratch, size_t scratch_bytes, int n, int h,
+                                         int w_, int cin, int cout, void* stream) {
+    return conv_result(ske_conv3x3_backward_bf16_impl(x, w, y, dy, dx, dw, db, scratch, scratch_bytes, n, h, w_, cin,
+                                                      cout, stream),
+                       "conv3x3_backward_bf16");
+}
+
+extern "C" size_t ske_conv3x3_backward_scratch(int n, int h, int w_, int cin, int cout, int relu) {
+    return BackwardScratch((int64_t)n * h * w_, cin, cout, relu != 0).total;
 }

@@ -175,10 +175,62 @@ def conv3x3_wgrad(x, dy, cout: int):
 def flip_transpose(w, cin: int, cout: int):
     """Weights of the data gradient: W'[ci][(ky*3+kx)*cout + co] = W[co][((2-ky)*3 + 2-kx)*cin + ci]."""
     import torch
+    if w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and tuple(w.shape) == (cout, kpad(cin)):
+        out = torch.empty((cin, kpad(cout)), dtype=w.dtype, device=w.device)
+        check(load().ske_flip_weights_bf16(C.c_void_p(w.data_ptr()), C.c_void_p(out.data_ptr()), cin, cout,
+                                           _stream(w)))
+        return out
     w9 = w[:, : 9 * cin].reshape(cout, 9, cin).flip(1).permute(2, 1, 0).reshape(cin, 9 * cout)
     out = torch.zeros((cin, kpad(cout)), dtype=w.dtype, device=w.device)
     out[:, : 9 * cout] = w9
     return out
+
+
+def _relu_grad_applies(dy, y) -> bool:
+    import torch
+    c = dy.shape[-1]
+    if not (dy.is_cuda and dy.dtype == torch.bfloat16 and dy.is_contiguous() and dy.numel() and c % 8 == 0
+            and c <= 2048 and 256 % (c // 8) == 0 and dy.data_ptr() % 16 == 0):
+        return False
+    return y is None or (y.shape == dy.shape and y.dtype == dy.dtype and y.is_contiguous() and y.device == dy.device)
+
+
+def conv3x3_backward(x, w, y, dy, need_dx: bool = True):
+    """(dx, dw, db) of conv3x3(x, w, b), with a ReLU when its output y is given, in
+    one call (ske_conv3x3_backward_bf16); None where its kernels do not apply."""
+    import torch
+    if not (_relu_grad_applies(dy, y) and dy.dim() == 4 and x.shape[:3] == dy.shape[:3] and x.device == dy.device):
+        return None
+    _need(x, "x", torch.bfloat16)
+    n, h, wd, cin = x.shape
+    cout = dy.shape[3]
+    _need(w, "w", torch.bfloat16, (cout, kpad(cin)), x.device)
+    lib = load()
+    size = lib.ske_conv3x3_backward_scratch(n, h, wd, cin, cout, int(y is not None))
+    scratch = torch.empty(size, dtype=torch.uint8, device=x.device)
+    dx = torch.empty_like(x) if need_dx else None
+    dw = torch.empty((cout, kpad(cin)), dtype=torch.float32, device=x.device)
+    db = torch.empty(cout, dtype=torch.float32, device=x.device)
+    check(lib.ske_conv3x3_backward_bf16(x.data_ptr(), w.data_ptr(), y.data_ptr() if y is not None else None,
+                                        dy.data_ptr(), dx.data_ptr() if need_dx else None, dw.data_ptr(),
+                                        db.data_ptr(), scratch.data_ptr(), size, n, h, wd, cin, cout, _stream(x)))
+    return dx, dw, db
+
+
+def relu_grad(dy, y=None):
+    """(dz, db): dz = dy * (y > 0) (dy itself without y) and its float32 sums over
+    all but the last dimension, in one pass (ske_relu_grad_bf16); None where that
+    kernel does not apply."""
+    import torch
+    if not _relu_grad_applies(dy, y):
+        return None
+    c = dy.shape[-1]
+    dz = dy if y is None else torch.empty_like(dy)
+    db = torch.empty(c, dtype=torch.float32, device=dy.device)
+    check(load().ske_relu_grad_bf16(C.c_void_p(y.data_ptr()) if y is not None else None, C.c_void_p(dy.data_ptr()),
+                                    C.c_void_p(dz.data_ptr()), C.c_void_p(db.data_ptr()), dy.numel() // c, c,
+                                    _stream(dy)))
+    return dz, db
 
 
 def _conv_fn():
@@ -196,11 +248,15 @@ def _conv_fn():
         @staticmethod
         def backward(ctx, dy):
             x, w, y = ctx.saved_tensors
+            need_dx = ctx.needs_input_grad[0]
+            fused = conv3x3_backward(x, w, y if ctx.relu else None, dy, need_dx)
+            if fused is not None:
+                return (*fused, None)
             if ctx.relu:
                 dy = dy * (y > 0)
             dy = dy.to(torch.bfloat16).contiguous()
             cin, cout = x.shape[3], w.shape[0]
-            dx = conv3x3(dy, flip_transpose(w, cin, cout)) if ctx.needs_input_grad[0] else None
+            dx = conv3x3(dy, flip_transpose(w, cin, cout)) if need_dx else None
             dw = conv3x3_wgrad(x, dy, cout)
             db = dy.float().sum((0, 1, 2))
             return dx, dw, db, None
