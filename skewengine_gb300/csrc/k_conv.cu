@@ -826,18 +826,27 @@ __global__ void __launch_bounds__(32 * kWco * kWci)
             }
 }
 
+constexpr int kWgDevices = 64;
+
 template <int kWco, int kWci, int kSeg>
 cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* dw, int n, int h, int w_, int cin, int cout,
                               int kpad, int sms, cudaStream_t st) {
     typedef WgRows<kWco, kWci, kSeg> Sm;
     const int smem = (int)sizeof(Sm);
     auto kern = k_conv3x3_wgrad_rows<kWco, kWci, kSeg>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     const int segs = (w_ + kSeg - 1) / kSeg, bi = (cin + Sm::kCi - 1) / Sm::kCi, bo = (cout + Sm::kCo - 1) / Sm::kCo;
-    int per_sm = 1;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Sm::kThr, smem);
+    // Per device, once: the kernel's shared-memory limit and its CTAs per SM.
+    static std::atomic<int> ctas[kWgDevices];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    int per_sm = dev < kWgDevices ? ctas[dev].load(std::memory_order_relaxed) : 0;
+    if (per_sm < 1) {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, Sm::kThr, smem);
+        if (e != cudaSuccess) return e;
+        if (dev < kWgDevices) ctas[dev].store(per_sm, std::memory_order_relaxed);
+    }
     // One wave of CTAs, at least 4 row segments each (a piece reads two rows of X
     // more than it covers, a CTA ends in 9 * kCo * kCi atomics).
     const int64_t total = (int64_t)n * segs * h, wave = (int64_t)sms * (per_sm < 1 ? 1 : per_sm);
@@ -1426,6 +1435,40 @@ bool ws_geometry(WsGeom* g, int n, int h, int w_, int cin, int cout, int c1, int
     return true;
 }
 
+// Stream-ordered temporaries (packed weights, partial sums) of one device, from a
+// pool of their own: the default pool gives its memory back to the driver whenever
+// the program synchronises, and mapping it again took 200 us of the next call.
+// The pool keeps at most kPoolKeep bytes over a synchronisation, is safe with any
+// threads and streams, and serves at most kWsDevices devices (others, and a
+// driver without pools, take the default pool).
+constexpr uint64_t kPoolKeep = 64ull << 20;
+cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st) {
+    static std::atomic<cudaMemPool_t> pools[kWsDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kWsDevices) {
+        cudaMemPool_t pool = pools[dev].load(std::memory_order_acquire);
+        if (!pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t made = nullptr;
+            uint64_t keep = kPoolKeep;
+            if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
+                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+                if (pools[dev].compare_exchange_strong(pool, made, std::memory_order_acq_rel)) pool = made;
+                else cudaMemPoolDestroy(made);  // another thread was first
+            }
+        }
+        if (pool) {
+            const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+            if (e == cudaSuccess) return e;
+        }
+        cudaGetLastError();
+    }
+    return cudaMallocAsync(p, bytes, st);
+}
+
 // Packs the weights into a stream-ordered temporary (freed after the launch)
 // and launches one CTA per SM.  SKE_ERR_UNSUPPORTED if the temporary cannot be
 // had (the caller then takes another kernel).
@@ -1451,7 +1494,7 @@ int launch_conv_ws(const WsGeom& g, const bf16* x, const bf16* w, const float* b
     const int kpad = (9 * g.Cin + kTcBK - 1) / kTcBK * kTcBK;
     const int rows = g.items * g.gs * 18 * g.Cout;  // 16-byte rows of the packed weights
     bf16* wp = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&wp), (size_t)rows * 16, st) != cudaSuccess) {
+    if (temp_alloc(reinterpret_cast<void**>(&wp), (size_t)rows * 16, st) != cudaSuccess) {
         cudaGetLastError();
         return SKE_ERR_UNSUPPORTED;
     }
@@ -1973,7 +2016,7 @@ static int ske_relu_grad_bf16_impl(const void* y, const void* dy, void* dz, floa
     if (!relu_grad_ok(y, dy, dz, db, pixels, c)) return SKE_ERR_INVALID;
     const cudaStream_t st = (cudaStream_t)stream;
     float* part = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(float) * (size_t)kReluBlocks * c, st) != cudaSuccess) {
+    if (temp_alloc(reinterpret_cast<void**>(&part), sizeof(float) * (size_t)kReluBlocks * c, st) != cudaSuccess) {
         cudaGetLastError();
         return SKE_ERR_CUDA;
     }
