@@ -25,7 +25,7 @@
 // window read from the staged segment), and max-deskews into the tile's
 // registers.  The skewed input and output never reach HBM; the orientations
 // (4 x N floats per image) stay L2-resident.
-#include "kernels.h"
+#include "cepstrum_bin.cuh"
 
 namespace ske {
 
@@ -70,10 +70,6 @@ __device__ __forceinline__ void fft32(float (&re)[32], float (&im)[32]) {
             }
         }
     }
-}
-
-__device__ __forceinline__ constexpr int brev5(int v) {
-    return ((v & 1) << 4) | ((v & 2) << 2) | (v & 4) | ((v & 8) >> 2) | ((v & 16) >> 4);
 }
 
 // Cepstrum peak of the 64-sample window w[0..63] (zeros outside the row), as
@@ -150,6 +146,8 @@ __global__ void __launch_bounds__(kCThreads, 2)
     k_cepstrum_fused(BatchTables T, DevGeometry g, TypeLists tl, int dim, int tiles_x, int tiles_y) {
     __shared__ float seg[kCBand][kCSeg];
     __shared__ float val[kCBand][32];
+    __shared__ unsigned short open_cells[kCBand * 32];  // band cells cepstrum_bin left open
+    __shared__ int n_open;
     const int per_type = tiles_x * tiles_y;
     const int t = blockIdx.x / per_type;
     const int tile = blockIdx.x - t * per_type;
@@ -167,6 +165,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
     const int nv = min(kCPer, i_end - i0 - ib);
     float* A = G.acc + t * n;
     const float* src = G.orient + t * n;
+    if (threadIdx.x == 0) n_open = 0;  // (the first sector's staging ends in a barrier)
     float o[kCPer];
 #pragma unroll
     for (int k = 0; k < kCPer; k++) {
@@ -191,14 +190,35 @@ __global__ void __launch_bounds__(kCThreads, 2)
             seg[rr][u] = v;
         }
         __syncthreads();
-        // Cepstrum of every valid band cell: warp = band row, lane = column.
+        // Bin of every valid band cell: warp = band row, lane = column.
         for (int rr = ty; rr < nrows; rr += kCThreads / 32) {
             const int r = r0 + rr;
+            const bool valid = r < d.H && j >= rfirst[r] && j < rlast[r];
             float v = 0.0f;
-            if (r < d.H && j >= rfirst[r] && j < rlast[r]) v = cepstrum_f32(&seg[rr][tx]);
+            bool open = false;
+            if (valid) {
+                const bool full = j - 32 >= rfirst[r] && j + 32 <= rlast[r];
+                const float bin = cepstrum_bin<true>(&seg[rr][tx], full ? seg[rr][tx + 32] : 0.0f);
+                open = bin < 0.0f;
+                v = __fmaf_rn(1000.0f, bin, 500.0f);
+            }
             val[rr][tx] = v;
+            const unsigned m = __ballot_sync(0xffffffffu, open);
+            if (m) {
+                int at = 0;
+                if (tx == 0) at = atomicAdd(&n_open, __popc(m));
+                at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << tx) - 1u));
+                if (open) open_cells[at] = (unsigned short)(rr * 32 + tx);
+            }
         }
         __syncthreads();
+        // The open cells, a thread each: the value itself.
+        for (int k = threadIdx.x; k < n_open; k += kCThreads) {
+            const int rr = open_cells[k] >> 5, x = open_cells[k] & 31;
+            val[rr][x] = cepstrum_f32(&seg[rr][x]);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) n_open = 0;  // counted again after the barrier below
         if (col_ok && nv > 0) {
             const int off = tg[j] - tmin;
 #pragma unroll
