@@ -17,7 +17,14 @@
 // the exact operator is measured and stated, and the exact operator stays the
 // parity mode.
 //
-// Fusion: a CTA owns a 128 x 32 tile of one orientation's accumulator of one
+// Most cells never run it: only the 1000-wide bin of a value is deskewed, and
+// cepstrum_bin (cepstrum_bin.cuh) arrives at it with half the operations wherever
+// its bound and this evaluation's leave no doubt; the cells they leave open (a few
+// in a hundred) are listed and take this one, a thread each.  The same bits:
+// 90.1 ms for 16 images of 512 x 512 with every cell here, 46.5 so, 40.3 with
+// 256-row tiles (1.13 cepstra per skewed cell, 128-row tiles form 1.27).
+//
+// Fusion: a CTA owns a 256 x 32 tile of one orientation's accumulator of one
 // image and walks that orientation's sectors in angle order.  Per sector it
 // gathers the skewed rows the tile needs (the reference's skew, gathered from
 // the orientation: skew_gather) as 96-cell row segments into shared memory,
@@ -31,11 +38,12 @@ namespace ske {
 
 namespace {
 
-constexpr int kCRows = 128;            // accumulator tile rows
+constexpr int kCRows = 256;            // accumulator tile rows
 constexpr int kCBand = kCRows + 34;    // skewed rows of a tile per sector (drift <= 32 over 32 columns)
 constexpr int kCSeg = 96;              // staged cells per band row: columns j0-32 .. j0+63
-constexpr int kCThreads = 256;
-constexpr int kCPer = kCRows / 8;      // accumulator rows per thread
+constexpr int kCThreads = 512;
+constexpr int kCWarps = kCThreads / 32;
+constexpr int kCPer = kCRows / kCWarps;  // accumulator rows per thread
 
 // W64^k = exp(-2 pi i k / 64) as float (cos, -sin), filled on the host.
 __constant__ float2 c_w64[64];
@@ -141,13 +149,20 @@ __device__ __forceinline__ float cepstrum_f32(const float* __restrict__ w) {
     return __fmul_rn(best, 10000.0f);
 }
 
+struct CSmem {
+    float seg[kCBand][kCSeg];
+    float val[kCBand][32];
+    unsigned short open_cells[kCBand * 32];  // band cells cepstrum_bin left open
+    int n_open;
+};
+
 // One launch: blockIdx.y = image; blockIdx.x = (type, tile row, tile column).
-__global__ void __launch_bounds__(kCThreads, 2)
+__global__ void __launch_bounds__(kCThreads, 1)
     k_cepstrum_fused(BatchTables T, DevGeometry g, TypeLists tl, int dim, int tiles_x, int tiles_y) {
-    __shared__ float seg[kCBand][kCSeg];
-    __shared__ float val[kCBand][32];
-    __shared__ unsigned short open_cells[kCBand * 32];  // band cells cepstrum_bin left open
-    __shared__ int n_open;
+    extern __shared__ __align__(16) unsigned char smem_c[];
+    CSmem& sm = *reinterpret_cast<CSmem*>(smem_c);
+    float(*seg)[kCSeg] = sm.seg;
+    float(*val)[32] = sm.val;
     const int per_type = tiles_x * tiles_y;
     const int t = blockIdx.x / per_type;
     const int tile = blockIdx.x - t * per_type;
@@ -165,7 +180,7 @@ __global__ void __launch_bounds__(kCThreads, 2)
     const int nv = min(kCPer, i_end - i0 - ib);
     float* A = G.acc + t * n;
     const float* src = G.orient + t * n;
-    if (threadIdx.x == 0) n_open = 0;  // (the first sector's staging ends in a barrier)
+    if (threadIdx.x == 0) sm.n_open = 0;  // (the first sector's staging ends in a barrier)
     float o[kCPer];
 #pragma unroll
     for (int k = 0; k < kCPer; k++) {
@@ -182,16 +197,36 @@ __global__ void __launch_bounds__(kCThreads, 2)
         const int r0 = i0 + tmin;
         const int nrows = (i_end - i0) + 1 + (tmax - tmin);  // <= kCBand for square grids
         // Stage the band's row segments (skewed cells gathered from the orientation).
-        for (int idx = threadIdx.x; idx < nrows * kCSeg; idx += kCThreads) {
-            const int rr = idx / kCSeg, u = idx - rr * kCSeg;
-            const int r = r0 + rr, x = j0 - 32 + u;
-            float v = 0.0f;
-            if (r < d.H && x >= rfirst[r] && x < rlast[r]) v = skew_gather(d, tg, wg, src, r, x);
-            seg[rr][u] = v;
+        // A warp per row, three columns per lane whose shifts and weights stay in
+        // registers.
+        int tc[kCSeg / 32];
+        float wc[kCSeg / 32];
+#pragma unroll
+        for (int k = 0; k < kCSeg / 32; k++) {
+            const int x = j0 - 32 + tx + 32 * k, xc = min(max(x, 0), dim - 1);
+            tc[k] = tg[xc];
+            wc[k] = wg[xc];
+        }
+#pragma unroll 4
+        for (int rr = ty; rr < nrows; rr += kCWarps) {
+            const int r = r0 + rr;
+            const int f = r < d.H ? rfirst[r] : 0, l = r < d.H ? rlast[r] : 0;
+#pragma unroll
+            for (int k = 0; k < kCSeg / 32; k++) {
+                const int x = j0 - 32 + tx + 32 * k, i = r - tc[k] - 1;
+                const bool in = x >= f && x < l;
+                const bool v0 = in && (unsigned)i < (unsigned)d.dim_o, v1 = in && (unsigned)(i + 1) < (unsigned)d.dim_o;
+                const float* p0 = src + ((int64_t)i * d.dim_i + x);
+                const float a = v0 ? p0[0] : 0.0f, e = v1 ? p0[d.dim_i] : 0.0f;
+                float acc = 0.0f;  // as skew_gather
+                acc = v0 ? __fadd_rn(acc, __fmul_rn(wc[k], a)) : acc;
+                acc = v1 ? __fadd_rn(acc, __fmul_rn(__fsub_rn(1.0f, wc[k]), e)) : acc;
+                seg[rr][tx + 32 * k] = acc;
+            }
         }
         __syncthreads();
         // Bin of every valid band cell: warp = band row, lane = column.
-        for (int rr = ty; rr < nrows; rr += kCThreads / 32) {
+        for (int rr = ty; rr < nrows; rr += kCWarps) {
             const int r = r0 + rr;
             const bool valid = r < d.H && j >= rfirst[r] && j < rlast[r];
             float v = 0.0f;
@@ -206,19 +241,19 @@ __global__ void __launch_bounds__(kCThreads, 2)
             const unsigned m = __ballot_sync(0xffffffffu, open);
             if (m) {
                 int at = 0;
-                if (tx == 0) at = atomicAdd(&n_open, __popc(m));
+                if (tx == 0) at = atomicAdd(&sm.n_open, __popc(m));
                 at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << tx) - 1u));
-                if (open) open_cells[at] = (unsigned short)(rr * 32 + tx);
+                if (open) sm.open_cells[at] = (unsigned short)(rr * 32 + tx);
             }
         }
         __syncthreads();
         // The open cells, a thread each: the value itself.
-        for (int k = threadIdx.x; k < n_open; k += kCThreads) {
-            const int rr = open_cells[k] >> 5, x = open_cells[k] & 31;
+        for (int k = threadIdx.x; k < sm.n_open; k += kCThreads) {
+            const int rr = sm.open_cells[k] >> 5, x = sm.open_cells[k] & 31;
             val[rr][x] = cepstrum_f32(&seg[rr][x]);
         }
         __syncthreads();
-        if (threadIdx.x == 0) n_open = 0;  // counted again after the barrier below
+        if (threadIdx.x == 0) sm.n_open = 0;  // counted again after the barrier below
         if (col_ok && nv > 0) {
             const int off = tg[j] - tmin;
 #pragma unroll
@@ -258,7 +293,10 @@ cudaError_t launch_cepstrum_f32(const BatchTables& t, int images, const DevGeome
     const int tiles_x = (dim + 31) / 32, tiles_y = (dim + kCRows - 1) / kCRows;
     const int64_t blocks = (int64_t)4 * tiles_x * tiles_y;
     if (blocks > 0x7fffffff || images > 65535) return cudaErrorInvalidValue;
-    k_cepstrum_fused<<<dim3((unsigned)blocks, (unsigned)images), kCThreads, 0, st>>>(t, g, tl, dim, tiles_x, tiles_y);
+    const int smem = (int)sizeof(CSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_cepstrum_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_cepstrum_fused<<<dim3((unsigned)blocks, (unsigned)images), kCThreads, smem, st>>>(t, g, tl, dim, tiles_x, tiles_y);
     return cudaGetLastError();
 }
 
