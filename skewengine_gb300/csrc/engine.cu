@@ -438,7 +438,7 @@ int tune_sweep(ske_engine e, const SdemLaunch& base, const std::vector<uint64_t>
     SKE_CK(cudaMemcpyAsync(e->d_tune_items, sample.data(), sizeof(uint64_t) * sample.size(), cudaMemcpyHostToDevice,
                            e->stream));
     const int max_ctas = sdem_max_ctas_per_sm(base);
-    const SweepShape sched[] = {{64, 0, 0}, {16, 48, 0}, {32, 0, 0}, {48, 0, 0}};
+    const SweepShape sched[] = {{64, 0, 0}, {16, 48, 0}, {32, 0, 0}, {32, 32, 0}};
     std::vector<SweepShape> cands;
     for (const SweepShape& c : sched) {
         cands.push_back(c);

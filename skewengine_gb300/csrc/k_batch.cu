@@ -1,6 +1,6 @@
 // Batched runs over grids of uneven size: one launch each for the orientations,
 // the skew, the deskew and the fold of every sector of every grid of a wave
-// (the sweep runs in between, k_sdem.cu).  The reference runs one grid per
+// (the sweep runs in between, k_sweep.cu).  The reference runs one grid per
 // program and its sectors one at a time per thread (src/main.cu:86-168); here
 // a wave's sectors of all grids form one work list.
 //

@@ -178,7 +178,7 @@ int64_t batch_prep_blocks(int dimx, int dimy);
 int64_t batch_deskew_tiles(int dimx, int dimy, int t);
 
 // --- operators ------------------------------------------------------------
-// Total viewshed sweep (k_sdem.cu).  items: sorted work list (see sdem_items).
+// Total viewshed sweeps (k_sweep.cu, k_sdem.cu).  items: sorted work list (see sdem_items).
 struct SdemLaunch {
     DevGeometry g;
     Batch b;
@@ -277,8 +277,9 @@ cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const flo
                                  int64_t len, int max_H, int max_cols, const double* tw64, const double* tw32,
                                  cudaStream_t st);
 
-// Constant tables used by the SDEM sweep, uploaded once per device.
-cudaError_t sdem_init_tables();
+// Constant tables used by the SDEM sweeps, uploaded once per device.
+cudaError_t sdem_init_tables();   // both sweeps'
+cudaError_t sweep_init_tables();  // the compacting sweep's
 
 // Record `msg` as the calling thread's last error (ske_last_error) and return code.
 int set_last_error(int code, const char* msg);
