@@ -15,8 +15,16 @@
 //    the logarithm itself by 2^-22 max(1, |log2|); log |X_n|^2 + log |X_{32-n}|^2
 //    is the logarithm of the product, 17 logarithms instead of 32.
 //  * Scaling X by a constant only moves c_0, which nothing reads.
+//  * 1 / |X_n|^2 + 1 / |X_{32-n}|^2 is their sum times the reciprocal of their
+//    product, whose logarithm is formed anyway; |window|^2 comes from the spectrum
+//    (Parseval), off by 10^-5 of itself against the 2 10^-3 the bound has to spare.
+//  * A thread evaluates two windows in the halves of f32x2 registers, from samples
+//    staged as such pairs: the transform and the sums take half the instructions
+//    (650 a cell against 1290).  What is left to the FMA pipe is the same, and it
+//    is the bound now (f32x2 occupies it for two cycles).
 //  * c_4 .. c_15 are cosine sums folded over n, 16 - n and 8 - n: 62
-//    multiply-adds; their roundings stay below 14 u times the sum of the logs.
+//    multiply-adds; their roundings stay below 14 u times the sum of the logs, at most 17
+//    times the largest.
 //  * The search is repeated for every sample that could be the first ascent;
 //    the cell is decided when all of them land in one bin with the bound to
 //    spare.
@@ -27,6 +35,7 @@
 //    room for both errors is the bin it arrives at.
 #pragma once
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace ske {
@@ -44,10 +53,32 @@ __device__ __forceinline__ constexpr int brev5(int v) {
     return ((v & 1) << 4) | ((v & 2) << 2) | (v & 4) | ((v & 8) >> 2) | ((v & 16) >> 4);
 }
 
-// 32-point complex FFT in registers, radix-2 decimation in time: input in
-// bit-reversed order, output in natural order.  A butterfly's sum takes four
-// fused operations and its difference 2a - sum two.
-__device__ __forceinline__ void fft32_fused(float (&re)[32], float (&im)[32]) {
+// The same constant in both halves.
+__device__ __forceinline__ f2 both(float c) { return pk(c, c); }
+
+// A packed pair stored as itself or as its negative (neg, known at compile time
+// once the loops are unrolled): f32x2 operations take no negated operands, and a
+// sign that only moves on to the next constant or from an addition to a
+// subtraction costs nothing.
+struct Signed {
+    f2 v;
+    bool neg;
+};
+__device__ __forceinline__ Signed operator-(Signed a) { return {a.v, !a.neg}; }
+__device__ __forceinline__ Signed operator+(Signed a, Signed b) {
+    if (a.neg == b.neg) return {add2(a.v, b.v), a.neg};
+    return a.neg ? Signed{sub2(b.v, a.v), false} : Signed{sub2(a.v, b.v), false};
+}
+__device__ __forceinline__ Signed operator-(Signed a, Signed b) { return a + -b; }
+// acc + x * c.
+__device__ __forceinline__ Signed mad(Signed x, float c, Signed acc) {
+    return {fma2(x.v, both(x.neg == acc.neg ? c : -c), acc.v), acc.neg};
+}
+
+// 32-point complex FFT in registers of two windows at a time, radix-2 decimation
+// in time: input in bit-reversed order, output in natural order.  A butterfly's
+// sum takes four fused operations and its difference 2a - sum two.
+__device__ __forceinline__ void fft32_fused(Signed (&re)[32], Signed (&im)[32]) {
 #pragma unroll
     for (int span = 1; span < 32; span <<= 1) {
 #pragma unroll
@@ -55,23 +86,23 @@ __device__ __forceinline__ void fft32_fused(float (&re)[32], float (&im)[32]) {
 #pragma unroll
             for (int k = 0; k < span; k++) {
                 const int a = start + k, b = a + span;
-                const float ar = re[a], ai = im[a], br = re[b], bi = im[b];
+                const Signed ar = re[a], ai = im[a], br = re[b], bi = im[b];
                 if (k == 0) {
-                    re[a] = __fadd_rn(ar, br);
-                    im[a] = __fadd_rn(ai, bi);
-                    re[b] = __fsub_rn(ar, br);
-                    im[b] = __fsub_rn(ai, bi);
+                    re[a] = ar + br;
+                    im[a] = ai + bi;
+                    re[b] = ar - br;
+                    im[b] = ai - bi;
                 } else if (2 * k == span) {  // twiddle -i
-                    re[a] = __fadd_rn(ar, bi);
-                    im[a] = __fsub_rn(ai, br);
-                    re[b] = __fsub_rn(ar, bi);
-                    im[b] = __fadd_rn(ai, br);
+                    re[a] = ar + bi;
+                    im[a] = ai - br;
+                    re[b] = ar - bi;
+                    im[b] = ai + br;
                 } else {
                     const float c = cos64(k * (32 / span)), s = sin64(k * (32 / span));  // twiddle c - i s
-                    re[a] = __fmaf_rn(br, c, __fmaf_rn(bi, s, ar));
-                    im[a] = __fmaf_rn(bi, c, __fmaf_rn(br, -s, ai));
-                    re[b] = __fmaf_rn(2.0f, ar, -re[a]);
-                    im[b] = __fmaf_rn(2.0f, ai, -im[a]);
+                    re[a] = mad(br, c, mad(bi, s, ar));
+                    im[a] = mad(bi, c, mad(br, -s, ai));
+                    re[b] = -mad(ar, -2.0f, re[a]);
+                    im[b] = -mad(ai, -2.0f, im[a]);
                 }
             }
         }
@@ -89,88 +120,14 @@ __device__ __forceinline__ float rcp(float x) {
     return y;
 }
 
-// The bin of the 64-sample window w[0..63], or -1 where float leaves it open.
-// mean: the window's centre sample where every sample lies inside the row, else 0.
-// kPlain: the bin cepstrum_f32 (k_cepstrum_f32.cu) arrives at, not the reference's.
+// The search for one window: its bin, or -1 where float leaves it open.
+// c: its c_4 .. c_15.  l2, inv, emax: |window|^2, the sum of 1 / |2 X_n|^2 and the
+// largest of the logarithms' magnitudes.
 template <bool kPlain>
-__device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float mean) {
+__device__ __forceinline__ float cepstrum_decide(const float (&c)[16], float l2, float inv, float emax, float mean) {
     constexpr float u = 5.9604644775390625e-8f;  // 2^-24
-    float re[32], im[32], l2 = 0.0f;
-#pragma unroll
-    for (int n = 0; n < 32; n++) {  // z_n = w[2n] + i w[2n+1], stored bit-reversed
-        const float a = __fsub_rn(w[2 * n], mean), c = __fsub_rn(w[2 * n + 1], mean);
-        re[brev5(n)] = a;
-        im[brev5(n)] = c;
-        l2 = __fmaf_rn(a, a, l2);
-        l2 = __fmaf_rn(c, c, l2);
-    }
-    fft32_fused(re, im);
-    // 2 X_k = E + W64^k O, E = Z_k + conj Z_{32-k}, O = -i (Z_k - conj Z_{32-k});
-    // 2 X_{32-k} = conj(E - W64^k O).  e[n] = log2 |2 X_n|^2 |2 X_{32-n}|^2, inv =
-    // sum of 1 / |2 X_n|^2, all: of the logs' magnitudes.
-    float e[17], inv = 0.0f, all = 0.0f;
-    {
-        const float x0 = __fmaf_rn(128.0f, mean, __fmul_rn(2.0f, __fadd_rn(re[0], im[0])));
-        const float p0 = __fmul_rn(x0, x0);
-        const float p16 = __fmul_rn(4.0f, __fmaf_rn(re[16], re[16], __fmul_rn(im[16], im[16])));
-        e[0] = lg2(p0);
-        e[16] = lg2(p16);
-        inv = rcp(p0) + rcp(p16);
-        all = fabsf(e[0]) + fabsf(e[16]);
-    }
-#pragma unroll
-    for (int k = 1; k < 16; k++) {
-        const int m = 32 - k;
-        const float er = __fadd_rn(re[k], re[m]), ei = __fsub_rn(im[k], im[m]);
-        const float orr = __fadd_rn(im[k], im[m]), oi = __fsub_rn(re[m], re[k]);
-        const float c = cos64(k), s = sin64(k);
-        const float ur = __fmaf_rn(orr, c, __fmaf_rn(oi, s, er)), ui = __fmaf_rn(oi, c, __fmaf_rn(orr, -s, ei));
-        const float vr = __fmaf_rn(2.0f, er, -ur), vi = __fmaf_rn(2.0f, ei, -ui);
-        const float pk = __fmaf_rn(ur, ur, __fmul_rn(ui, ui)), pm = __fmaf_rn(vr, vr, __fmul_rn(vi, vi));
-        e[k] = lg2(__fmul_rn(pk, pm));
-        inv += rcp(pk);
-        inv += rcp(pm);
-        all += fabsf(e[k]);
-    }
-    // T_k = e_0 + (-1)^k e_16 + sum over 0 < n < 16 of e_n cos(2 pi k n / 32); c_k = T_k ln 2 / sqrt(32).
-    constexpr float kScale = 0.12253274f;
-    float c[16];
-    float f[8], o[8];
-#pragma unroll
-    for (int n = 1; n < 8; n++) {
-        f[n] = __fadd_rn(e[n], e[16 - n]);
-        o[n] = __fsub_rn(e[n], e[16 - n]);
-    }
-    const float odd = __fsub_rn(e[0], e[16]), sum = __fadd_rn(e[0], e[16]);
-    const float ev = __fadd_rn(sum, e[8]), eo = __fsub_rn(sum, e[8]);
-#pragma unroll
-    for (int k = 5; k < 16; k += 2) {
-        float acc = odd;
-#pragma unroll
-        for (int n = 1; n < 8; n++) acc = __fmaf_rn(o[n], cos64(2 * k * n), acc);
-        c[k] = acc;
-    }
-    float g[4], h[4];
-#pragma unroll
-    for (int n = 1; n < 4; n++) {
-        g[n] = __fadd_rn(f[n], f[8 - n]);
-        h[n] = __fsub_rn(f[n], f[8 - n]);
-    }
-#pragma unroll
-    for (int k = 6; k < 16; k += 4) {
-        float acc = eo;
-#pragma unroll
-        for (int n = 1; n < 4; n++) acc = __fmaf_rn(h[n], cos64(2 * k * n), acc);
-        c[k] = acc;
-    }
-#pragma unroll
-    for (int k = 4; k < 16; k += 4) {
-        float acc = k == 8 ? __fadd_rn(ev, f[4]) : __fsub_rn(ev, f[4]);
-#pragma unroll
-        for (int n = 1; n < 4; n++) acc = __fmaf_rn(g[n], cos64(2 * k * n), acc);
-        c[k] = acc;
-    }
     // The bound of every c_k: 0.17678 = 1 / sqrt(32); 2 X is off by 480 u |window|.
+    const float all = 17.0f * emax;  // bounds the sum of the logs' magnitudes
     const float dx = 481.0f * u * sqrtf(l2 * inv);
     float err = 0.17678f * (2.2f * dx + 0.7f * (4.0f * u * (17.0f + all) + 14.0f * u * all)) + 100.0f * u;
     float far = dx;
@@ -183,10 +140,7 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
     }
     float s[16], top = 0.0f;
 #pragma unroll
-    for (int k = 15; k >= 4; k--) {
-        c[k] = __fmul_rn(c[k], kScale);
-        s[k] = fmaxf(-c[k], 0.0f);
-    }
+    for (int k = 15; k >= 4; k--) s[k] = fmaxf(-c[k], 0.0f);
     // Samples after i: top.  Every sample i that may be the first ascent gives
     // the result max(s_{i-1}, top_i); lo and hi span those up to the first that
     // must be one (going down: a sure ascent discards what lies after it).
@@ -202,8 +156,114 @@ __device__ __forceinline__ float cepstrum_bin(const float* __restrict__ w, float
     }
     const float slack = err + 8.0f * u * hi;
     const float b0 = floorf(10.0f * fmaxf(lo - slack, 0.0f)), b1 = floorf(10.0f * (hi + slack));
-    const bool sure = b0 == b1 && far < 0.05f && all < 1e4f && l2 > 1e-20f && l2 < 1e24f;
+    // Logarithms below 126: no product |2 X_n|^2 |2 X_{32-n}|^2 and no reciprocal left the float range.
+    const bool sure = b0 == b1 && far < 0.05f && emax < 126.0f && l2 > 1e-20f && l2 < 1e24f;
     return sure ? b0 : -1.0f;
+}
+
+// The bins of two 64-sample windows, the halves of w[0..63], or -1 where float
+// leaves one open.  mean: each window's centre sample where all of its samples lie
+// inside its row, else 0.
+// kPlain: the bin cepstrum_f32 (k_cepstrum_f32.cu) arrives at, not the reference's.
+template <bool kPlain>
+__device__ __forceinline__ float2 cepstrum_bin(const f2* __restrict__ w, f2 mean) {
+    Signed re[32], im[32];
+#pragma unroll
+    for (int n = 0; n < 32; n++) {  // z_n = w[2n] + i w[2n+1], stored bit-reversed
+        re[brev5(n)] = {sub2(w[2 * n], mean), false};
+        im[brev5(n)] = {sub2(w[2 * n + 1], mean), false};
+    }
+    fft32_fused(re, im);
+    // 2 X_k = E + W64^k O, E = Z_k + conj Z_{32-k}, O = -i (Z_k - conj Z_{32-k});
+    // 2 X_{32-k} = conj(E - W64^k O).  e[n] = log2 |2 X_n|^2 |2 X_{32-n}|^2, inv =
+    // sum of 1 / |2 X_n|^2, e_max: the largest of the logs' magnitudes.
+    // Parseval: 256 |window|^2 = |2 X_0|^2 + |2 X_32|^2 + 2 sum over 0 < n < 32 of |2 X_n|^2, X_0 without the mean.
+    f2 e[17], inv, pw;
+    float e_max0, e_max1;
+    const f2 two = both(2.0f), four = both(4.0f);
+    {
+        const Signed z0 = re[0] + im[0];
+        const f2 y0 = mul2(both(z0.neg ? -2.0f : 2.0f), z0.v), y32 = mul2(two, (re[0] - im[0]).v);
+        const f2 x0 = fma2(both(128.0f), mean, y0);
+        const f2 p0 = mul2(x0, x0);
+        const f2 p16 = mul2(four, fma2(re[16].v, re[16].v, mul2(im[16].v, im[16].v)));
+        float a, b, c, d;
+        upk(p0, a, b);
+        upk(p16, c, d);
+        inv = pk(rcp(a) + rcp(c), rcp(b) + rcp(d));
+        a = lg2(a), b = lg2(b), c = lg2(c), d = lg2(d);
+        e[0] = pk(a, b);
+        e[16] = pk(c, d);
+        e_max0 = fmaxf(fabsf(a), fabsf(c));
+        e_max1 = fmaxf(fabsf(b), fabsf(d));
+        pw = fma2(two, p16, fma2(y0, y0, mul2(y32, y32)));
+    }
+#pragma unroll
+    for (int k = 1; k < 16; k++) {
+        const int m = 32 - k;
+        const Signed er = re[k] + re[m], ei = im[k] - im[m], orr = im[k] + im[m], oi = re[m] - re[k];
+        const float c = cos64(k), s = sin64(k);
+        const Signed ur = mad(orr, c, mad(oi, s, er)), ui = mad(oi, c, mad(orr, -s, ei));
+        const f2 vr = mad(er, -2.0f, ur).v, vi = mad(ei, -2.0f, ui).v;
+        const f2 pu = fma2(ur.v, ur.v, mul2(ui.v, ui.v)), pv = fma2(vr, vr, mul2(vi, vi));
+        const f2 prod = mul2(pu, pv), sum = add2(pu, pv);
+        float a, b;
+        upk(prod, a, b);
+        inv = fma2(sum, pk(rcp(a), rcp(b)), inv);  // 1 / pu + 1 / pv
+        a = lg2(a), b = lg2(b);
+        e[k] = pk(a, b);
+        e_max0 = fmaxf(e_max0, fabsf(a));
+        e_max1 = fmaxf(e_max1, fabsf(b));
+        pw = fma2(two, sum, pw);
+    }
+    // T_k = e_0 + (-1)^k e_16 + sum over 0 < n < 16 of e_n cos(2 pi k n / 32); c_k = T_k ln 2 / sqrt(32).
+    constexpr float kScale = 0.12253274f;
+    f2 c[16];
+    f2 f[8], o[8];
+#pragma unroll
+    for (int n = 1; n < 8; n++) {
+        f[n] = add2(e[n], e[16 - n]);
+        o[n] = sub2(e[n], e[16 - n]);
+    }
+    const f2 odd = sub2(e[0], e[16]), sum = add2(e[0], e[16]);
+    const f2 ev = add2(sum, e[8]), eo = sub2(sum, e[8]);
+#pragma unroll
+    for (int k = 5; k < 16; k += 2) {
+        f2 acc = odd;
+#pragma unroll
+        for (int n = 1; n < 8; n++) acc = fma2(o[n], both(cos64(2 * k * n)), acc);
+        c[k] = acc;
+    }
+    f2 g[4], h[4];
+#pragma unroll
+    for (int n = 1; n < 4; n++) {
+        g[n] = add2(f[n], f[8 - n]);
+        h[n] = sub2(f[n], f[8 - n]);
+    }
+#pragma unroll
+    for (int k = 6; k < 16; k += 4) {
+        f2 acc = eo;
+#pragma unroll
+        for (int n = 1; n < 4; n++) acc = fma2(h[n], both(cos64(2 * k * n)), acc);
+        c[k] = acc;
+    }
+#pragma unroll
+    for (int k = 4; k < 16; k += 4) {
+        f2 acc = k == 8 ? add2(ev, f[4]) : sub2(ev, f[4]);
+#pragma unroll
+        for (int n = 1; n < 4; n++) acc = fma2(g[n], both(cos64(2 * k * n)), acc);
+        c[k] = acc;
+    }
+    float c0[16], c1[16];
+#pragma unroll
+    for (int k = 4; k < 16; k++) upk(mul2(c[k], both(kScale)), c0[k], c1[k]);
+    const f2 l2 = mul2(pw, both(1.0f / 256.0f));
+    float l20, l21, inv0, inv1, m0, m1;
+    upk(l2, l20, l21);
+    upk(inv, inv0, inv1);
+    upk(mean, m0, m1);
+    return make_float2(cepstrum_decide<kPlain>(c0, l20, inv0, e_max0, m0),
+                       cepstrum_decide<kPlain>(c1, l21, inv1, e_max1, m1));
 }
 
 }  // namespace ske

@@ -20,10 +20,10 @@
 // GB300 does 1/64 as many binary64 as float operations, and the exact kernel
 // held a 512 x 512 image at the FP64 pipe's rate (353 ms for 180 angles, that
 // pipe 84% busy).  So the cepstrum is formed in float with a bound on its error
-// (one thread per cell, the window in registers), and only the cells whose bin
+// (a thread per two cells, the windows in registers), and only the cells whose bin
 // that leaves open run the exact kernel.  The whole run of a 512 x 512 texture
-// (180 angles): 353.3 ms with every cell in binary64, 3.20 ms so (the float
-// kernel 2.2, the open cells 0.6).
+// (180 angles): 353.3 ms with every cell in binary64, 2.86 ms so (the float
+// kernel 1.9, the open cells 0.6); 3.20 with a thread per cell.
 // cepstrum_bin.cuh has the evaluation and its bounds.
 #include "cepstrum_bin.cuh"
 
@@ -130,36 +130,53 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
 
 // ---- bins in float -------------------------------------------------------------
 
-// One warp per 32 consecutive valid cells of a skewed row.
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, 2)
+// Four CTAs of four warps, 128 registers: 1.86 ms; three, without the few spills,
+// 1.91.
+constexpr int kBinWarps = 4;
+
+// One warp per 32 columns of two skewed rows, the upper and lower half of the pair
+// that a lane holds.
+__global__ void __launch_bounds__(kBinWarps * 32, 4)
     k_cepstrum_bins(DevGeometry g, Batch b, const float* __restrict__ SI, float* __restrict__ SO, int64_t stride,
                     int col_blocks) {
-    __shared__ float seg[kWarpsPerBlock][32 + kWin];
+    __shared__ f2 seg[kBinWarps][32 + kWin];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slot = blockIdx.y;
     const SectorDesc& d = g.desc[b.angle[slot]];
-    const int unit = blockIdx.x * kWarpsPerBlock + warp;
-    const int r = unit / col_blocks;
+    const int unit = blockIdx.x * kBinWarps + warp;
+    const int r = 2 * (unit / col_blocks);
     if (r >= d.H) return;
+    const bool two = r + 1 < d.H;
     const int32_t* first = g.first + d.row_off;
     const int32_t* last = g.last + d.row_off;
-    const int f = first[r], l = last[r];
-    const int j0 = f + (unit % col_blocks) * 32;
-    if (j0 >= l) return;  // warp-uniform
+    const int f0 = first[r], l0 = last[r];
+    const int f1 = two ? first[r + 1] : f0, l1 = two ? last[r + 1] : f0;
     const int64_t base = (int64_t)r * d.dim_i;
     const float* in = SI + slot * stride + base;
-    float* sw = seg[warp];
+    f2* sw = seg[warp];
+    // (Two rows together may span more columns than the longest one.)
+    for (int j0 = min(f0, f1) + (unit % col_blocks) * 32; j0 < max(l0, l1); j0 += col_blocks * 32) {
+        __syncwarp();
 #pragma unroll
-    for (int t = 0; t < 3; t++) {
-        const int x = j0 - kWin / 2 + lane + 32 * t;
-        sw[lane + 32 * t] = x >= f && x < l ? in[x] : 0.0f;
+        for (int t = 0; t < 3; t++) {
+            const int x = j0 - kWin / 2 + lane + 32 * t;
+            sw[lane + 32 * t] = pk(x >= f0 && x < l0 ? in[x] : 0.0f, x >= f1 && x < l1 ? in[x + d.dim_i] : 0.0f);
+        }
+        __syncwarp();
+        const int j = j0 + lane;
+        const bool own0 = j >= f0 && j < l0 && (j < d.dim_i || owner_row(d, first, last, base + j) == r);
+        const bool own1 =
+            j >= f1 && j < l1 && (j < d.dim_i || owner_row(d, first, last, base + d.dim_i + j) == r + 1);
+        if (!own0 && !own1) continue;
+        float m0, m1;
+        upk(sw[lane + kWin / 2], m0, m1);
+        const f2 mean = pk(j - kWin / 2 >= f0 && j + kWin / 2 <= l0 ? m0 : 0.0f,
+                           j - kWin / 2 >= f1 && j + kWin / 2 <= l1 ? m1 : 0.0f);
+        const float2 bin = cepstrum_bin<false>(sw + lane, mean);
+        float* out = SO + slot * stride + base + j;
+        if (own0) out[0] = bin.x >= 0.0f ? __fmaf_rn(1000.0f, bin.x, 500.0f) : kOpen;
+        if (own1) out[d.dim_i] = bin.y >= 0.0f ? __fmaf_rn(1000.0f, bin.y, 500.0f) : kOpen;
     }
-    __syncwarp();
-    const int j = j0 + lane;
-    if (j >= l || (j >= d.dim_i && owner_row(d, first, last, base + j) != r)) return;
-    const bool full = j - kWin / 2 >= f && j + kWin / 2 <= l;
-    const float bin = cepstrum_bin<false>(sw + lane, full ? sw[lane + kWin / 2] : 0.0f);
-    SO[slot * stride + base + j] = bin >= 0.0f ? __fmaf_rn(1000.0f, bin, 500.0f) : kOpen;
 }
 
 }  // namespace
@@ -177,9 +194,9 @@ cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const flo
                                  int64_t len, int max_H, int max_cols, const double* tw64, const double* tw32,
                                  cudaStream_t st) {
     const int col_blocks = (max_cols + 31) / 32;
-    const int64_t units = (int64_t)max_H * col_blocks;
-    k_cepstrum_bins<<<dim3((unsigned)((units + kWarpsPerBlock - 1) / kWarpsPerBlock), b.count), kWarpsPerBlock * 32, 0,
-                      st>>>(g, b, SI, SO, stride, col_blocks);
+    const int64_t units = (int64_t)((max_H + 1) / 2) * col_blocks;
+    k_cepstrum_bins<<<dim3((unsigned)((units + kBinWarps - 1) / kBinWarps), b.count), kBinWarps * 32, 0, st>>>(
+        g, b, SI, SO, stride, col_blocks);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     int64_t blocks = (len + kWarpsPerBlock * 32 - 1) / (kWarpsPerBlock * 32);

@@ -22,15 +22,17 @@
 // its bound and this evaluation's leave no doubt; the cells they leave open (a few
 // in a hundred) are listed and take this one, a thread each.  The same bits:
 // 90.1 ms for 16 images of 512 x 512 with every cell here, 46.5 so, 40.3 with
-// 256-row tiles (1.13 cepstra per skewed cell, 128-row tiles form 1.27).
+// 256-row tiles (1.13 cepstra per skewed cell, 128-row tiles form 1.27), 34.7
+// with two cells to a thread (16 warps of 128 registers; 12 of 168 take 35.9, 8
+// of 188 41.7).
 //
 // Fusion: a CTA owns a 256 x 32 tile of one orientation's accumulator of one
 // image and walks that orientation's sectors in angle order.  Per sector it
 // gathers the skewed rows the tile needs (the reference's skew, gathered from
 // the orientation: skew_gather) as 96-cell row segments into shared memory,
-// computes the cepstrum of every band cell (one thread per cell, the 64-cell
-// window read from the staged segment), and max-deskews into the tile's
-// registers.  The skewed input and output never reach HBM; the orientations
+// computes the cepstrum of every band cell (a thread per two rows' cells, the
+// 64-cell windows read from the staged segments), and max-deskews into the tile's
+// accumulator in shared memory.  The skewed input and output never reach HBM; the orientations
 // (4 x N floats per image) stay L2-resident.
 #include "cepstrum_bin.cuh"
 
@@ -43,7 +45,6 @@ constexpr int kCBand = kCRows + 34;    // skewed rows of a tile per sector (drif
 constexpr int kCSeg = 96;              // staged cells per band row: columns j0-32 .. j0+63
 constexpr int kCThreads = 512;
 constexpr int kCWarps = kCThreads / 32;
-constexpr int kCPer = kCRows / kCWarps;  // accumulator rows per thread
 
 // W64^k = exp(-2 pi i k / 64) as float (cos, -sin), filled on the host.
 __constant__ float2 c_w64[64];
@@ -81,13 +82,13 @@ __device__ __forceinline__ void fft32(float (&re)[32], float (&im)[32]) {
 }
 
 // Cepstrum peak of the 64-sample window w[0..63] (zeros outside the row), as
-// lineCepstrum computes it, in float32.
+// lineCepstrum computes it, in float32.  w: its samples, two floats apart.
 __device__ __forceinline__ float cepstrum_f32(const float* __restrict__ w) {
     float re[32], im[32];
 #pragma unroll
     for (int n = 0; n < 32; n++) {  // z_n = w[2n] + i w[2n+1], stored bit-reversed
-        re[brev5(n)] = w[2 * n];
-        im[brev5(n)] = w[2 * n + 1];
+        re[brev5(n)] = w[4 * n];
+        im[brev5(n)] = w[4 * n + 2];
     }
     fft32(re, im);
     // X_k = E_k + W64^k O_k, E = (Z_k + conj Z_{32-k}) / 2, O = -i (Z_k - conj Z_{32-k}) / 2;
@@ -150,8 +151,9 @@ __device__ __forceinline__ float cepstrum_f32(const float* __restrict__ w) {
 }
 
 struct CSmem {
-    float seg[kCBand][kCSeg];
+    f2 seg[kCBand / 2][kCSeg];  // two band rows in the halves
     float val[kCBand][32];
+    float acc[kCRows][32];  // the tile's accumulator
     unsigned short open_cells[kCBand * 32];  // band cells cepstrum_bin left open
     int n_open;
 };
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
     k_cepstrum_fused(BatchTables T, DevGeometry g, TypeLists tl, int dim, int tiles_x, int tiles_y) {
     extern __shared__ __align__(16) unsigned char smem_c[];
     CSmem& sm = *reinterpret_cast<CSmem*>(smem_c);
-    float(*seg)[kCSeg] = sm.seg;
+    f2(*seg)[kCSeg] = sm.seg;
     float(*val)[32] = sm.val;
     const int per_type = tiles_x * tiles_y;
     const int t = blockIdx.x / per_type;
@@ -176,17 +178,12 @@ __global__ void __launch_bounds__(kCThreads, 1)
     const bool col_ok = j < dim;
     const int jlast = min(j0 + 32, dim) - 1;
     const int i_end = min(i0 + kCRows, dim);
-    const int ib = ty * kCPer;
-    const int nv = min(kCPer, i_end - i0 - ib);
+    const int ni = i_end - i0;
     float* A = G.acc + t * n;
     const float* src = G.orient + t * n;
     if (threadIdx.x == 0) sm.n_open = 0;  // (the first sector's staging ends in a barrier)
-    float o[kCPer];
-#pragma unroll
-    for (int k = 0; k < kCPer; k++) {
-        const int i = i0 + ib + k;
-        o[k] = (col_ok && i < i_end) ? A[(int64_t)i * dim + j] : 0.0f;
-    }
+    if (col_ok)
+        for (int i = ty; i < ni; i += kCWarps) sm.acc[i][tx] = A[(int64_t)(i0 + i) * dim + j];
     for (int q = 0; q < cnt; q++) {
         const SectorDesc d = g.desc[tl.angle[t][q]];
         const int32_t* tg = g.target + d.col_off;
@@ -195,7 +192,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
         const int32_t* rlast = g.last + d.row_off;
         const int tmin = tg[j0], tmax = tg[jlast];
         const int r0 = i0 + tmin;
-        const int nrows = (i_end - i0) + 1 + (tmax - tmin);  // <= kCBand for square grids
+        const int nrows = ni + 1 + (tmax - tmin);  // <= kCBand for square grids
         // Stage the band's row segments (skewed cells gathered from the orientation).
         // A warp per row, three columns per lane whose shifts and weights stay in
         // registers.
@@ -207,73 +204,85 @@ __global__ void __launch_bounds__(kCThreads, 1)
             tc[k] = tg[xc];
             wc[k] = wg[xc];
         }
-#pragma unroll 4
-        for (int rr = ty; rr < nrows; rr += kCWarps) {
-            const int r = r0 + rr;
-            const int f = r < d.H ? rfirst[r] : 0, l = r < d.H ? rlast[r] : 0;
+#pragma unroll 2
+        for (int p = ty; 2 * p < nrows; p += kCWarps) {
+            float cell[2][kCSeg / 32];
 #pragma unroll
-            for (int k = 0; k < kCSeg / 32; k++) {
-                const int x = j0 - 32 + tx + 32 * k, i = r - tc[k] - 1;
-                const bool in = x >= f && x < l;
-                const bool v0 = in && (unsigned)i < (unsigned)d.dim_o, v1 = in && (unsigned)(i + 1) < (unsigned)d.dim_o;
-                const float* p0 = src + ((int64_t)i * d.dim_i + x);
-                const float a = v0 ? p0[0] : 0.0f, e = v1 ? p0[d.dim_i] : 0.0f;
-                float acc = 0.0f;  // as skew_gather
-                acc = v0 ? __fadd_rn(acc, __fmul_rn(wc[k], a)) : acc;
-                acc = v1 ? __fadd_rn(acc, __fmul_rn(__fsub_rn(1.0f, wc[k]), e)) : acc;
-                seg[rr][tx + 32 * k] = acc;
+            for (int y = 0; y < 2; y++) {
+                const int r = r0 + 2 * p + y;
+                const int f = r < d.H ? rfirst[r] : 0, l = r < d.H ? rlast[r] : 0;
+#pragma unroll
+                for (int k = 0; k < kCSeg / 32; k++) {
+                    const int x = j0 - 32 + tx + 32 * k, i = r - tc[k] - 1;
+                    const bool in = x >= f && x < l;
+                    const bool v0 = in && (unsigned)i < (unsigned)d.dim_o;
+                    const bool v1 = in && (unsigned)(i + 1) < (unsigned)d.dim_o;
+                    const float* p0 = src + ((int64_t)i * d.dim_i + x);
+                    const float a = v0 ? p0[0] : 0.0f, e = v1 ? p0[d.dim_i] : 0.0f;
+                    float acc = 0.0f;  // as skew_gather
+                    acc = v0 ? __fadd_rn(acc, __fmul_rn(wc[k], a)) : acc;
+                    acc = v1 ? __fadd_rn(acc, __fmul_rn(__fsub_rn(1.0f, wc[k]), e)) : acc;
+                    cell[y][k] = acc;
+                }
             }
+#pragma unroll
+            for (int k = 0; k < kCSeg / 32; k++) seg[p][tx + 32 * k] = pk(cell[0][k], cell[1][k]);
         }
         __syncthreads();
-        // Bin of every valid band cell: warp = band row, lane = column.
-        for (int rr = ty; rr < nrows; rr += kCWarps) {
-            const int r = r0 + rr;
-            const bool valid = r < d.H && j >= rfirst[r] && j < rlast[r];
-            float v = 0.0f;
-            bool open = false;
-            if (valid) {
-                const bool full = j - 32 >= rfirst[r] && j + 32 <= rlast[r];
-                const float bin = cepstrum_bin<true>(&seg[rr][tx], full ? seg[rr][tx + 32] : 0.0f);
-                open = bin < 0.0f;
-                v = __fmaf_rn(1000.0f, bin, 500.0f);
+        // Bin of every valid band cell: warp = two band rows, lane = column.
+        for (int p = ty; 2 * p < nrows; p += kCWarps) {
+            const int r = r0 + 2 * p;
+            bool valid[2], full[2];
+#pragma unroll
+            for (int y = 0; y < 2; y++) {
+                const int f = r + y < d.H ? rfirst[r + y] : 0, l = r + y < d.H ? rlast[r + y] : 0;
+                valid[y] = 2 * p + y < nrows && j >= f && j < l;
+                full[y] = j - 32 >= f && j + 32 <= l;
             }
-            val[rr][tx] = v;
-            const unsigned m = __ballot_sync(0xffffffffu, open);
-            if (m) {
-                int at = 0;
-                if (tx == 0) at = atomicAdd(&sm.n_open, __popc(m));
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << tx) - 1u));
-                if (open) sm.open_cells[at] = (unsigned short)(rr * 32 + tx);
+            float2 bin = make_float2(0.0f, 0.0f);
+            if (valid[0] || valid[1]) {
+                float m0, m1;
+                upk(seg[p][tx + 32], m0, m1);
+                bin = cepstrum_bin<true>(&seg[p][tx], pk(full[0] ? m0 : 0.0f, full[1] ? m1 : 0.0f));
+            }
+#pragma unroll
+            for (int y = 0; y < 2; y++) {
+                const float v = y ? bin.y : bin.x;
+                const bool open = valid[y] && v < 0.0f;
+                val[2 * p + y][tx] = valid[y] ? __fmaf_rn(1000.0f, v, 500.0f) : 0.0f;
+                const unsigned m = __ballot_sync(0xffffffffu, open);
+                if (m) {
+                    int at = 0;
+                    if (tx == 0) at = atomicAdd(&sm.n_open, __popc(m));
+                    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << tx) - 1u));
+                    if (open) sm.open_cells[at] = (unsigned short)((2 * p + y) * 32 + tx);
+                }
             }
         }
         __syncthreads();
         // The open cells, a thread each: the value itself.
         for (int k = threadIdx.x; k < sm.n_open; k += kCThreads) {
             const int rr = sm.open_cells[k] >> 5, x = sm.open_cells[k] & 31;
-            val[rr][x] = cepstrum_f32(&seg[rr][x]);
+            val[rr][x] = cepstrum_f32(reinterpret_cast<const float*>(&seg[rr >> 1][x]) + (rr & 1));
         }
         __syncthreads();
         if (threadIdx.x == 0) sm.n_open = 0;  // counted again after the barrier below
-        if (col_ok && nv > 0) {
+        if (col_ok) {
             const int off = tg[j] - tmin;
-#pragma unroll
-            for (int k = 0; k < kCPer; k++) {
-                if (k >= nv) continue;
-                const float lo = val[ib + k + off][tx], hi = val[ib + k + 1 + off][tx];
+#pragma unroll 4
+            for (int i = ty; i < ni; i += kCWarps) {
+                const float lo = val[i + off][tx], hi = val[i + 1 + off][tx];
                 const float m = (lo < hi) ? hi : lo;  // std::max(lo, hi)
-                const float v = (o[k] < m) ? m : o[k];
+                const float o = sm.acc[i][tx];
+                const float v = (o < m) ? m : o;
                 // a + 1000*(int)(v/1000): the low decimal digits carry the angle.
-                o[k] = __int2float_rn(d.angle + 1000 * __float2int_rz(__fdiv_rn(v, 1000.0f)));
+                sm.acc[i][tx] = __int2float_rn(d.angle + 1000 * __float2int_rz(__fdiv_rn(v, 1000.0f)));
             }
         }
         __syncthreads();  // seg and val are rewritten for the next sector
     }
     if (!col_ok) return;
-#pragma unroll
-    for (int k = 0; k < kCPer; k++) {
-        const int i = i0 + ib + k;
-        if (i < i_end) A[(int64_t)i * dim + j] = o[k];
-    }
+    for (int i = ty; i < ni; i += kCWarps) A[(int64_t)(i0 + i) * dim + j] = sm.acc[i][tx];
 }
 
 }  // namespace

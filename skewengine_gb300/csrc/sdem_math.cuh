@@ -1,6 +1,7 @@
 // Arithmetic shared by the total-viewshed sweeps (k_sweep.cu, k_sdem.cu).
 #pragma once
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace ske {
@@ -30,30 +31,6 @@ __device__ __forceinline__ float div_fast(float a, float negd, float y) {
     return __fmaf_rn(r, y, q0);
 }
 
-// Packed pairs of floats for the f32x2 instructions: two independent IEEE
-// operations, round to nearest, no flush to zero.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0,%1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
-    f2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 // Both halves of a/d correctly rounded (div_fast on each half).
 __device__ __forceinline__ f2 div2(f2 a, f2 negd, f2 y) {
     const f2 q0 = mul2(a, y);
