@@ -34,6 +34,8 @@
 // 64-cell windows read from the staged segments), and max-deskews into the tile's
 // accumulator in shared memory.  The skewed input and output never reach HBM; the orientations
 // (4 x N floats per image) stay L2-resident.
+#include <cooperative_groups.h>
+
 #include "cepstrum_bin.cuh"
 
 namespace ske {
@@ -152,19 +154,29 @@ __device__ __forceinline__ float cepstrum_f32(const float* __restrict__ w) {
 
 struct CSmem {
     f2 seg[kCBand / 2][kCSeg];  // two band rows in the halves
-    float val[kCBand][32];
-    float acc[kCRows][32];  // the tile's accumulator
+    int val[kCBand][32];   // bins
+    int acc[kCRows][32];   // the tile's accumulator: see k_cepstrum_fused
     unsigned short open_cells[kCBand * 32];  // band cells cepstrum_bin left open
     int n_open;
 };
 
-// One launch: blockIdx.y = image; blockIdx.x = (type, tile row, tile column).
+// The reference's max+angle update o = angle + 1000*(int)(max(o, m)/1000) keeps
+// the last sector's angle and the largest bin (int)(m/1000), except that the bin
+// of an infinite m saturates and 1000 times it wraps to -1000: the cell becomes
+// angle - 1000, as if its largest bin were -1, whatever came before.  So a cell's
+// state over any run of sectors is that bin (-1: none, or just emptied) and
+// whether it was emptied, and runs of consecutive sectors can be formed apart.
+constexpr int kEmptied = 1 << 30;  // in CSmem::acc, beside the largest bin + 1
+
+// One launch: blockIdx.y = image; blockIdx.x = (type, tile row, tile column);
+// blockIdx.z, the rank in the cluster: which of the type's runs of sectors.  The
+// CTAs of a cluster join their runs through distributed shared memory.
 __global__ void __launch_bounds__(kCThreads, 1)
     k_cepstrum_fused(BatchTables T, DevGeometry g, TypeLists tl, int dim, int tiles_x, int tiles_y) {
     extern __shared__ __align__(16) unsigned char smem_c[];
     CSmem& sm = *reinterpret_cast<CSmem*>(smem_c);
     f2(*seg)[kCSeg] = sm.seg;
-    float(*val)[32] = sm.val;
+    int(*val)[32] = sm.val;
     const int per_type = tiles_x * tiles_y;
     const int t = blockIdx.x / per_type;
     const int tile = blockIdx.x - t * per_type;
@@ -182,9 +194,10 @@ __global__ void __launch_bounds__(kCThreads, 1)
     float* A = G.acc + t * n;
     const float* src = G.orient + t * n;
     if (threadIdx.x == 0) sm.n_open = 0;  // (the first sector's staging ends in a barrier)
-    if (col_ok)
-        for (int i = ty; i < ni; i += kCWarps) sm.acc[i][tx] = A[(int64_t)(i0 + i) * dim + j];
-    for (int q = 0; q < cnt; q++) {
+    // The accumulators are zero before the first sector: bin 0.
+    for (int i = ty; i < ni; i += kCWarps) sm.acc[i][tx] = blockIdx.z == 0 ? 1 : 0;
+    const int q0 = cnt * (int)blockIdx.z / (int)gridDim.z, q1 = cnt * ((int)blockIdx.z + 1) / (int)gridDim.z;
+    for (int q = q0; q < q1; q++) {
         const SectorDesc d = g.desc[tl.angle[t][q]];
         const int32_t* tg = g.target + d.col_off;
         const float* wg = g.weight + d.col_off;
@@ -249,7 +262,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
             for (int y = 0; y < 2; y++) {
                 const float v = y ? bin.y : bin.x;
                 const bool open = valid[y] && v < 0.0f;
-                val[2 * p + y][tx] = valid[y] ? __fmaf_rn(1000.0f, v, 500.0f) : 0.0f;
+                val[2 * p + y][tx] = valid[y] ? __float2int_rz(v) : 0;
                 const unsigned m = __ballot_sync(0xffffffffu, open);
                 if (m) {
                     int at = 0;
@@ -263,7 +276,8 @@ __global__ void __launch_bounds__(kCThreads, 1)
         // The open cells, a thread each: the value itself.
         for (int k = threadIdx.x; k < sm.n_open; k += kCThreads) {
             const int rr = sm.open_cells[k] >> 5, x = sm.open_cells[k] & 31;
-            val[rr][x] = cepstrum_f32(reinterpret_cast<const float*>(&seg[rr >> 1][x]) + (rr & 1));
+            const float v = cepstrum_f32(reinterpret_cast<const float*>(&seg[rr >> 1][x]) + (rr & 1));
+            val[rr][x] = __float2int_rz(__fdiv_rn(v, 1000.0f));
         }
         __syncthreads();
         if (threadIdx.x == 0) sm.n_open = 0;  // counted again after the barrier below
@@ -271,18 +285,26 @@ __global__ void __launch_bounds__(kCThreads, 1)
             const int off = tg[j] - tmin;
 #pragma unroll 4
             for (int i = ty; i < ni; i += kCWarps) {
-                const float lo = val[i + off][tx], hi = val[i + 1 + off][tx];
-                const float m = (lo < hi) ? hi : lo;  // std::max(lo, hi)
-                const float o = sm.acc[i][tx];
-                const float v = (o < m) ? m : o;
-                // a + 1000*(int)(v/1000): the low decimal digits carry the angle.
-                sm.acc[i][tx] = __int2float_rn(d.angle + 1000 * __float2int_rz(__fdiv_rn(v, 1000.0f)));
+                const int m = max(val[i + off][tx], val[i + 1 + off][tx]);
+                const int o = sm.acc[i][tx];
+                sm.acc[i][tx] = m == 0x7fffffff ? kEmptied : max(o & (kEmptied - 1), m + 1) | (o & kEmptied);
             }
         }
         __syncthreads();  // seg and val are rewritten for the next sector
     }
-    if (!col_ok) return;
-    for (int i = ty; i < ni; i += kCWarps) A[(int64_t)(i0 + i) * dim + j] = sm.acc[i][tx];
+    // The runs in order, a share of the tile's rows to each CTA.
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    const int last_angle = tl.angle[t][cnt - 1];
+    for (int i = ty + kCWarps * (int)blockIdx.z; i < ni; i += kCWarps * (int)gridDim.z) {
+        int o = 0;
+        for (unsigned z = 0; z < gridDim.z; z++) {
+            const int v = *cluster.map_shared_rank(&sm.acc[i][tx], z);
+            o = v & kEmptied ? v & (kEmptied - 1) : max(o, v);
+        }
+        if (col_ok) A[(int64_t)(i0 + i) * dim + j] = __int2float_rn(last_angle + 1000 * (o - 1));
+    }
+    cluster.sync();  // no CTA leaves while another reads its rows
 }
 
 }  // namespace
@@ -305,8 +327,37 @@ cudaError_t launch_cepstrum_f32(const BatchTables& t, int images, const DevGeome
     const int smem = (int)sizeof(CSmem);
     cudaError_t e = cudaFuncSetAttribute(k_cepstrum_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_cepstrum_fused<<<dim3((unsigned)blocks, (unsigned)images), kCThreads, smem, st>>>(t, g, tl, dim, tiles_x, tiles_y);
-    return cudaGetLastError();
+    // Runs of sectors per tile: the fewest whose waves of clusters, each as long as
+    // a run, come within 2% of the least.  Two images of 64x64 have 16 tiles, and
+    // walking their 45 sectors in turn left the other SMs idle: 1009 us with one
+    // run, 342 with eight (one image of 256x256: 2568 and 733).  16 images of
+    // 512x512 (2048 tiles, 13.5 waves of 152): 34.7 ms in one run, 34.0 in two.
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kCThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int runs = 1;
+    double least = 0.0;
+    for (int s = 1; s <= 8; s *= 2) {
+        attr.val.clusterDim = {1, 1, (unsigned)s};
+        cfg.gridDim = dim3((unsigned)blocks, (unsigned)images, (unsigned)s);
+        int resident = 0;
+        if (cudaOccupancyMaxActiveClusters(&resident, k_cepstrum_fused, &cfg) != cudaSuccess) cudaGetLastError();
+        if (resident < 1) continue;
+        const int64_t clusters = blocks * images;
+        const double time = (double)((clusters + resident - 1) / resident) / s;
+        if (s == 1 || time < 0.98 * least) {
+            least = time;
+            runs = s;
+        }
+    }
+    attr.val.clusterDim = {1, 1, (unsigned)runs};
+    cfg.gridDim = dim3((unsigned)blocks, (unsigned)images, (unsigned)runs);
+    return cudaLaunchKernelEx(&cfg, k_cepstrum_fused, t, g, tl, dim, tiles_x, tiles_y);
 }
 
 }  // namespace ske
