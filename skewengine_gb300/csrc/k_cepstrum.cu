@@ -22,8 +22,8 @@
 // pipe 84% busy).  So the cepstrum is formed in float with a bound on its error
 // (a thread per two cells, the windows in registers), and only the cells whose bin
 // that leaves open run the exact kernel.  The whole run of a 512 x 512 texture
-// (180 angles): 353.3 ms with every cell in binary64, 2.86 ms so (the float
-// kernel 1.9, the open cells 0.6); 3.20 with a thread per cell.
+// (180 angles): 353.3 ms with every cell in binary64, 2.75 ms so (the float
+// kernel 1.9, the open cells 0.56); 3.20 with a thread per cell.
 // cepstrum_bin.cuh has the evaluation and its bounds.
 #include "cepstrum_bin.cuh"
 
@@ -35,7 +35,7 @@ constexpr int kWin = kBlurWindow;  // 64
 constexpr int kWarpsPerBlock = 8;
 constexpr float kOpen = -1.0f;  // left in SO by k_cepstrum_bins for k_cepstrum (no value is negative)
 
-// kMarked: only the cells that hold kOpen, looked for 32 at a time.
+// kMarked: only the cells that hold kOpen (MarkScan).
 template <bool kMarked>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
     k_cepstrum(DevGeometry g, Batch b, const float* __restrict__ SI, float* __restrict__ SO, int64_t stride,
@@ -56,12 +56,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
     const double norm64 = __ddiv_rn(1.0, __dsqrt_rn(64.0));
     const double norm32 = __ddiv_rn(1.0, __dsqrt_rn(32.0));
     const int64_t warps = (int64_t)gridDim.x * kWarpsPerBlock;
-    constexpr int kStep = kMarked ? 32 : 1;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * kStep; q0 < len; q0 += warps * kStep) {
-        unsigned todo = 1u;
-        if (kMarked) todo = __ballot_sync(0xffffffffu, q0 + lane < len && out[q0 + lane] == kOpen);
-        for (; todo; todo &= todo - 1) {
-            const int64_t p = q0 + __ffs(todo) - 1;
+    constexpr int kStep = kMarked ? 32 : 1, kGroups = kMarked ? kScanGroups : 1;
+    const int64_t far = warps * kStep;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * kStep; q0 < len; q0 += far * kGroups) {
+        MarkScan marks;
+        if (kMarked) marks.read(out, q0, far, len, kOpen, lane);
+        int64_t p = q0;
+        for (bool some = kMarked ? marks.next(q0, far, p) : true; some; some = kMarked && marks.next(q0, far, p)) {
             const int r = owner_row(d, first, last, p);  // warp-uniform
             if (r < 0) {
                 if (lane == 0) out[p] = 0.0f;
@@ -199,10 +200,8 @@ cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const flo
         g, b, SI, SO, stride, col_blocks);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    int64_t blocks = (len + kWarpsPerBlock * 32 - 1) / (kWarpsPerBlock * 32);
-    if (blocks > 1024) blocks = 1024;
-    k_cepstrum<true><<<dim3((unsigned)blocks, b.count), kWarpsPerBlock * 32, 0, st>>>(g, b, SI, SO, stride, len, tw64,
-                                                                                       tw32);
+    k_cepstrum<true><<<dim3(mark_blocks(len, kWarpsPerBlock, b.count), b.count), kWarpsPerBlock * 32, 0, st>>>(
+        g, b, SI, SO, stride, len, tw64, tw32);
     return cudaGetLastError();
 }
 

@@ -15,8 +15,8 @@
 // per 512 x 512 image at all 180 angles, that pipe 83% busy).  Every value the
 // output depends on is a comparison or one rounding to float, so a cheaper
 // evaluation with a proven error decides it unless it falls within that error
-// of a tie (the whole run of that image: 278.7 ms before, 3.7 ms so, of it 0.25 ms
-// in step 1, 2.4 in step 2 and 0.6 in step 3):
+// of a tie (the whole run of that image: 278.7 ms before, 3.4 ms so, of it 0.25 ms
+// in step 1, 2.4 in step 2 and 0.35 in step 3):
 //  1. k_lradon_sums: W of every row, once per column (the tile-by-tile form
 //     recomputed each about three times), as exact 64-bit integer prefix sums
 //     where the reference's sequential binary64 sums make no rounding.
@@ -32,21 +32,22 @@
 //
 // W of a column of a tile is hi + lo in units of g, the largest |W| of the column
 // being 2^26 .. 2^27 of them: hi an integer, |lo| <= 1/2.  F is an integer of
-// 2^-30 units plus a rest.  Error bounds in g (u = 2^-24, maxW = the largest |W|
+// 2^-33 units (|F| < 1/4) plus a rest.  Error bounds in g (u = 2^-24, maxW = the largest |W|
 // of the cell's rows, SF_m = sum over q of |F_m[q]| times the W it multiplies):
 //  * float Z_m: lo left out, SF_m / 2; rounding of hi, of the pair's sum, of F_m
 //    and of the last sum, u each; and u for every addition from q's own to the
 //    end of its chain, q/2 + 1 of them since the chains run from q = 32 down to
 //    0, towards the large F: together u maxW SW_m, SW_m = sum of (q/2 + 5) times
 //    |F_m[q]|, formed per sector (LrTable).
-//  * integer Z_m: lo and the rest of F are good to 2^-24 and 2^-55; the two float
-//    chains of 33 corrections below 1 and 5 leave at most 33 u (1 + 5) = 1.2e-5;
+//  * integer Z_m: each component takes two float chains of 33 corrections, of lo
+//    (partial sums below sum of |F_m[q]| < 0.46) and of the rest of F (33 times
+//    2^28 2^-34 = 0.52): 33 u 0.98 = 1.9e-6, and 1.1e-6 for the inputs' own
+//    roundings and joining the parts; together below 5e-6 for the complex value.
 //    F_m itself is good to 2^-46 maxW.
 //  * the reference's own binary64 result differs from the exact one by the
 //    rounding of its 12 stages and its iterated twiddles (up to 15 * 2^-53 off
 //    the unit circle in a stage of 64 points, 61 over a transform's stages): at
-//    most 45 * 2^-53 S, S = sum of |W| gauss <= maxW sum gauss; 2^-47 maxW sum
-//    gauss is used.
+//    most 45 * 2^-53 S = 5e-15 S, S = sum of |W| gauss <= maxW sum gauss.
 #include <climits>
 #include <cmath>
 
@@ -166,7 +167,7 @@ constexpr int kQn = kHalf + 1;    // 33
 constexpr int kQp = kQn + 1;      // row pitch of the float table (16-byte rows)
 
 struct LrTable {
-    int4 fix[kQn][kMn];    // {re, im} in 2^-30 units, {re, im} as float bits
+    int4 fix[kQn][kMn];    // {re, im} in 2^-33 units, {re, im} as float bits
     float2 rest[kQn][kMn];  // what the integers leave of re and im
     float2 one[kMn][kQp];  // {re, im}, rows for the float search
     float sf[kMn], sw[kMn];  // SF_m and SW_m, rounded up
@@ -185,9 +186,9 @@ __global__ void __launch_bounds__(256)
         const int q = k / kMn, m = k % kMn;
         const double2 K = g_lr_kernel[k];
         const double re = K.x * gauss[kHalf - q], im = K.y * gauss[kHalf - q];
-        const int ri = __double2int_rn(re * 1073741824.0), ii = __double2int_rn(im * 1073741824.0);
+        const int ri = __double2int_rn(re * 8589934592.0), ii = __double2int_rn(im * 8589934592.0);
         t.fix[q][m] = make_int4(ri, ii, __float_as_int((float)re), __float_as_int((float)im));
-        t.rest[q][m] = make_float2((float)(re - ri * 9.3132257461547852e-10), (float)(im - ii * 9.3132257461547852e-10));
+        t.rest[q][m] = make_float2((float)(re - ri * 1.1641532182693481e-10), (float)(im - ii * 1.1641532182693481e-10));
         t.one[m][q] = make_float2((float)re, (float)im);
         if (q == 0) t.one[m][kQn] = make_float2(0.0f, 0.0f);
     }
@@ -256,12 +257,12 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
     t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
-// acc 2^-30 + c as a normalised float pair (|acc 2^-30| < 2^30, |c| small).
+// acc 2^-33 + c as a normalised float pair (|acc 2^-33| < 2^30, |c| small).
 __device__ __forceinline__ void to_pair(long long acc, float c, float& h, float& l) {
-    const int ah = (int)(acc >> 30);
+    const int ah = (int)(acc >> 33);
     const float fh = __int2float_rn(ah);
     const float rest = __int2float_rn(ah - __float2int_rn(fh));
-    const float low = __fmaf_rn(__int2float_rn((int)(acc & 0x3fffffff)), 9.3132257461547852e-10f, rest);
+    const float low = __fmaf_rn(__int2float_rn((int)((acc >> 3) & 0x3fffffff)), 9.3132257461547852e-10f, rest);
     two_sum(fh, __fadd_rn(low, c), h, l);
 }
 
@@ -454,8 +455,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
                 float a, r;
                 two_sum(p0, p1, a, r);
                 r = __fadd_rn(r, __fadd_rn(r0, r1));
-                // 2^-46 of F, 2^-47 sum gauss of the reference; 2^-42 a of the squares.
-                const float e = __fmaf_rn(mw[c] + 1.0f, 1.4210854715202004e-14f + 7.1054273576010019e-15f * sg, 1.6e-5f);
+                // 2^-46 of F, 5e-15 sum gauss of the reference; 2^-42 a of the squares.
+                const float e = __fmaf_rn(mw[c] + 1.0f, 1.4210854715202004e-14f + 5.05e-15f * sg, 5e-6f);
                 const float del = __fmaf_rn(e, __fmaf_rn(2.01f, sqrt_approx(a), e), 2.2737367544323206e-13f * a);
                 bool next = true;  // this m becomes the last one
                 if (step > 0) {
@@ -485,8 +486,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 // twiddle sequence, binary64, no fused operations).  The 1/sqrt(64) scaling is
 // the reference's complex multiplication by (0.125, 0).  Cells whose W are all
 // finite use warp_fft_real and real scalings: the same values up to the sign of
-// zeros, so the squared magnitudes are bit-identical.  A warp looks over 32
-// cells of SO at a time for the mark k_lradon_cells left.
+// zeros, so the squared magnitudes are bit-identical.  The cells are
+// those that hold the mark k_lradon_cells left (MarkScan).  98 binary64 operations a
+// cell hold this kernel at that pipe's rate (81%), so its time is the number of
+// cells: 98.8 thousand of a 512 x 512 texture's 47 million and 0.64 ms with F in
+// 2^-30 units and wider bounds, 0.35 ms as it is.
 __global__ void __launch_bounds__(kWarps * 32)
     k_lradon_exact(DevGeometry g, Batch b, int slot0, const double* __restrict__ W, int64_t wstride,
                    float* __restrict__ SO, int64_t stride, int64_t len, const double* __restrict__ gauss_all,
@@ -507,12 +511,11 @@ __global__ void __launch_bounds__(kWarps * 32)
     cd* x = xs[warp];
     const cd scale{0.125, 0.0};  // 1/sqrt(64) (helper.h:102-104)
     const int64_t end = min((int64_t)len, (int64_t)(d.H - 1) * d.dim_i + d.diml);
-    const int64_t step = (int64_t)gridDim.x * kWarps * 32;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; q0 < end; q0 += step) {
-        unsigned todo = __ballot_sync(0xffffffffu, q0 + lane < end && out[q0 + lane] == kUndecided);
-        while (todo) {
-            const int64_t p = q0 + __ffs(todo) - 1;
-            todo &= todo - 1;
+    const int64_t far = (int64_t)gridDim.x * kWarps * 32;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; q0 < end; q0 += far * kScanGroups) {
+        MarkScan marks;
+        marks.read(out, q0, far, end, kUndecided, lane);
+        for (int64_t p; marks.next(q0, far, p);) {
             const int i = owner_row(d, first, last, p);  // warp-uniform, >= 0: only valid cells are marked
             const int j = (int)(p - (int64_t)i * d.dim_i);
             bool fin = true;
@@ -602,10 +605,8 @@ cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, 
                                                                                         SO, stride, tiles_j);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int64_t chunks = (len + kWarps * 32 - 1) / (kWarps * 32);
-    const unsigned blocks = (unsigned)(chunks < 256 ? (chunks < 1 ? 1 : chunks) : 256);
-    k_lradon_exact<<<dim3(blocks, count), kWarps * 32, 0, st>>>(g, b, slot0, W, wstride, SO, stride, len, gauss, taper,
-                                                               tw64);
+    k_lradon_exact<<<dim3(mark_blocks(len, kWarps, count), count), kWarps * 32, 0, st>>>(
+        g, b, slot0, W, wstride, SO, stride, len, gauss, taper, tw64);
     return cudaGetLastError();
 }
 

@@ -243,4 +243,47 @@ __device__ __forceinline__ void warp_fft_real(cd* x, int n, const double* __rest
     __syncwarp();
 }
 
+// Cells of out that an earlier kernel marked for an exact one, a warp per cell:
+// the warp reads kScanGroups groups of 32 at once, `far` cells apart (marked cells
+// lie together, and neighbouring groups belong to other warps), and then takes the
+// marked ones in turn.
+constexpr int kScanGroups = 8;
+struct MarkScan {
+    unsigned mask, groups;  // mask: the marked cells of group `lane`, groups: the groups with any
+    int lane;
+    // All lanes together.
+    __device__ __forceinline__ void read(const float* out, int64_t q0, int64_t far, int64_t end, float mark, int lane_) {
+        lane = lane_;
+        mask = 0;
+        bool hit[kScanGroups];
+#pragma unroll
+        for (int t = 0; t < kScanGroups; t++) {
+            const int64_t q = q0 + far * t + lane;
+            hit[t] = (q < end ? out[q] : 0.0f) == mark;
+        }
+#pragma unroll
+        for (int t = 0; t < kScanGroups; t++) {
+            const unsigned m = __ballot_sync(0xffffffffu, hit[t]);
+            mask = lane == t ? m : mask;
+        }
+        groups = __ballot_sync(0xffffffffu, mask != 0);
+    }
+    // The next marked cell, the same for all lanes.
+    __device__ __forceinline__ bool next(int64_t q0, int64_t far, int64_t& p) {
+        if (!groups) return false;
+        const int t = __ffs(groups) - 1;
+        unsigned m = __shfl_sync(0xffffffffu, mask, t);
+        p = q0 + far * t + __ffs(m) - 1;
+        m &= m - 1;
+        if (lane == t) mask = m;
+        if (!m) groups &= groups - 1;
+        return true;
+    }
+};
+// Blocks per sector for such a kernel.
+inline unsigned mark_blocks(int64_t len, int warps, int count) {
+    const int64_t reads = (len + kScanGroups * 32 * warps - 1) / (kScanGroups * 32 * warps), most = 16384 / count + 1;
+    return (unsigned)(reads < 1 ? 1 : reads < most ? reads : most);
+}
+
 }  // namespace ske
