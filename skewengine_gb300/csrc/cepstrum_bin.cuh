@@ -5,19 +5,24 @@
 //  * Windows with all 64 cells inside the row lose their centre cell's value
 //    first: only X_0 depends on the mean, and a smaller window makes every bound
 //    smaller.
-//  * X is off, as a vector, by at most 240 u |window| (u = 2^-24, Euclidean
-//    norms): the transform is sqrt(32) times a unitary one, and its stages are
-//    off by u (two stages of plain additions), 5.8 u (three of fused
-//    butterflies), 8 u (the real-input split) and u (the subtraction) of their
-//    norm, 29 u together; X_0 takes another sqrt(2).
-//  * log |X_n|^2 is off by at most 2.2 |dX_n| / |X_n| while that is below 0.05,
-//    the sum over n by Cauchy's inequality by 2.2 |dX| (sum of 1 / |X_n|^2)^1/2;
+//  * X is off, as a vector, by at most 162 u |window| (u = 2^-24, Euclidean
+//    norms): the transform is sqrt(32) times a unitary one, and each stage is off
+//    by a share of its norm.  The subtraction and two stages of plain additions:
+//    u each.  A fused butterfly of a and b, n = (|a|^2 + |b|^2)^1/2: its inner
+//    operations u (|a| + |b|), its constant u |b|, the outer one u |sum|, and the
+//    difference 2a - sum all of that and u |difference|; over both outputs, of norm
+//    sqrt(2) n, 5^1/2 u from the first two and ((3 + 5^1/2) / 2)^1/2 u from the
+//    roundings of the outputs, 3.86 u (three stages).  The real-input split: the
+//    same and sqrt(2) u for its two sums, 5.27 u.  Together 19.9 u, 20.3 u with the
+//    terms in u^2; X_0 takes another sqrt(2).
+//  * log |X_n|^2 is off by at most 2.1 |dX_n| / |X_n| while that is below 0.05,
+//    the sum over n by Cauchy's inequality by 2.1 |dX| (sum of 1 / |X_n|^2)^1/2;
 //    the logarithm itself by 2^-22 max(1, |log2|); log |X_n|^2 + log |X_{32-n}|^2
 //    is the logarithm of the product, 17 logarithms instead of 32.
 //  * Scaling X by a constant only moves c_0, which nothing reads.
 //  * 1 / |X_n|^2 + 1 / |X_{32-n}|^2 is their sum times the reciprocal of their
 //    product, whose logarithm is formed anyway; |window|^2 comes from the spectrum
-//    (Parseval), off by 10^-5 of itself against the 2 10^-3 the bound has to spare.
+//    (Parseval), off by 10^-5 of itself against the 3 10^-3 the bound has to spare.
 //  * A thread evaluates two windows in the halves of f32x2 registers, from samples
 //    staged as such pairs: the transform and the sums take half the instructions
 //    (650 a cell against 1290).  What is left to the FMA pipe is the same, and it
@@ -29,8 +34,10 @@
 //    the cell is decided when all of them land in one bin with the bound to
 //    spare.
 //  * cepstrum_f32, the float32 mode's own evaluation, is off by as much from the
-//    window with its mean (kPlain): 30 u sqrt(32) |window| for its transform, whose
-//    butterflies round three times (5 u a stage), and 24 u times the sum of its
+//    window with its mean (kPlain): 172 u |window| for its transform, whose
+//    butterflies are off by 5^1/2 u |b| in the product, u |b| in its constant and u
+//    in each sum, 4.25 u a stage (the second stage 2 u), whose split is off by 5.36
+//    u in the same way, 21.1 u together, 21.5 u with the rest; and 24 u times the sum of its
 //    logarithms for logf, the sums' additions and coefficients.  A bin that leaves
 //    room for both errors is the bin it arrives at.
 #pragma once
@@ -126,17 +133,17 @@ __device__ __forceinline__ float rcp(float x) {
 template <bool kPlain>
 __device__ __forceinline__ float cepstrum_decide(const float (&c)[16], float l2, float inv, float emax, float mean) {
     constexpr float u = 5.9604644775390625e-8f;  // 2^-24
-    // The bound of every c_k: 0.17678 = 1 / sqrt(32); 2 X is off by 480 u |window|.
+    // The bound of every c_k: 0.17678 = 1 / sqrt(32); 2 X is off by 324 u |window|.
     const float all = 17.0f * emax;  // bounds the sum of the logs' magnitudes
-    const float dx = 481.0f * u * sqrtf(l2 * inv);
-    float err = 0.17678f * (2.2f * dx + 0.7f * (4.0f * u * (17.0f + all) + 14.0f * u * all)) + 100.0f * u;
+    const float dx = 325.0f * u * sqrtf(l2 * inv);
+    float err = 0.17678f * (2.1f * dx + 0.7f * (4.0f * u * (17.0f + all) + 14.0f * u * all)) + 100.0f * u;
     float far = dx;
     if (kPlain) {
         const float norm = sqrtf(l2) + 8.0f * fabsf(mean);  // of the window as it is, at most
-        far = 481.0f * u * norm * sqrtf(inv);
+        far = 345.0f * u * norm * sqrtf(inv);
         // Every |2 X_n|^2 lies between 1 / inv and 256 norm^2; the other's logarithms are of |X_n / 8|^2.
         const float logs = fmaxf(fabsf(lg2(256.0f * norm * norm)), fabsf(lg2(inv))) + 9.0f;
-        err += 0.17678f * (2.2f * far + 24.0f * u * 32.0f * 0.7f * logs) + 100.0f * u;
+        err += 0.17678f * (2.1f * far + 24.0f * u * 32.0f * 0.7f * logs) + 100.0f * u;
     }
     float s[16], top = 0.0f;
 #pragma unroll
