@@ -4,6 +4,7 @@
 // All are HBM/L2-bound integer-indexed copies with one or two fp32 multiply-adds
 // per cell; the arithmetic that must match the reference uses explicit _rn
 // intrinsics (no contraction).
+#include <type_traits>
 #include <vector>
 
 #include <cuda.h>
@@ -370,17 +371,47 @@ __global__ void __launch_bounds__(128) k_deskew_small(DevGeometry g, TypeLists t
 // eight before: one barrier for eight sectors, and no global load in the loop
 // over them.  With a sector staged at a time, two barriers and dependent loads
 // of the column tables each, the kernel waited: 100 us per 512 x 512 image at
-// 180 angles, so 39 us.
+// 180 angles, so 31 us (39 with a branch per cell, past the last row, and with
+// blocks for tiles that a type does not have).
+//
+// kOver: a tile of an overrunning type holds the band of the steeper drift (up to
+// twice the square's) and both rows' values of a cell.  Sectors past the square's
+// band went cell by cell through global memory and took most of the kernel's
+// time: 383 x 509, 86 us, so 45.
 constexpr int kRowSectors = 8;
+// Rows of a band: with overrunning rows a sector's columns drift by up to
+// 2 * 31 + 2 rows over a tile (dim_l <= 2 dim_i), else as in k_deskew.
+template <bool kOver>
+constexpr int kBandRows = kDeskewRows + (kOver ? 68 : 34);
+// A thread reads all its rows, also past the band's last.
+template <bool kOver>
+constexpr int kRowBand = kBandRows<kOver> + 8;
 
 template <bool kOver>
 struct RowStage {
-    float2 row[kRowSectors][kDeskewBand];  // (value, mask bits)
-    // kOver: (mask of the columns the previous row reaches, its value alone, its
-    // value with this row's).
-    float3 over[kOver ? kRowSectors : 1][kOver ? kDeskewBand : 1];
-    float2 col[kRowSectors][kTile];        // (weight, row of the band its cells start at, or -1)
+    // (value, mask bits); kOver: (value, the previous row's, both, 0).
+    typename std::conditional<kOver, float4, float2>::type row[kRowSectors][kRowBand<kOver>];
+    // kOver: masks of the columns in the row's range and of those the previous row reaches.
+    uint2 over[kOver ? kRowSectors : 1][kOver ? kRowBand<kOver> : 1];
+    float2 col[kRowSectors][kTile];  // (weight, row of the band its cells start at, or -1)
 };
+
+// Cells of the skewed rows a thread's accumulator rows need, of the staged sector.
+template <bool kOver, int kCells>
+__device__ __forceinline__ void row_cells(const RowStage<kOver>& st, int u, int at, unsigned bit, float (&cell)[kCells]) {
+#pragma unroll
+    for (int k = 0; k < kCells; k++) {
+        if constexpr (kOver) {
+            const float4 e = st.row[u][at + k];
+            const uint2 m = st.over[u][at + k];
+            const float x = (m.y & bit) ? e.z : e.x, y = (m.y & bit) ? e.y : 0.0f;
+            cell[k] = (m.x & bit) ? x : y;
+        } else {
+            const float2 e = st.row[u][at + k];
+            cell[k] = (__float_as_uint(e.y) & bit) ? e.x : 0.0f;
+        }
+    }
+}
 
 __device__ __forceinline__ float row_add(float v, double q) { return __double2float_rn(__dadd_rn((double)v, q)); }
 
@@ -395,20 +426,14 @@ __device__ __forceinline__ float row_cell(const SectorDesc& d, const int32_t* __
 }
 
 template <bool kKahan, bool kOver>
-__global__ void __launch_bounds__(256, kKahan ? 2 : 4)
-    k_deskew_rows(DevGeometry g, TypeLists tl, const RowValue* __restrict__ Q, int64_t pstride, float* __restrict__ acc,
-                  float* __restrict__ comp, int dimx, int dimy) {
-    __shared__ RowStage<kOver> stage[2];
+__device__ __forceinline__ void deskew_rows_tile(const DevGeometry& g, const TypeLists& tl,
+                                                 const RowValue* __restrict__ Q, int64_t pstride,
+                                                 float* __restrict__ acc, float* __restrict__ comp, int64_t n, int t,
+                                                 int dim_i, int dim_o, int j0, int i0, RowStage<kOver>* stage) {
     constexpr int kPer = kDeskewRows / 8;
-    const int t = blockIdx.z;
     const int cnt = tl.count[t];
-    if (cnt == 0) return;
-    const int64_t n = (int64_t)dimx * dimy;
-    const int dim_i = (t == 1 || t == 2) ? dimy : dimx;
-    const int dim_o = (t == 1 || t == 2) ? dimx : dimy;
-    const int j0 = blockIdx.x * kTile, i0 = blockIdx.y * kDeskewRows;
-    if (j0 >= dim_i || i0 >= dim_o) return;
     const int tx = threadIdx.x, ty = threadIdx.y, j = j0 + tx;
+    const unsigned bit = 1u << tx;
     const bool col_ok = j < dim_i;
     const int jlast = min(j0 + kTile, dim_i) - 1;
     const int i_end = min(i0 + kDeskewRows, dim_o);
@@ -429,7 +454,7 @@ __global__ void __launch_bounds__(256, kKahan ? 2 : 4)
         const SectorDesc& d = g.desc[tl.angle[t][q]];
         const int32_t* tg = g.target + d.col_off;
         const int tmin = tg[j0], nrows = (i_end - i0) + 1 + (tg[jlast] - tmin);
-        const bool staged = nrows <= kDeskewBand;
+        const bool staged = nrows <= kBandRows<kOver>;
         const int jc = min(j, jlast);
         st.col[ty][tx] = make_float2(g.weight[d.col_off + jc], __int_as_float(staged ? tg[jc] - tmin : -1));
         if (!staged) return;
@@ -437,21 +462,22 @@ __global__ void __launch_bounds__(256, kKahan ? 2 : 4)
         const int32_t* rfirst = g.first + d.row_off;
         const int32_t* rlast = g.last + d.row_off;
         const RowValue* qv = Q + tl.slot[t][q] * pstride;
+        // Loads with clamped rows, none behind a branch: a warp waits once.
+#pragma unroll 1
         for (int k = tx; k < nrows; k += 32) {
-            const int r = r0 + k;
-            float2 e = make_float2(0.0f, 0.0f);
-            if (r < d.H) e = make_float2(qv[r].alone, __uint_as_float(column_mask(rfirst[r], rlast[r], j0)));
-            st.row[ty][k] = e;
-            if (kOver) {
-                float3 o = make_float3(0.0f, 0.0f, 0.0f);
-                if (r >= 1 && r <= d.H) {
-                    const unsigned mo = column_mask(rfirst[r - 1] - dim_i, rlast[r - 1] - dim_i, j0);
-                    if (mo) {
-                        const float before = qv[r - 1].alone;
-                        o = make_float3(__uint_as_float(mo), before, r < d.H ? row_add(before, qv[r].q) : 0.0f);
-                    }
-                }
-                st.over[ty][k] = o;
+            const int r = r0 + k, rc = min(r, d.H - 1);
+            const float v = qv[rc].alone;
+            const unsigned m = r < d.H ? column_mask(rfirst[rc], rlast[rc], j0) : 0u;
+            if constexpr (kOver) {
+                const int rp = min(max(r - 1, 0), d.H - 1);
+                const float before = qv[rp].alone;
+                const double q = qv[rc].q;
+                const unsigned mo =
+                    r >= 1 && r <= d.H ? column_mask(rfirst[rp] - dim_i, rlast[rp] - dim_i, j0) : 0u;
+                st.row[ty][k] = make_float4(v, before, mo ? row_add(before, q) : 0.0f, 0.0f);
+                st.over[ty][k] = make_uint2(m, mo);
+            } else {
+                st.row[ty][k] = make_float2(v, __uint_as_float(m));
             }
         }
     };
@@ -468,19 +494,7 @@ __global__ void __launch_bounds__(256, kKahan ? 2 : 4)
             // Cells of the skewed rows this thread's accumulator rows need.
             float cell[kPer + 1];
             if (off >= 0) {
-                const float2* row = st.row[u] + ib + off;
-#pragma unroll
-                for (int kk = 0; kk <= kPer; kk++) {
-                    cell[kk] = 0.0f;
-                    if (kk > nv) continue;
-                    const float2 e = row[kk];
-                    const bool in = (__float_as_uint(e.y) >> tx) & 1u;
-                    cell[kk] = in ? e.x : 0.0f;
-                    if (kOver) {
-                        const float3 o = st.over[u][ib + off + kk];
-                        if ((__float_as_uint(o.x) >> tx) & 1u) cell[kk] = in ? o.z : o.y;
-                    }
-                }
+                row_cells(st, u, ib + off, bit, cell);
             } else {
                 const SectorDesc& d = g.desc[tl.angle[t][q0 + u]];
                 const int tj = g.target[d.col_off + j];
@@ -512,6 +526,33 @@ __global__ void __launch_bounds__(256, kKahan ? 2 : 4)
         A[at] = s[k];
         if (kKahan) comp[t * n + at] = c[k];
     }
+}
+
+template <bool kKahan, bool kOver>
+__global__ void __launch_bounds__(256, kKahan ? 2 : kOver ? 3 : 4)
+    k_deskew_rows(DevGeometry g, TypeLists tl, const RowValue* __restrict__ Q, int64_t pstride, float* __restrict__ acc,
+                  float* __restrict__ comp, int dimx, int dimy) {
+    extern __shared__ __align__(16) unsigned char smem_rows[];
+    // The types' tiles in turn (types 0 and 3, then the transposed ones).
+    const int tiles_j = (dimx + kTile - 1) / kTile, tiles_jt = (dimy + kTile - 1) / kTile;
+    const int tiles = tiles_j * ((dimy + kDeskewRows - 1) / kDeskewRows);
+    const int tiles_t = tiles_jt * ((dimx + kDeskewRows - 1) / kDeskewRows);
+    const bool tr = (int)blockIdx.x >= 2 * tiles;
+    const int at = tr ? blockIdx.x - 2 * tiles : blockIdx.x, per = tr ? tiles_t : tiles;
+    const int t = tr ? 1 + at / per : 3 * (at / per);
+    const int tile = at % per;
+    if (tl.count[t] == 0) return;
+    const int64_t n = (int64_t)dimx * dimy;
+    const int dim_i = tr ? dimy : dimx;
+    const int dim_o = tr ? dimx : dimy;
+    const int j0 = tile % (tr ? tiles_jt : tiles_j) * kTile, i0 = tile / (tr ? tiles_jt : tiles_j) * kDeskewRows;
+    // Only the orientations whose width is the grid's shorter side overrun it.
+    if (kOver && dim_i < max(dimx, dimy))
+        deskew_rows_tile<kKahan, true>(g, tl, Q, pstride, acc, comp, n, t, dim_i, dim_o, j0, i0,
+                                       reinterpret_cast<RowStage<true>*>(smem_rows));
+    else
+        deskew_rows_tile<kKahan, false>(g, tl, Q, pstride, acc, comp, n, t, dim_i, dim_o, j0, i0,
+                                        reinterpret_cast<RowStage<false>*>(smem_rows));
 }
 
 // ---- TMA-staged deskew ------------------------------------------------------
@@ -1001,7 +1042,12 @@ cudaError_t launch_deskew_add(const DevGeometry& g, const TypeLists& tl, const f
         const bool kahan = accum_mode == kAccumKahan;
         auto kern = rows_over ? (kahan ? k_deskew_rows<true, true> : k_deskew_rows<false, true>)
                               : (kahan ? k_deskew_rows<true, false> : k_deskew_rows<false, false>);
-        kern<<<grid, block, 0, st>>>(g, tl, Q, pstride, acc, kahan ? comp : nullptr, dimx, dimy);
+        const int tiles = ((dimx + kTile - 1) / kTile) * ((dimy + kDeskewRows - 1) / kDeskewRows);
+        const int tiles_t = ((dimy + kTile - 1) / kTile) * ((dimx + kDeskewRows - 1) / kDeskewRows);
+        const size_t smem = rows_over ? 2 * sizeof(RowStage<true>) : 2 * sizeof(RowStage<false>);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<2 * (tiles + tiles_t), block, smem, st>>>(g, tl, Q, pstride, acc, kahan ? comp : nullptr, dimx, dimy);
     } else if (accum_mode == kAccumKahan) {
         k_deskew<kDeskewKahan><<<grid, block, 0, st>>>(g, tl, SO, stride, acc, comp, dimx, dimy);
     } else {
