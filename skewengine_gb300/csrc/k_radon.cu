@@ -146,8 +146,12 @@ __global__ void __launch_bounds__(kSumWarps * 32)
 // column of the sector's own orientation is a row.  A warp per row, lanes along
 // its columns, touched up to 32 lines a load at 45 degrees, took 15 integer
 // operations a cell to add it up exactly and reduced every row over the lanes:
-// 137 us per 512 x 512 image at 180 angles, this form 69 us (bound by issue:
-// 36 instructions a cell, 13 of them the cuts).
+// 137 us per 512 x 512 image at 180 angles, this form 62 us in binary64's stead
+// (13 instructions a cell are the cuts) and 45 us in float at 383 x 509.
+// Where all 32 rows hold a batch of 32 columns with both their sources, which is
+// most of a sector, a cell is two loads at one address, two products and a sum,
+// 16 columns in flight; elsewhere each source is tested, 69 us for all of them
+// (both shapes).  The next batch's shifts and weights are on their way meanwhile.
 // A cell is the skew's, w x[r-t-1] + (1-w) x[r-t], up to the sign of a zero.
 //
 // Exact sums in float.  With |cell| <= 2^E (E from the grid's largest finite
@@ -220,6 +224,8 @@ __global__ void __launch_bounds__(kRowWarps * 32)
         float w;
         int t;
         int64_t off;  // of the w term's source cell from the lane's row
+        // Columns taken by `inside`: w and t's bits are the weights of the lower
+        // and the upper address.
     };
     __shared__ Column meta[kRowWarps][32];
     __shared__ RowPart parts[kF32 ? 1 : kRowWarps][32];
@@ -248,6 +254,7 @@ __global__ void __launch_bounds__(kRowWarps * 32)
     if (d.type == 1) base += n_cells - 1;
     if (d.type == 2) base += n_cells - dimx, is = 1;
     const float* mine = base + (int64_t)r * is;
+    const float* low = mine + min(is, 0);
     const unsigned width = (unsigned)max(l - f, 0);
     auto column = [&](int j) {
         const int over = kOver && j >= dim_i ? 1 : 0, c = j - (over ? dim_i : 0);
@@ -272,15 +279,49 @@ __global__ void __launch_bounds__(kRowWarps * 32)
     const int j0 = lo + warp * each, j1 = min(j0 + each, hi);
     // add(v): kRowStep cells of consecutive columns.
     auto walk = [&](auto add) {
+        Column next = column(j0 + lane);  // a batch ahead
         for (int jb = j0; jb < j1; jb += 32) {
+            Column m = next;
+            next = column(jb + 32 + lane);
+            const int n = min(32, j1 - jb), n8 = (n + kRowStep - 1) / kRowStep * kRowStep;
+            const int ta = __reduce_min_sync(0xffffffffu, lane < n8 ? m.t : INT_MAX);
+            const int tb = __reduce_max_sync(0xffffffffu, lane < n8 ? m.t : INT_MIN);
+            // Every cell of the 32 rows valid and with both its sources.
+            const bool inside = __all_sync(0xffffffffu, f <= jb && l >= jb + n8 && r > tb && r - ta < dim_o) &&
+                                (!kOver || jb + n8 <= dim_i);
+            if (inside) {
+                const float w1 = __fsub_rn(1.0f, m.w);
+                m.t = __float_as_int(is > 0 ? w1 : m.w);
+                m.w = is > 0 ? m.w : w1;
+            }
             __syncwarp();
-            meta[warp][lane] = column(jb + lane);
+            meta[warp][lane] = m;
             __syncwarp();
-            const int n = min(32, j1 - jb);
-            for (int k = 0; k < n; k += kRowStep) {
-                float v[kRowStep];
+            int k = 0;
+            for (; inside && k + 2 * kRowStep <= n8; k += 2 * kRowStep) {
+                float v[2 * kRowStep];
 #pragma unroll
-                for (int q = 0; q < kRowStep; q++) v[q] = cell(jb + k + q, meta[warp][k + q]);
+                for (int q = 0; q < 2 * kRowStep; q++) {
+                    const Column c = meta[warp][k + q];
+                    const float* x = low + c.off;
+                    v[q] = __fadd_rn(__fmul_rn(c.w, x[0]), __fmul_rn(__int_as_float(c.t), x[1]));
+                }
+                add(v);
+                add(v + kRowStep);
+            }
+            for (; k < n; k += kRowStep) {
+                float v[kRowStep];
+                if (inside) {
+#pragma unroll
+                    for (int q = 0; q < kRowStep; q++) {
+                        const Column c = meta[warp][k + q];
+                        const float* x = low + c.off;
+                        v[q] = __fadd_rn(__fmul_rn(c.w, x[0]), __fmul_rn(__int_as_float(c.t), x[1]));
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kRowStep; q++) v[q] = cell(jb + k + q, meta[warp][k + q]);
+                }
                 add(v);
             }
         }
