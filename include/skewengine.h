@@ -515,9 +515,10 @@ int ske_conv_select(int path);
 int ske_conv_stage_channels(int channels);
 
 /* Weight-gradient kernel for later calls of ske_conv3x3_wgrad_bf16: 1 (default)
- * = ldmatrix + mma.sync; 0 = tcgen05 (dY and X staged once per tile as
- * 8-channel planes and read in place as MN-major operands, the 9 taps'
- * accumulators in tensor memory, float32 atomics into dw), measured slower on
+ * = ldmatrix + mma.sync, by image rows for 32 input channels and more, else by
+ * 64-column tiles; 0 = tcgen05 (dY and X staged once per tile as 8-channel planes
+ * and read in place as MN-major operands, the 9 taps' accumulators in tensor
+ * memory, float32 atomics into dw), measured slower than the 64-column tiles on
  * the surrogate's layers except the widest.  Same sums in other orders.  No
  * reference counterpart. */
 int ske_conv_wgrad_select(int path);

@@ -707,7 +707,7 @@ int aligned8(const void* p) { return ((uintptr_t)p & 7) == 0; }
 // of four rows), so X and dY leave L2 once per channel block instead of once per
 // tap, and nine taps share every dY fragment: 11 ldmatrix for 36 MMAs of a warp,
 // against 4 for 8.  Bound by the mma.sync rate.  At 64 -> 64 channels, 16 images
-// of 128 x 128: 139 us by 64-column tiles, WGRAD_US so.
+// of 128 x 128: 139 us by 64-column tiles, 66 us so.
 template <int kWco, int kWci, int kSeg>
 struct WgRows {
     static constexpr int kThr = 32 * kWco * kWci;

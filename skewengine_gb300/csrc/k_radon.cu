@@ -8,11 +8,12 @@
 // (helper.h:59-106) with its exact twiddle sequence, computed in binary64 with
 // no fused operations, so the result is bit-identical to the reference.
 //
-// Three launches per batch: row sums (one warp per row), transform (one CTA per
-// sector), back-projection (one thread per cell).  Where no row is longer than
+// Three launches per batch: row sums (k_radon_sums, one warp per row), transform (a
+// cluster of four CTAs per sector, or one CTA), back-projection (one thread per
+// cell).  Where no row is longer than
 // twice its width (every grid up to 2:1) the engine skips the back-projection
-// (its deskew reads the filtered row values) and the skew (the row sums gather
-// the skewed cells from the oriented input themselves).  Selectable for sectors
+// (its deskew reads the filtered row values) and the skew (k_radon_rows, a lane
+// per row, gathers the skewed cells from the oriented input itself).  Selectable for sectors
 // whose rows stay within their width: sums and transform as one fused sector
 // kernel (k_radon_sector, a thread-block cluster per sector).
 #include <climits>

@@ -14,8 +14,9 @@ with bfloat16 operands and float32 accumulation).  At inference the decoder's
 upsampling and concatenation are read in place by the convolution
 (``ske_conv3x3_upcat_bf16``), the last convolution and the 1x1 output layer are
 one kernel (``ske_conv3x3_head_bf16``) and pooling is a kernel of its own
-(``ske_maxpool2_bf16``); in training those, the loss and the optimiser are
-PyTorch operations around the convolutions.
+(``ske_maxpool2_bf16``).  In training a convolution's whole backward pass (ReLU,
+bias, data and weight gradient) is one call (``ske_conv3x3_backward_bf16``); the
+rest, the loss and the optimiser are PyTorch operations around the convolutions.
 
 Tensors are NHWC.  Input channels: 0 = the tile's heights minus their mean,
 divided by the tile's height range (or 1 for a flat tile), 1 = log(1 + range)
