@@ -87,7 +87,7 @@ int dev_alloc(T** p, size_t count) {
 int pinned_alloc(float** p, size_t count) {
     *p = nullptr;
     if (injected_alloc_failure()) return fail(SKE_ERR_CUDA, "injected pinned allocation failure");
-    SKE_CK(cudaHostAlloc((void**)p, sizeof(float) * count, cudaHostAllocPortable));
+    SKE_CK(cudaHostAlloc((void**)p, sizeof(float) * count, cudaHostAllocPortable | cudaHostAllocMapped));
     return SKE_OK;
 }
 
@@ -141,7 +141,9 @@ struct ske_engine_s {
     int64_t tw_off_host[32] = {0};
     int64_t lr_gauss_off = 0, lr_taper_off = 0;  // local Radon tables inside d_tw
     unsigned* d_counter = nullptr;
-    int* d_status = nullptr;
+    // Set by a kernel that gives up: page-locked host memory mapped to the device,
+    // so that a call reads it without a copy (h_status, after the stream's end).
+    int *h_status = nullptr, *d_status = nullptr;
     unsigned* d_xmax = nullptr;  // bits of the input's largest finite magnitude, past d_comp's end
     // Tensor maps of d_SO for the TMA-staged deskew, for the buffer they were
     // encoded for.
@@ -284,11 +286,10 @@ int download(ske_engine e, float* dst, const float* src, int64_t n) {
 }
 
 int check_status(ske_engine e) {
-    int st = 0;
-    SKE_CK(cudaMemcpyAsync(&st, e->d_status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     SKE_CK(cudaStreamSynchronize(e->stream));
+    const int st = *static_cast<volatile int*>(e->h_status);
     if (st != 0) {
-        cudaMemsetAsync(e->d_status, 0, sizeof(int), e->stream);
+        *e->h_status = 0;
         return fail(SKE_ERR_DEVICE, "device status %d reported by a kernel", st);
     }
     return SKE_OK;
@@ -611,8 +612,7 @@ int run_prepare(ske_engine e, const float* input, int on_device) {
         SKE_TRY(upload(e, e->d_in, input, e->N));
         src = e->d_in;
     }
-    SKE_CK(cudaMemsetAsync(e->d_acc, 0, sizeof(float) * 4 * e->N, e->stream));
-    SKE_CK(cudaMemsetAsync(e->d_comp, 0, sizeof(float) * (4 * e->N + 1), e->stream));  // and d_xmax
+    SKE_CK(cudaMemsetAsync(e->d_acc, 0, sizeof(float) * (8 * e->N + 1), e->stream));  // and d_comp, d_xmax
     {
         LaunchScope ls(e, "prepare", 1);
         SKE_TRY(ls.done(launch_prepare(src, e->d_orient, e->dimx, e->dimy, e->d_xmax, e->stream)));
@@ -1489,13 +1489,16 @@ int init_engine(ske_engine e, int dimx, int dimy, int device, void* stream, ske_
     SKE_TRY(dev_alloc(&e->d_in, e->N));
     SKE_TRY(dev_alloc(&e->d_orient, 4 * e->N));
     encode_skew_maps(&e->skew_maps, e->d_orient, e->dimx, e->dimy);  // ok = false: the gather kernel runs
-    SKE_TRY(dev_alloc(&e->d_acc, 4 * e->N));
-    SKE_TRY(dev_alloc(&e->d_comp, 4 * e->N + 1));
+    SKE_TRY(dev_alloc(&e->d_acc, 8 * e->N + 1));  // one clear for the accumulators, compensations and maximum
+    e->d_comp = e->d_acc + 4 * e->N;
     e->d_xmax = reinterpret_cast<unsigned*>(e->d_comp + 4 * e->N);
     SKE_TRY(dev_alloc(&e->d_out, e->N));
     SKE_TRY(dev_alloc(&e->d_counter, 1));
-    SKE_TRY(dev_alloc(&e->d_status, 1));
-    SKE_CK(cudaMemset(e->d_status, 0, sizeof(int)));
+    float* status = nullptr;
+    SKE_TRY(pinned_alloc(&status, 1));
+    e->h_status = reinterpret_cast<int*>(status);
+    *e->h_status = 0;
+    SKE_CK(cudaHostGetDevicePointer((void**)&e->d_status, e->h_status, 0));
     SKE_TRY(pinned_alloc(&e->h_pin, (size_t)std::max<int64_t>(e->N, e->len)));
     return ensure_slots(e, 1);
 }
@@ -1520,10 +1523,10 @@ int ske_destroy(ske_engine e) {
     }
     for (cudaEvent_t ev : e->event_pool) cudaEventDestroy(ev);
     void* bufs[] = {e->d_desc, e->d_target, e->d_first, e->d_last, e->d_weight, e->d_in, e->d_orient, e->d_acc,
-                    e->d_comp, e->d_out, e->d_SI, e->d_SO, e->d_P, e->d_tw, e->d_tw_off, e->d_counter, e->d_status,
-                    e->d_lists, e->d_lradon};
+                    e->d_out, e->d_SI, e->d_SO, e->d_P, e->d_tw, e->d_tw_off, e->d_counter, e->d_lists, e->d_lradon};
     for (void* b : bufs) cudaFree(b);
     if (e->h_pin) cudaFreeHost(e->h_pin);
+    if (e->h_status) cudaFreeHost(e->h_status);
     if (e->own_stream) cudaStreamDestroy(e->stream);
     delete e;
     return SKE_OK;
