@@ -20,7 +20,9 @@
 // Most cells never run it: only the 1000-wide bin of a value is deskewed, and
 // cepstrum_bin (cepstrum_bin.cuh) arrives at it with half the operations wherever
 // its bound and this evaluation's leave no doubt; the cells they leave open (a few
-// in a hundred) are listed and take this one, a thread each.  The same bits:
+// in a hundred) are listed and take this one, a thread each; windows of one value
+// (empty borders and backgrounds) are left open by the bound and answered without it
+// (an empty 512 x 512 image: 7.3 -> 3.7 ms, a phantom 7.0 -> 5.2).  The same bits:
 // 90.1 ms for 16 images of 512 x 512 with every cell here, 46.5 so, 40.3 with
 // 256-row tiles (1.13 cepstra per skewed cell, 128-row tiles form 1.27), 34.7
 // with two cells to a thread (16 warps of 128 registers; 12 of 168 take 35.9, 8
@@ -152,6 +154,18 @@ __device__ __forceinline__ float cepstrum_f32(const float* __restrict__ w) {
     return __fmul_rn(best, 10000.0f);
 }
 
+// Whether all 64 samples of the window are one moderate value (as cepstrum_f32's
+// w).  Every X_k but X_0 is then exactly zero, its logarithm -inf, every c_k past
+// the first a sum of both infinities, and no sample ascends: the value is 0.
+__device__ __forceinline__ bool constant_window(const float* __restrict__ w) {
+    const float a = w[0];
+    if (a != w[64] || a != w[126] || !(fabsf(a) < 1e15f)) return false;
+    bool same = true;
+#pragma unroll
+    for (int n = 1; n < 63; n++) same = same && w[2 * n] == a;
+    return same;
+}
+
 struct CSmem {
     f2 seg[kCBand / 2][kCSeg];  // two band rows in the halves
     int val[kCBand][32];   // bins
@@ -276,8 +290,8 @@ __global__ void __launch_bounds__(kCThreads, 1)
         // The open cells, a thread each: the value itself.
         for (int k = threadIdx.x; k < sm.n_open; k += kCThreads) {
             const int rr = sm.open_cells[k] >> 5, x = sm.open_cells[k] & 31;
-            const float v = cepstrum_f32(reinterpret_cast<const float*>(&seg[rr >> 1][x]) + (rr & 1));
-            val[rr][x] = __float2int_rz(__fdiv_rn(v, 1000.0f));
+            const float* w = reinterpret_cast<const float*>(&seg[rr >> 1][x]) + (rr & 1);
+            val[rr][x] = constant_window(w) ? 0 : __float2int_rz(__fdiv_rn(cepstrum_f32(w), 1000.0f));
         }
         __syncthreads();
         if (threadIdx.x == 0) sm.n_open = 0;  // counted again after the barrier below

@@ -37,3 +37,18 @@ def test_runs_of_sectors_join_to_the_same_bits(gpu_lib, angles):
         with ske.SkewEngine(SIDE, SIDE) as eng:
             alone = eng.run(4, x, povh=synthetic.POVH, angles=angles, flags=ske.FLAG_CEPSTRUM_F32)
         assert bits_equal(got, alone)
+
+
+def test_windows_of_one_value(gpu_lib):
+    """An empty image and the cells of a flat one whose whole window is inside: no
+    ascent anywhere, as in the exact operator."""
+    import skewengine_gb300 as ske
+    n = 128
+    with ske.SkewEngine(n, n) as eng:
+        zero = np.zeros((n, n), np.float32)
+        assert bits_equal(eng.run(4, zero, flags=ske.FLAG_CEPSTRUM_F32), eng.run(4, zero))
+        for value in (0.7, -3.0, 1e6):
+            flat = np.full((n, n), value, np.float32)
+            got = eng.run(4, flat, angles=[0], flags=ske.FLAG_CEPSTRUM_F32)
+            assert bits_equal(got[:, 32:96], eng.run(4, flat, angles=[0])[:, 32:96])
+            assert np.all(got[:, 32:96] == 0)
