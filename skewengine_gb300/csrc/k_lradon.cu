@@ -228,7 +228,8 @@ struct CellSmem {
 
 // Binary64 w in units of 2^(emax - 1023 - 26), emax at least w's exponent field:
 // hi the nearest integer, lo the rest to 2^-25 (bit operations: conversions run
-// on the FP64 pipe).
+// on the FP64 pipe).  lo is 2^-26 at least where w is not zero and hi is, so that
+// only zeros have neither (a texture beside 1e17 lies below 2^-26 units).
 __device__ __forceinline__ void split(double w, int emax, int* hi, float* lo) {
     const long long bits = __double_as_longlong(w);
     const int e = (int)((bits >> 52) & 0x7ff);
@@ -239,7 +240,8 @@ __device__ __forceinline__ void split(double w, int emax, int* hi, float* lo) {
         h = (s + (1ll << (t - 1))) >> t;
         rem = s - (h << t);
     }
-    const float l = __fmul_rn(__int2float_rn((int)(rem >> min(t - 26, 63))), 1.4901161193847656e-8f);  // 2^-26
+    const int low = (int)(rem >> min(t - 26, 63)) | (t > 60 && s != 0);
+    const float l = __fmul_rn(__int2float_rn(low), 1.4901161193847656e-8f);  // 2^-26
     *hi = bits < 0 ? -(int)h : (int)h;
     *lo = bits < 0 ? -l : l;
 }
