@@ -31,4 +31,12 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+
+// (s, t) with s = fl(a + b) and t the exact rest (Knuth's two-sum).
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+}
+
 }  // namespace ske

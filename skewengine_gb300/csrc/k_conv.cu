@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "../../include/skewengine.h"
+#include "f32x2.cuh"
 
 namespace {
 
@@ -870,14 +871,34 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* dw, int n, i
 // dZ = dY where y > 0, dY * 0 elsewhere (bfloat16, the tensor expression
 // dY * (y > 0)), and the sums of dZ over the pixels in float32.  A thread owns 8
 // channels of every 256 / (C / 8)-th pixel of its block's share; the block's sums
-// go to a row of `part`, which k_bias_sum adds up in block order.  Memory bound
-// (6 bytes a value): 100 MB at 16 x 128 x 128 x 64, RELU_US against 195 us for the
-// comparison, product, conversion and reduction one after another.
+// go to a row of `part`, which k_bias_sum adds up in block order.  A thread's own
+// sum is plain float32 additions (27 pixels of a million of 32 channels), from
+// there on the roundings are carried along: plain to the end, the gradient was up
+// to twice as far from float64 as the tensor reduction's.  Memory bound (6 bytes a
+// value): 100 MB at 16 x 128 x 128 x 64, 17 us against 195 us for the comparison,
+// product, conversion and reduction one after another.
 constexpr int kReluBlocks = 608;   // 4 per SM
 constexpr int kReluMaxC = 2048;    // channels: C / 8 divides 256
 
+// A float32 sum with its roundings carried along.
+struct CarriedSum {
+    float sum = 0.0f, rest = 0.0f;
+    __device__ __forceinline__ void add(float v) {
+        float s, t;
+        ske::two_sum(sum, v, s, t);
+        sum = s;
+        rest += t;
+    }
+    __device__ __forceinline__ void add(float2 v) {
+        add(v.x);
+        rest += v.y;
+    }
+    // (The rest of an infinite sum is NaN.)
+    __device__ __forceinline__ float value() const { return isfinite(sum) ? sum + rest : sum; }
+};
+
 __global__ void __launch_bounds__(256) k_relu_grad(const uint4* __restrict__ y, const uint4* __restrict__ dy,
-                                                   uint4* __restrict__ dz, float* __restrict__ part, int64_t pixels,
+                                                   uint4* __restrict__ dz, float2* __restrict__ part, int64_t pixels,
                                                    int groups) {
     __shared__ float sums[256][9];
     const int g = threadIdx.x % groups;
@@ -915,24 +936,24 @@ __global__ void __launch_bounds__(256) k_relu_grad(const uint4* __restrict__ y, 
     for (int k = 0; k < 8; k++) sums[threadIdx.x][k] = s[k];
     __syncthreads();
     for (int c = threadIdx.x; c < 8 * groups; c += 256) {
-        float t = 0.0f;
-        for (int r = c / 8; r < 256; r += groups) t += sums[r][c & 7];
-        part[(int64_t)blockIdx.x * 8 * groups + c] = t;
+        CarriedSum t;
+        for (int r = c / 8; r < 256; r += groups) t.add(sums[r][c & 7]);
+        part[(int64_t)blockIdx.x * 8 * groups + c] = make_float2(t.sum, t.rest);
     }
 }
 
-__global__ void __launch_bounds__(1024) k_bias_sum(const float* __restrict__ part, float* __restrict__ db, int blocks,
+__global__ void __launch_bounds__(1024) k_bias_sum(const float2* __restrict__ part, float* __restrict__ db, int blocks,
                                                    int C) {
-    __shared__ float sums[32][33];
+    __shared__ float2 sums[32][33];
     const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, w = threadIdx.x >> 5;
-    float t = 0.0f;
+    CarriedSum t;
 #pragma unroll 8
-    for (int b = w; b < blocks; b += 32) t += c < C ? part[(int64_t)b * C + c] : 0.0f;
-    sums[w][lane] = t;
+    for (int b = w; b < blocks; b += 32) t.add(c < C ? part[(int64_t)b * C + c] : make_float2(0.0f, 0.0f));
+    sums[w][lane] = make_float2(t.sum, t.rest);
     __syncthreads();
     if (w == 0 && c < C) {
-        for (int k = 1; k < 32; k++) t += sums[k][lane];
-        db[c] = t;
+        for (int k = 1; k < 32; k++) t.add(sums[k][lane]);
+        db[c] = t.value();
     }
 }
 
@@ -2006,8 +2027,8 @@ static bool relu_grad_ok(const void* y, const void* dy, const void* dz, const fl
            aligned(y, 16) && aligned(dy, 16) && aligned(dz, 16) && aligned(db, 4);
 }
 
-// part: kReluBlocks * c floats.
-static cudaError_t launch_relu_grad(const void* y, const void* dy, void* dz, float* db, float* part, int64_t pixels,
+// part: kReluBlocks * c pairs.
+static cudaError_t launch_relu_grad(const void* y, const void* dy, void* dz, float* db, float2* part, int64_t pixels,
                                     int c, cudaStream_t st) {
     const int groups = c / 8;
     const int64_t want = (pixels + 256 / groups - 1) / (256 / groups);
@@ -2021,8 +2042,8 @@ static int ske_relu_grad_bf16_impl(const void* y, const void* dy, void* dz, floa
                                   void* stream) {
     if (!relu_grad_ok(y, dy, dz, db, pixels, c)) return SKE_ERR_INVALID;
     const cudaStream_t st = (cudaStream_t)stream;
-    float* part = nullptr;
-    if (temp_alloc(reinterpret_cast<void**>(&part), sizeof(float) * (size_t)kReluBlocks * c, st) != cudaSuccess) {
+    float2* part = nullptr;
+    if (temp_alloc(reinterpret_cast<void**>(&part), sizeof(float2) * (size_t)kReluBlocks * c, st) != cudaSuccess) {
         cudaGetLastError();
         return SKE_ERR_CUDA;
     }
@@ -2060,7 +2081,7 @@ struct BackwardScratch {
         dz = 0;
         flip = relu ? ((size_t)pixels * cout * 2 + 255) / 256 * 256 : 0;
         part = flip + (cin * kout * 2 + 255) / 256 * 256;
-        total = part + sizeof(float) * kReluBlocks * (size_t)cout;
+        total = part + sizeof(float2) * kReluBlocks * (size_t)cout;
     }
 };
 
@@ -2076,7 +2097,7 @@ static int ske_conv3x3_backward_bf16_impl(const void* x, const void* w, const vo
     void* dz = y ? base + at.dz : nullptr;
     if (scratch_bytes < at.total || !relu_grad_ok(y, dy, dz, db, pixels, cout)) return SKE_ERR_INVALID;
     const cudaStream_t st = (cudaStream_t)stream;
-    if (launch_relu_grad(y, dy, dz, db, reinterpret_cast<float*>(base + at.part), pixels, cout, st) != cudaSuccess)
+    if (launch_relu_grad(y, dy, dz, db, reinterpret_cast<float2*>(base + at.part), pixels, cout, st) != cudaSuccess)
         return SKE_ERR_CUDA;
     const void* g = y ? dz : dy;
     if (dx) {

@@ -51,6 +51,7 @@
 #include <climits>
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace ske {
@@ -250,13 +251,6 @@ __device__ __forceinline__ float sqrt_approx(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// (s, t) with s = fl(a + b) and t the exact rest (Knuth's two-sum).
-__device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
-    s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
 // acc 2^-33 + c as a normalised float pair (|acc 2^-33| < 2^30, |c| small).

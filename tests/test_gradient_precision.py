@@ -31,3 +31,24 @@ def test_wgrad_chains_stay_short(gpu_lib, n, h, w, cin, cout):
     segments = n * h * -(-w // (64 if w > 32 else 32))
     chains = -(-segments * (64 if w > 32 else 32) // 1024)
     assert _wgrad_error(sur, n, h, w, cin, cout) <= 2 * one + chains * 2.0 ** -24
+
+
+@pytest.mark.parametrize("n,h,w,c", [(2, 256, 256, 32), (16, 32, 32, 256), (1, 37, 41, 256), (3, 131, 129, 64),
+                                     (4, 512, 512, 32), (1, 37, 41, 2048)])
+def test_bias_gradient_as_close_as_the_tensor_reduction(gpu_lib, n, h, w, c):
+    """Root mean square error over the channels of eight gradients of positive terms,
+    against float64: no larger than that of the float32 reduction the kernel
+    replaces (more pixels than the kernel has threads in all but the third)."""
+    import torch
+    from skewengine_gb300 import surrogate as sur
+    mine = theirs = 0.0
+    for seed in range(8):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        dy = torch.randn((n, h, w, c), generator=g, device="cuda").abs_().to(torch.bfloat16)
+        x = torch.zeros((n, h, w, 8), dtype=torch.bfloat16, device="cuda")
+        wt = torch.zeros((c, sur.kpad(8)), dtype=torch.bfloat16, device="cuda")
+        ref = dy.double().sum((0, 1, 2))
+        db = sur.conv3x3_backward(x, wt, None, dy, need_dx=False)[2]
+        mine += float(((db.double() - ref) / ref).pow(2).mean())
+        theirs += float(((dy.float().sum((0, 1, 2)).double() - ref) / ref).pow(2).mean())
+    assert mine <= theirs
