@@ -1466,7 +1466,7 @@ bool ws_geometry(WsGeom* g, int n, int h, int w_, int cin, int cout, int c1, int
 // pool of their own: the default pool gives its memory back to the driver whenever
 // the program synchronises, and mapping it again took 200 us of the next call.
 // The pool keeps at most kPoolKeep bytes over a synchronisation, is safe with any
-// threads and streams, and serves at most kWsDevices devices (others, and a
+// threads and streams, under capture too, and serves at most kWsDevices devices (others, and a
 // driver without pools, take the default pool).
 constexpr uint64_t kPoolKeep = 64ull << 20;
 cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st) {
@@ -1481,11 +1481,15 @@ cudaError_t temp_alloc(void** p, size_t bytes, cudaStream_t st) {
             props.location.id = dev;
             cudaMemPool_t made = nullptr;
             uint64_t keep = kPoolKeep;
-            if (cudaMemPoolCreate(&made, &props) == cudaSuccess) {
-                cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
-                if (pools[dev].compare_exchange_strong(pool, made, std::memory_order_acq_rel)) pool = made;
-                else cudaMemPoolDestroy(made);  // another thread was first
-            }
+            // (A capture in progress, this thread's or another's, forbids the creation in
+            // the other modes, and would be lost.)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            const bool ok = cudaMemPoolCreate(&made, &props) == cudaSuccess &&
+                            cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
+            if (ok && pools[dev].compare_exchange_strong(pool, made, std::memory_order_acq_rel)) pool = made;
+            else if (made) cudaMemPoolDestroy(made);  // another thread was first
+            cudaThreadExchangeStreamCaptureMode(&mode);
         }
         if (pool) {
             const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
