@@ -193,14 +193,16 @@ def _relu_grad_applies(dy, y) -> bool:
     if not (dy.is_cuda and dy.dtype == torch.bfloat16 and dy.is_contiguous() and dy.numel() and c % 8 == 0
             and c <= 2048 and 256 % (c // 8) == 0 and dy.data_ptr() % 16 == 0):
         return False
-    return y is None or (y.shape == dy.shape and y.dtype == dy.dtype and y.is_contiguous() and y.device == dy.device)
+    return y is None or (y.shape == dy.shape and y.dtype == dy.dtype and y.is_contiguous() and y.device == dy.device
+                         and y.data_ptr() % 16 == 0)
 
 
 def conv3x3_backward(x, w, y, dy, need_dx: bool = True):
     """(dx, dw, db) of conv3x3(x, w, b), with a ReLU when its output y is given, in
     one call (ske_conv3x3_backward_bf16); None where its kernels do not apply."""
     import torch
-    if not (_relu_grad_applies(dy, y) and dy.dim() == 4 and x.shape[:3] == dy.shape[:3] and x.device == dy.device):
+    if not (_relu_grad_applies(dy, y) and dy.dim() == 4 and x.shape[:3] == dy.shape[:3] and x.device == dy.device
+            and w.is_contiguous()):
         return None
     _need(x, "x", torch.bfloat16)
     n, h, wd, cin = x.shape
