@@ -255,14 +255,17 @@ def _conv_fn():
             fused = conv3x3_backward(x, w, y if ctx.relu else None, dy, need_dx)
             if fused is not None:
                 return (*fused, None)
-            if ctx.relu:
-                dy = dy * (y > 0)
-            dy = dy.to(torch.bfloat16).contiguous()
+            dy = dy.to(torch.bfloat16).contiguous()  # (a sum's gradient is an expanded scalar)
+            grads = relu_grad(dy, y if ctx.relu else None)
+            if grads is not None:
+                dy, db = grads
+            else:
+                if ctx.relu:
+                    dy = (dy * (y > 0)).contiguous()
+                db = dy.float().sum((0, 1, 2))
             cin, cout = x.shape[3], w.shape[0]
             dx = conv3x3(dy, flip_transpose(w, cin, cout)) if need_dx else None
-            dw = conv3x3_wgrad(x, dy, cout)
-            db = dy.float().sum((0, 1, 2))
-            return dx, dw, db, None
+            return dx, conv3x3_wgrad(x, dy, cout), db, None
 
     return Conv3x3
 
