@@ -212,7 +212,8 @@ int ske_accumulate(ske_engine e, int kernel, const float* input, int input_on_de
 /* Test hook (no reference counterpart): the device or pinned-host allocation
  * `after` allocations from now fails as if out of memory (0 = the next one);
  * negative turns injection off.  Calls that hit it return SKE_ERR_CUDA with
- * nothing leaked; used to test failure handling without faulting a GPU. */
+ * nothing leaked (a local Radon run without its scratch takes a slower path
+ * instead); used to test failure handling without faulting a GPU. */
 int ske_inject_alloc_failure(int64_t after);
 
 /* Checkpoint / resume at sector granularity.  Like ske_accumulate, but the

@@ -338,8 +338,15 @@ int ensure_lists(ske_engine e, size_t bytes) {
     return SKE_OK;
 }
 
-// Scratch of the local Radon transform for as many of `want` sectors as 4 GB or
-// a quarter of the free memory hold (at least one); *slots: how many that is.
+// The local Radon transform's window sums take half as much per sector as the
+// skewed buffers and are kept with them, up to this size; larger grids (from 1250 x
+// 1250 at 180 angles) go in groups of sectors.  2000 x 2000: 45.5 ms, 46.4 with 1 GB
+// and 49.7 with a quarter of that.
+constexpr size_t kLradonMost = (size_t)4 << 30;
+
+// Scratch of the local Radon transform for as many of `want` sectors as kLradonMost
+// or a quarter of the free memory hold (at least one); *slots: how many that is, 0
+// where there is not the memory for one.
 int ensure_lradon(ske_engine e, int want, int* slots) {
     const size_t one = lradon_scratch_bytes(e->geo.max_H, std::max(e->dimx, e->dimy), 1);
     ske_engine own = e->parent ? e->parent : e;  // a child engine borrows its parent's
@@ -349,15 +356,15 @@ int ensure_lradon(ske_engine e, int want, int* slots) {
             cudaGetLastError();
             free_b = (size_t)1 << 30;
         }
-        const size_t budget = std::min((size_t)4 << 30, free_b / 4);
+        const size_t budget = std::min(kLradonMost, free_b / 4);
         const size_t bytes = one * std::min<size_t>(want, std::max<size_t>(1, budget / one));
         if (bytes > own->lradon_bytes) {
             SKE_CK(cudaStreamSynchronize(e->stream));
             cudaFree(own->d_lradon);
             own->d_lradon = nullptr;
             own->lradon_bytes = 0;
-            SKE_TRY(dev_alloc(&own->d_lradon, bytes));
-            own->lradon_bytes = bytes;
+            if (dev_alloc(&own->d_lradon, bytes) == SKE_OK) own->lradon_bytes = bytes;
+            else cudaGetLastError();
         }
     }
     *slots = (int)std::min<size_t>(want, own->lradon_bytes / one);
@@ -543,6 +550,12 @@ int run_operator(ske_engine e, int kernel, const Batch& b, float povh, int count
             }
             int step = 1;
             SKE_TRY(ensure_lradon(e, b.count, &step));
+            if (step == 0) {  // no memory for window sums
+                LaunchScope ls(e, "local_radon", 1);
+                return ls.done(launch_local_radon_direct(e->dg, b, e->d_SI, e->d_SO, e->stride, e->len,
+                                                         e->d_tw + e->lr_gauss_off, e->d_tw + e->lr_taper_off,
+                                                         e->d_tw + e->tw_off_host[6], e->stream));
+            }
             for (int s0 = 0; s0 < b.count; s0 += step) {
                 LaunchScope ls(e, "local_radon", kLocalRadonLaunches);
                 SKE_TRY(ls.done(launch_local_radon(

@@ -48,6 +48,7 @@
 //    rounding of its 12 stages and its iterated twiddles (up to 15 * 2^-53 off
 //    the unit circle in a stage of 64 points, 61 over a transform's stages): at
 //    most 45 * 2^-53 S = 5e-15 S, S = sum of |W| gauss <= maxW sum gauss.
+#include <algorithm>
 #include <climits>
 #include <cmath>
 
@@ -487,10 +488,16 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 // cell hold this kernel at that pipe's rate (81%), so its time is the number of
 // cells: 98.8 thousand of a 512 x 512 texture's 47 million and 0.64 ms with F in
 // 2^-30 units and wider bounds, 0.35 ms as it is.
+//
+// kDirect: every cell, each window sum formed here from the skewed input; what runs
+// where the memory for W is not to be had (a 256 x 256 image at 180 angles: 252 ms, 2.5
+// with it).
+template <bool kDirect>
 __global__ void __launch_bounds__(kWarps * 32)
-    k_lradon_exact(DevGeometry g, Batch b, int slot0, const double* __restrict__ W, int64_t wstride,
-                   float* __restrict__ SO, int64_t stride, int64_t len, const double* __restrict__ gauss_all,
-                   const double* __restrict__ taper_all, const double* __restrict__ tw64) {
+    k_lradon_exact(DevGeometry g, Batch b, int slot0, const float* __restrict__ SI, const double* __restrict__ W,
+                   int64_t wstride, float* __restrict__ SO, int64_t stride, int64_t len,
+                   const double* __restrict__ gauss_all, const double* __restrict__ taper_all,
+                   const double* __restrict__ tw64) {
     __shared__ cd xs[kWarps][kW];
     __shared__ double tw[2 * (kW - 1)], gauss[kW], taper[kLocalRadonKeep];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -503,21 +510,31 @@ __global__ void __launch_bounds__(kWarps * 32)
     const int32_t* first = g.first + d.row_off;
     const int32_t* last = g.last + d.row_off;
     const double* w = W + blockIdx.y * wstride;
+    const float* in = SI + slot * stride;
     float* out = SO + slot * stride;
     cd* x = xs[warp];
     const cd scale{0.125, 0.0};  // 1/sqrt(64) (helper.h:102-104)
     const int64_t end = min((int64_t)len, (int64_t)(d.H - 1) * d.dim_i + d.diml);
-    const int64_t far = (int64_t)gridDim.x * kWarps * 32;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * 32; q0 < end; q0 += far * kScanGroups) {
+    constexpr int kStep = kDirect ? 1 : 32, kGroups = kDirect ? 1 : kScanGroups;
+    const int64_t far = (int64_t)gridDim.x * kWarps * kStep;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * kStep; q0 < end; q0 += far * kGroups) {
         MarkScan marks;
-        marks.read(out, q0, far, end, kUndecided, lane);
-        for (int64_t p; marks.next(q0, far, p);) {
-            const int i = owner_row(d, first, last, p);  // warp-uniform, >= 0: only valid cells are marked
+        if (!kDirect) marks.read(out, q0, far, end, kUndecided, lane);
+        int64_t p = q0;
+        for (bool some = kDirect ? true : marks.next(q0, far, p); some; some = !kDirect && marks.next(q0, far, p)) {
+            const int i = owner_row(d, first, last, p);  // warp-uniform; only valid cells are marked
+            if (kDirect && i < 0) continue;
             const int j = (int)(p - (int64_t)i * d.dim_i);
             bool fin = true;
             for (int m = lane; m < kW; m += 32) {
                 const int k = i - kHalf + m;
-                const double v = k >= 0 && k < d.H ? w[(int64_t)k * d.diml + j] : 0.0;
+                double v = 0.0;
+                if (kDirect && k >= 0 && k < d.H) {
+                    const int f = first[k], l = last[k];
+                    for (int c = j - kHalf; c <= j + kHalf; c++)
+                        v = __dadd_rn(v, c >= f && c < l ? (double)in[(int64_t)k * d.dim_i + c] : 0.0);
+                }
+                if (!kDirect && k >= 0 && k < d.H) v = w[(int64_t)k * d.diml + j];
                 fin = fin && isfinite(v);
                 x[m] = cd{__dmul_rn(v, gauss[m]), 0.0};
             }
@@ -601,8 +618,18 @@ cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, 
                                                                                         SO, stride, tiles_j);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_lradon_exact<<<dim3(mark_blocks(len, kWarps, count), count), kWarps * 32, 0, st>>>(
-        g, b, slot0, W, wstride, SO, stride, len, gauss, taper, tw64);
+    k_lradon_exact<false><<<dim3(mark_blocks(len, kWarps, count), count), kWarps * 32, 0, st>>>(
+        g, b, slot0, SI, W, wstride, SO, stride, len, gauss, taper, tw64);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_local_radon_direct(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
+                                      int64_t len, const double* gauss, const double* taper, const double* tw64,
+                                      cudaStream_t st) {
+    if (b.count == 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)std::min<int64_t>((len + kWarps - 1) / kWarps, 8192);
+    k_lradon_exact<true><<<dim3(blocks, b.count), kWarps * 32, 0, st>>>(g, b, 0, SI, nullptr, 0, SO, stride, len, gauss,
+                                                                       taper, tw64);
     return cudaGetLastError();
 }
 

@@ -246,6 +246,10 @@ cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, 
                                int64_t stride, int64_t len, int max_H, int max_cols, const double* gauss,
                                const double* taper, const double* tw64, void* scratch, cudaStream_t st);
 constexpr int kLocalRadonLaunches = 4;  // kernels of one launch_local_radon
+// The same values of all slots without scratch, in binary64 throughout.
+cudaError_t launch_local_radon_direct(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
+                                      int64_t len, const double* gauss, const double* taper, const double* tw64,
+                                      cudaStream_t st);
 // The window sums of `slots` sectors of up to max_rows rows, and their filters.
 size_t lradon_scratch_bytes(int64_t max_rows, int diml, int slots);
 cudaError_t lradon_init_tables();  // the composed filters' kernel, once per device
