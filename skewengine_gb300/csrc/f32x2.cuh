@@ -39,4 +39,21 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& t) {
     t = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
+// A float32 sum with its roundings carried along.
+struct CarriedSum {
+    float sum = 0.0f, rest = 0.0f;
+    __device__ __forceinline__ void add(float v) {
+        float s, t;
+        two_sum(sum, v, s, t);
+        sum = s;
+        rest += t;
+    }
+    __device__ __forceinline__ void add(float2 v) {
+        add(v.x);
+        rest += v.y;
+    }
+    // (The rest of an infinite sum is NaN.)
+    __device__ __forceinline__ float value() const { return isfinite(sum) ? sum + rest : sum; }
+};
+
 }  // namespace ske

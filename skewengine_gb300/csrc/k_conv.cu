@@ -880,23 +880,6 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* dw, int n, i
 constexpr int kReluBlocks = 608;   // 4 per SM
 constexpr int kReluMaxC = 2048;    // channels: C / 8 divides 256
 
-// A float32 sum with its roundings carried along.
-struct CarriedSum {
-    float sum = 0.0f, rest = 0.0f;
-    __device__ __forceinline__ void add(float v) {
-        float s, t;
-        ske::two_sum(sum, v, s, t);
-        sum = s;
-        rest += t;
-    }
-    __device__ __forceinline__ void add(float2 v) {
-        add(v.x);
-        rest += v.y;
-    }
-    // (The rest of an infinite sum is NaN.)
-    __device__ __forceinline__ float value() const { return isfinite(sum) ? sum + rest : sum; }
-};
-
 __global__ void __launch_bounds__(256) k_relu_grad(const uint4* __restrict__ y, const uint4* __restrict__ dy,
                                                    uint4* __restrict__ dz, float2* __restrict__ part, int64_t pixels,
                                                    int groups) {
@@ -936,7 +919,7 @@ __global__ void __launch_bounds__(256) k_relu_grad(const uint4* __restrict__ y, 
     for (int k = 0; k < 8; k++) sums[threadIdx.x][k] = s[k];
     __syncthreads();
     for (int c = threadIdx.x; c < 8 * groups; c += 256) {
-        CarriedSum t;
+        ske::CarriedSum t;
         for (int r = c / 8; r < 256; r += groups) t.add(sums[r][c & 7]);
         part[(int64_t)blockIdx.x * 8 * groups + c] = make_float2(t.sum, t.rest);
     }
@@ -946,7 +929,7 @@ __global__ void __launch_bounds__(1024) k_bias_sum(const float2* __restrict__ pa
                                                    int C) {
     __shared__ float2 sums[32][33];
     const int lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane, w = threadIdx.x >> 5;
-    CarriedSum t;
+    ske::CarriedSum t;
 #pragma unroll 8
     for (int b = w; b < blocks; b += 32) t.add(c < C ? part[(int64_t)b * C + c] : make_float2(0.0f, 0.0f));
     sums[w][lane] = make_float2(t.sum, t.rest);

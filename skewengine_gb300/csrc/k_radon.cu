@@ -20,6 +20,7 @@
 
 #include <cooperative_groups.h>
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace ske {
@@ -165,9 +166,11 @@ __global__ void __launch_bounds__(kSumWarps * 32)
 // (RowPart), and where those do not fit either, left to right in binary64.
 //
 // kOver: rows may overrun their width into the next row's cells (and past the
-// last row into zeros).  kF32: float sums in blocks of kRowStep columns.
+// last row into zeros).  kF32: float sums, of kRowStep columns by pairs, those in
+// turn with their roundings carried along: plainly added the output's error was 2 to 8%
+// larger than by a warp's lanes, so it is 3 to 9% smaller (383 x 509: 45.5 -> 47.6 us).
 constexpr int kRowWarps = 4;
-constexpr int kRowStep = 8;  // columns in flight
+constexpr int kRowStep = 8;  // columns of one addition
 
 // Exact integer sum of one row's cells in units of 2^(emin - 150).
 struct RowPart {
@@ -328,13 +331,15 @@ __global__ void __launch_bounds__(kRowWarps * 32)
         }
     };
     if (kF32) {
-        float acc = 0.0f;
-        walk([&](const float* v) { acc += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])); });
-        sums[0][warp][lane] = acc;
+        CarriedSum acc;
+        walk([&](const float* v) { acc.add(((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))); });
+        sums[0][warp][lane] = acc.sum;
+        sums[1][warp][lane] = acc.rest;
         __syncthreads();
         if (warp != 0 || r >= H2) return;
-        const float s = (sums[0][0][lane] + sums[0][1][lane]) + (sums[0][2][lane] + sums[0][3][lane]);
-        p[r] = {(double)s, 0.0};
+        CarriedSum s;
+        for (int k = 0; k < kRowWarps; k++) s.add(make_float2(sums[0][k][lane], sums[1][k][lane]));
+        p[r] = {(double)s.value(), 0.0};
         return;
     }
     // Exponents of the cuts; 1.5 * 2^23 units of q added and taken away leave the
