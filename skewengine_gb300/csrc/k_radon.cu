@@ -169,8 +169,15 @@ __global__ void __launch_bounds__(kSumWarps * 32)
 // last row into zeros).  kF32: float sums, of kRowStep columns by pairs, those in
 // turn with their roundings carried along: plainly added the output's error was 2 to 8%
 // larger than by a warp's lanes, so it is 3 to 9% smaller (383 x 509: 45.5 -> 47.6 us).
+//
+// kFlight * kRowStep columns are in flight.  With fewer CTAs than the SMs hold (one to
+// a dozen sectors) the float32 sums wait for their loads, and twice as many at a time
+// take less (a whole run of 2000 x 2000, one sector: 235 -> 220 us; 15 sectors, 1920
+// CTAs: 292 both; 45: 409 both; all 180: 944 and 947).  The binary64 cuts have no registers
+// for more than 16 (one sector 260 -> 276).  The same sums.
 constexpr int kRowWarps = 4;
 constexpr int kRowStep = 8;  // columns of one addition
+constexpr int64_t kRowFewCtas = 12 * 152;
 
 // Exact integer sum of one row's cells in units of 2^(emin - 150).
 struct RowPart {
@@ -220,7 +227,7 @@ __device__ __forceinline__ float2 sub_pair(float2 a, float2 b) {
     return r;
 }
 
-template <bool kF32, bool kOver>
+template <bool kF32, bool kOver, int kFlight>
 __global__ void __launch_bounds__(kRowWarps * 32)
     k_radon_rows(DevGeometry g, Batch b, const float* __restrict__ orient, int64_t n_cells, int dimx, int dimy,
                  const unsigned* __restrict__ xmax, cd* __restrict__ P, int64_t pstride) {
@@ -302,16 +309,16 @@ __global__ void __launch_bounds__(kRowWarps * 32)
             meta[warp][lane] = m;
             __syncwarp();
             int k = 0;
-            for (; inside && k + 2 * kRowStep <= n8; k += 2 * kRowStep) {
-                float v[2 * kRowStep];
+            for (; inside && k + kFlight * kRowStep <= n8; k += kFlight * kRowStep) {
+                float v[kFlight * kRowStep];
 #pragma unroll
-                for (int q = 0; q < 2 * kRowStep; q++) {
+                for (int q = 0; q < kFlight * kRowStep; q++) {
                     const Column c = meta[warp][k + q];
                     const float* x = low + c.off;
                     v[q] = __fadd_rn(__fmul_rn(c.w, x[0]), __fmul_rn(__int_as_float(c.t), x[1]));
                 }
-                add(v);
-                add(v + kRowStep);
+#pragma unroll
+                for (int q = 0; q < kFlight; q++) add(v + q * kRowStep);
             }
             for (; k < n; k += kRowStep) {
                 float v[kRowStep];
@@ -836,12 +843,14 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
     cd* Pc = reinterpret_cast<cd*>(P);
     if (f32 && max_H2 <= kSmemH2) {
         dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count), gr((max_H2 + 31) / 32, b.count);
-        if (orient && in_width)
-            k_radon_rows<true, false><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
-        else if (orient)
-            k_radon_rows<true, true><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
-        else
+        if (orient) {
+            const bool few = (int64_t)gr.x * gr.y <= kRowFewCtas;
+            auto kern = in_width ? (few ? k_radon_rows<true, false, 4> : k_radon_rows<true, false, 2>)
+                                 : (few ? k_radon_rows<true, true, 4> : k_radon_rows<true, true, 2>);
+            kern<<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
+        } else {
             k_radon_sums_f32<<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, Pc, pstride);
+        }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         const int smem = max_H2 * (int)sizeof(float2);
@@ -868,9 +877,9 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
     }
     dim3 g1((max_H2 + kSumWarps - 1) / kSumWarps, b.count), gr((max_H2 + 31) / 32, b.count);
     if (orient && in_width)
-        k_radon_rows<false, false><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
+        k_radon_rows<false, false, 2><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
     else if (orient)
-        k_radon_rows<false, true><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
+        k_radon_rows<false, true, 2><<<gr, kRowWarps * 32, 0, st>>>(g, b, orient, n_cells, dimx, dimy, xmax, Pc, pstride);
     else
         k_radon_sums<<<g1, kSumWarps * 32, 0, st>>>(g, b, SI, stride, Pc, pstride);
     cudaError_t e = cudaGetLastError();

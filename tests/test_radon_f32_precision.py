@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from skewengine_gb300 import synthetic
+from tests.conftest import bits_equal
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +33,18 @@ def test_error_no_larger_than_by_lanes(gpu_lib, kind, dimx, dimy):
             diff = eng.run("radon", x, flags=ske.FLAG_RADON_F32) - want
             rms.append(np.sqrt((diff ** 2).mean()) / np.abs(want).max())
     assert np.mean(rms) <= BY_LANES[kind, dimx, dimy], np.mean(rms)
+
+
+@pytest.mark.parametrize("dims", [(1024, 1024), (700, 1200)])
+def test_row_sums_do_not_depend_on_the_number_of_sectors(gpu_lib, dims):
+    """The sectors of one type in one run, whose row sums keep 16 columns in flight,
+    against each by itself (32 in flight), added up in turn: the same bits."""
+    import skewengine_gb300 as ske
+    x = synthetic.ellipse_phantom(dims[0], 3, side_y=dims[1])
+    angles = list(range(0, 44))
+    with ske.SkewEngine(*dims) as eng:
+        together = eng.run("radon", x, angles=angles, flags=ske.FLAG_RADON_F32)
+        want = np.zeros_like(together)
+        for a in angles:
+            want += eng.run("radon", x, angles=[a], flags=ske.FLAG_RADON_F32)
+    assert bits_equal(together, want)
