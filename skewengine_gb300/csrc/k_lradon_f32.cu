@@ -18,10 +18,10 @@
 // same address (broadcast, 16 bytes per load), with the 26 bins unrolled in
 // registers.  Two cells per thread (a twiddle row serves both), their bins in
 // packed f32x2 operations; the second transform stops at the bin where both have
-// ascended.  A CTA of 256 threads owns a 128 x 32 tile of cells, stages the
-// skewed rows it needs (191 rows x 96 columns) and forms each W once.  Bound by
-// the FP32 pipe: 1.4e9 packed multiply-adds per 512 x 512 image (32-row tiles
-// formed every W three times, and all 28 bins of every cell: 9.4 ms).
+// ascended.  A CTA of 256 threads owns a 128 x 32 tile of cells (32 x 32 where those
+// are few), stages the skewed rows it needs (191 rows x 96 columns) and forms each W
+// once.  Bound by the FP32 pipe: 1.4e9 packed multiply-adds per 512 x 512 image
+// (32-row tiles and all 28 bins of every cell: 9.4 ms; 3.8 so).
 // The order of the float32 sums differs from the reference's binary64 FFT, so
 // values differ in their last bits, and where two successive |Z|^2 nearly tie
 // the first ascent can fall on another bin: the rate of output cells that
@@ -30,6 +30,7 @@
 // follows owner_row as in k_lradon.
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace ske {
@@ -39,10 +40,17 @@ namespace {
 constexpr int kW = kLocalRadonWindow;  // 64
 constexpr int kHalf = kW / 2;          // 32
 constexpr int kKeep = kLocalRadonKeep;  // 26
-constexpr int kTI = 128, kTJ = 32;   // cells of a tile
-constexpr int kRows = kTI + kW - 1;  // 191 W rows a tile needs
+constexpr int kTJ = 32;              // columns of a tile
+template <int kTI>
+constexpr int kRowsOf = kTI + kW - 1;  // W rows a tile of kTI rows needs
 constexpr int kCols = kTJ + kW;      // 96 staged columns
 constexpr int kThreads = 256;
+// Rows of a tile.  Tall ones form each W fewer times; but a dozen to an SM or fewer of
+// them leave it waiting for the longest (us of a run, 32 against 128 rows: one
+// sector of 300 x 200 117 and 198, of 512 x 512 116 and 141, empty 137 and 203;
+// 15 sectors of 512 x 512, 1920 tall tiles, 435 and 436; 30 of them 784 and 759).
+constexpr int kTallTile = 128, kLowTile = 32;
+constexpr int64_t kFewTiles = 12 * 152;
 constexpr int kZ0 = 4, kZ1 = 32;  // |Z_m|^2 formed for m = kZ0 .. kZ1 - 1
 constexpr int kZn = kZ1 - kZ0;
 constexpr int kKP = 28;  // twiddle row pitch (kKeep padded to 16 bytes)
@@ -54,22 +62,9 @@ constexpr int kKP = 28;  // twiddle row pitch (kKeep padded to 16 bytes)
 __device__ float g_tx[kW * kKP];
 __device__ float2 g_tz[kZn * kKeep];  // {cos, sin}
 
-// Packed pairs of floats (f32x2): two independent IEEE operations, round to
-// nearest, so the bits of the scalar ones.
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f2 v, float& a, float& b) { asm("mov.b64 {%0,%1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
+template <int kTI>
 struct SmemF {
+    static constexpr int kRows = kRowsOf<kTI>;
     int2 range[kRows];  // {first, last} of the staged rows ({0, 0} outside the grid)
     int2 pad;
     float s[kRows][kCols];
@@ -80,11 +75,13 @@ struct SmemF {
     float2 tz[kZn][kKeep];  // {cos, sin}
 };
 
+template <int kTI>
 __global__ void __launch_bounds__(kThreads)
     k_lradon_f32(DevGeometry g, Batch b, const float* __restrict__ SI, float* __restrict__ SO, int64_t stride,
                  int tiles_j, const double* __restrict__ gauss_all, const double* __restrict__ taper) {
+    constexpr int kRows = kRowsOf<kTI>;
     extern __shared__ __align__(16) float smem_f[];
-    SmemF& sm = *reinterpret_cast<SmemF*>(smem_f);
+    SmemF<kTI>& sm = *reinterpret_cast<SmemF<kTI>*>(smem_f);
     const int slot = blockIdx.y;
     const SectorDesc& d = g.desc[b.angle[slot]];
     const int i0 = (blockIdx.x / tiles_j) * kTI, j0 = (blockIdx.x % tiles_j) * kTJ;
@@ -244,17 +241,25 @@ int lradon_f32_init_tables() {
     return 0;
 }
 
+template <int kTI>
+static cudaError_t launch_tiles(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
+                                int max_H, int max_cols, const double* gauss, const double* taper, cudaStream_t st) {
+    const int tiles_i = (max_H + kTI - 1) / kTI, tiles_j = (max_cols + kTJ - 1) / kTJ;
+    const size_t smem = sizeof(SmemF<kTI>);
+    cudaError_t e = cudaFuncSetAttribute(k_lradon_f32<kTI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_lradon_f32<kTI><<<dim3((unsigned)(tiles_i * tiles_j), b.count), kThreads, smem, st>>>(g, b, SI, SO, stride,
+                                                                                          tiles_j, gauss, taper);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_local_radon_f32(const DevGeometry& g, const Batch& b, const float* SI, float* SO, int64_t stride,
                                    int max_H, int max_cols, const double* gauss, const double* taper,
                                    cudaStream_t st) {
     if (b.count == 0) return cudaSuccess;
-    const int tiles_i = (max_H + kTI - 1) / kTI, tiles_j = (max_cols + kTJ - 1) / kTJ;
-    const size_t smem = sizeof(SmemF);
-    cudaError_t e = cudaFuncSetAttribute(k_lradon_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k_lradon_f32<<<dim3((unsigned)(tiles_i * tiles_j), b.count), kThreads, smem, st>>>(g, b, SI, SO, stride, tiles_j,
-                                                                                     gauss, taper);
-    return cudaGetLastError();
+    const int64_t tiles = (int64_t)((max_H + kTallTile - 1) / kTallTile) * ((max_cols + kTJ - 1) / kTJ) * b.count;
+    auto launch = tiles <= kFewTiles ? launch_tiles<kLowTile> : launch_tiles<kTallTile>;
+    return launch(g, b, SI, SO, stride, max_H, max_cols, gauss, taper, st);
 }
 
 }  // namespace ske
