@@ -39,7 +39,7 @@ constexpr float kOpen = -1.0f;  // left in SO by k_cepstrum_bins for k_cepstrum 
 template <bool kMarked>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
     k_cepstrum(DevGeometry g, Batch b, const float* __restrict__ SI, float* __restrict__ SO, int64_t stride,
-               int64_t len, const double* __restrict__ tw64, const double* __restrict__ tw32) {
+               int64_t len, MarkShape shape, const double* __restrict__ tw64, const double* __restrict__ tw32) {
     __shared__ cd xs[kWarpsPerBlock][kWin];
     __shared__ double twa[2 * (kWin - 1)], twb[2 * (kWin / 2 - 1)];
     for (int i = threadIdx.x; i < 2 * (kWin - 1); i += blockDim.x) twa[i] = tw64[i];
@@ -56,11 +56,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, 6)
     const double norm64 = __ddiv_rn(1.0, __dsqrt_rn(64.0));
     const double norm32 = __ddiv_rn(1.0, __dsqrt_rn(32.0));
     const int64_t warps = (int64_t)gridDim.x * kWarpsPerBlock;
-    constexpr int kStep = kMarked ? 32 : 1, kGroups = kMarked ? kScanGroups : 1;
-    const int64_t far = warps * kStep;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * kStep; q0 < len; q0 += far * kGroups) {
+    const int step = kMarked ? shape.step : 1, groups = kMarked ? shape.groups : 1;
+    const int64_t far = warps * step;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarpsPerBlock + warp) * step; q0 < len; q0 += far * groups) {
         MarkScan marks;
-        if (kMarked) marks.read(out, q0, far, len, kOpen, lane);
+        if (kMarked) marks.read(out, q0, far, len, shape, kOpen, lane);
         int64_t p = q0;
         for (bool some = kMarked ? marks.next(q0, far, p) : true; some; some = kMarked && marks.next(q0, far, p)) {
             const int r = owner_row(d, first, last, p);  // warp-uniform
@@ -186,8 +186,8 @@ cudaError_t launch_cepstrum(const DevGeometry& g, const Batch& b, const float* S
                             int64_t len, const double* tw64, const double* tw32, cudaStream_t st) {
     int64_t blocks = (len + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (blocks > 8192) blocks = 8192;
-    k_cepstrum<false><<<dim3((unsigned)blocks, b.count), kWarpsPerBlock * 32, 0, st>>>(g, b, SI, SO, stride, len, tw64,
-                                                                                        tw32);
+    k_cepstrum<false><<<dim3((unsigned)blocks, b.count), kWarpsPerBlock * 32, 0, st>>>(g, b, SI, SO, stride, len,
+                                                                                        MarkShape(), tw64, tw32);
     return cudaGetLastError();
 }
 
@@ -200,8 +200,9 @@ cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const flo
         g, b, SI, SO, stride, col_blocks);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_cepstrum<true><<<dim3(mark_blocks(len, kWarpsPerBlock, b.count), b.count), kWarpsPerBlock * 32, 0, st>>>(
-        g, b, SI, SO, stride, len, tw64, tw32);
+    const MarkShape shape = mark_shape(len, kWarpsPerBlock, b.count);
+    k_cepstrum<true><<<dim3(shape.blocks, b.count), kWarpsPerBlock * 32, 0, st>>>(g, b, SI, SO, stride, len, shape, tw64,
+                                                                                  tw32);
     return cudaGetLastError();
 }
 

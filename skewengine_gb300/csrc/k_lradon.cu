@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 template <bool kDirect>
 __global__ void __launch_bounds__(kWarps * 32)
     k_lradon_exact(DevGeometry g, Batch b, int slot0, const float* __restrict__ SI, const double* __restrict__ W,
-                   int64_t wstride, float* __restrict__ SO, int64_t stride, int64_t len,
+                   int64_t wstride, float* __restrict__ SO, int64_t stride, int64_t len, MarkShape shape,
                    const double* __restrict__ gauss_all, const double* __restrict__ taper_all,
                    const double* __restrict__ tw64) {
     __shared__ cd xs[kWarps][kW];
@@ -515,11 +515,11 @@ __global__ void __launch_bounds__(kWarps * 32)
     cd* x = xs[warp];
     const cd scale{0.125, 0.0};  // 1/sqrt(64) (helper.h:102-104)
     const int64_t end = min((int64_t)len, (int64_t)(d.H - 1) * d.dim_i + d.diml);
-    constexpr int kStep = kDirect ? 1 : 32, kGroups = kDirect ? 1 : kScanGroups;
-    const int64_t far = (int64_t)gridDim.x * kWarps * kStep;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * kStep; q0 < end; q0 += far * kGroups) {
+    const int step = kDirect ? 1 : shape.step, groups = kDirect ? 1 : shape.groups;
+    const int64_t far = (int64_t)gridDim.x * kWarps * step;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kWarps + warp) * step; q0 < end; q0 += far * groups) {
         MarkScan marks;
-        if (!kDirect) marks.read(out, q0, far, end, kUndecided, lane);
+        if (!kDirect) marks.read(out, q0, far, end, shape, kUndecided, lane);
         int64_t p = q0;
         for (bool some = kDirect ? true : marks.next(q0, far, p); some; some = !kDirect && marks.next(q0, far, p)) {
             const int i = owner_row(d, first, last, p);  // warp-uniform; only valid cells are marked
@@ -618,8 +618,9 @@ cudaError_t launch_local_radon(const DevGeometry& g, const Batch& b, int slot0, 
                                                                                         SO, stride, tiles_j);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_lradon_exact<false><<<dim3(mark_blocks(len, kWarps, count), count), kWarps * 32, 0, st>>>(
-        g, b, slot0, SI, W, wstride, SO, stride, len, gauss, taper, tw64);
+    const MarkShape shape = mark_shape(len, kWarps, count);
+    k_lradon_exact<false><<<dim3(shape.blocks, count), kWarps * 32, 0, st>>>(g, b, slot0, SI, W, wstride, SO, stride, len,
+                                                                            shape, gauss, taper, tw64);
     return cudaGetLastError();
 }
 
@@ -628,8 +629,8 @@ cudaError_t launch_local_radon_direct(const DevGeometry& g, const Batch& b, cons
                                       cudaStream_t st) {
     if (b.count == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<int64_t>((len + kWarps - 1) / kWarps, 8192);
-    k_lradon_exact<true><<<dim3(blocks, b.count), kWarps * 32, 0, st>>>(g, b, 0, SI, nullptr, 0, SO, stride, len, gauss,
-                                                                       taper, tw64);
+    k_lradon_exact<true><<<dim3(blocks, b.count), kWarps * 32, 0, st>>>(g, b, 0, SI, nullptr, 0, SO, stride, len,
+                                                                       MarkShape(), gauss, taper, tw64);
     return cudaGetLastError();
 }
 
