@@ -36,6 +36,9 @@
 // 64-cell windows read from the staged segments), and max-deskews into the tile's
 // accumulator in shared memory.  The skewed input and output never reach HBM; the orientations
 // (4 x N floats per image) stay L2-resident.
+#include <algorithm>
+#include <atomic>
+
 #include <cooperative_groups.h>
 
 #include "cepstrum_bin.cuh"
@@ -44,8 +47,7 @@ namespace ske {
 
 namespace {
 
-constexpr int kCRows = 256;            // accumulator tile rows
-constexpr int kCBand = kCRows + 34;    // skewed rows of a tile per sector (drift <= 32 over 32 columns)
+constexpr int kCTall = 256, kCLow = 64;  // accumulator tile rows, by launch_cepstrum_f32
 constexpr int kCSeg = 96;              // staged cells per band row: columns j0-32 .. j0+63
 constexpr int kCThreads = 512;
 constexpr int kCWarps = kCThreads / 32;
@@ -166,7 +168,9 @@ __device__ __forceinline__ bool constant_window(const float* __restrict__ w) {
     return same;
 }
 
+template <int kCRows>
 struct CSmem {
+    static constexpr int kCBand = kCRows + 34;  // skewed rows of a tile per sector (drift <= 32 over 32 columns)
     f2 seg[kCBand / 2][kCSeg];  // two band rows in the halves
     int val[kCBand][32];   // bins
     int acc[kCRows][32];   // the tile's accumulator: see k_cepstrum_fused
@@ -179,9 +183,9 @@ struct CSmem {
 // A tile three quarters of whose cells cepstrum_bin left for cepstrum_f32 (a flat
 // image's, one far from 1) goes without it for a sector, then for two, four and up
 // to kMostDirect, until it decides again: a flat 512 x 512 image 7.09 -> 5.85 ms (6.64
-// with every cell in cepstrum_f32), one of 1e-30 7.23 -> 5.50 (5.25).  Half of the cells
-// as the limit, or a longer first wait, costs images that are flat along some angles
-// only (ramps, checks) more than it gains the others.
+// with every cell in cepstrum_f32), one of 1e-30 7.23 -> 5.50 (5.25), a flat 2048 x 2048
+// one 99.0 -> 82.9 (79.3).  Waits that grow by four (80.3) cost a 512 x 512 ramp, flat
+// along some angles only, 3.97 ms for 3.19.
 constexpr int kFirstDirect = 1, kMostDirect = 16;
 
 // The reference's max+angle update o = angle + 1000*(int)(max(o, m)/1000) keeps
@@ -195,10 +199,12 @@ constexpr int kEmptied = 1 << 30;  // in CSmem::acc, beside the largest bin + 1
 // One launch: blockIdx.y = image; blockIdx.x = (type, tile row, tile column);
 // blockIdx.z, the rank in the cluster: which of the type's runs of sectors.  The
 // CTAs of a cluster join their runs through distributed shared memory.
+template <int kCRows>
 __global__ void __launch_bounds__(kCThreads, 1)
     k_cepstrum_fused(BatchTables T, DevGeometry g, TypeLists tl, int dim, int tiles_x, int tiles_y) {
     extern __shared__ __align__(16) unsigned char smem_c[];
-    CSmem& sm = *reinterpret_cast<CSmem*>(smem_c);
+    typedef CSmem<kCRows> Smem;
+    Smem& sm = *reinterpret_cast<Smem*>(smem_c);
     f2(*seg)[kCSeg] = sm.seg;
     int(*val)[32] = sm.val;
     const int per_type = tiles_x * tiles_y;
@@ -232,7 +238,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
         const int32_t* rlast = g.last + d.row_off;
         const int tmin = tg[j0], tmax = tg[jlast];
         const int r0 = i0 + tmin;
-        const int nrows = ni + 1 + (tmax - tmin);  // <= kCBand for square grids
+        const int nrows = ni + 1 + (tmax - tmin);  // <= Smem::kCBand for square grids
         // Stage the band's row segments (skewed cells gathered from the orientation).
         // A warp per row, three columns per lane whose shifts and weights stay in
         // registers.
@@ -361,20 +367,43 @@ cudaError_t cepstrum_f32_init_tables() {
     return cudaMemcpyToSymbol(c_w64, w, sizeof(w));
 }
 
-cudaError_t launch_cepstrum_f32(const BatchTables& t, int images, const DevGeometry& g, const TypeLists& tl, int dim,
-                                cudaStream_t st) {
-    if (images <= 0) return cudaSuccess;
+// Resident clusters of `size` CTAs of the kernel with kCRows-row tiles (0: that size
+// does not run), asked once per device.
+template <int kCRows>
+static int resident_clusters(int size, cudaLaunchConfig_t cfg) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices][4];  // + 1
+    int dev = 0, resident = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    std::atomic<int>* slot = dev < kDevices ? &known[dev][size < 2 ? 0 : size < 4 ? 1 : size < 8 ? 2 : 3] : nullptr;
+    if (slot && slot->load(std::memory_order_relaxed) > 0) return slot->load(std::memory_order_relaxed) - 1;
+    if (cudaOccupancyMaxActiveClusters(&resident, k_cepstrum_fused<kCRows>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        resident = 0;
+    }
+    if (slot) slot->store(resident + 1, std::memory_order_relaxed);
+    return resident;
+}
+
+namespace {
+struct FusedLaunch {
+    int rows = 0, runs = 1;
+    double time = 0.0;  // of the slowest SM, in rows of a band
+};
+}  // namespace
+
+// kCRows-row tiles: notes in best which numbers of runs take less than what it holds,
+// or (null) launches with `runs`.
+template <int kCRows>
+static cudaError_t fused(const BatchTables& t, int images, const DevGeometry& g, const TypeLists& tl, int dim,
+                         cudaStream_t st, FusedLaunch* best, int runs) {
     const int tiles_x = (dim + 31) / 32, tiles_y = (dim + kCRows - 1) / kCRows;
     const int64_t blocks = (int64_t)4 * tiles_x * tiles_y;
     if (blocks > 0x7fffffff || images > 65535) return cudaErrorInvalidValue;
-    const int smem = (int)sizeof(CSmem);
-    cudaError_t e = cudaFuncSetAttribute(k_cepstrum_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int smem = (int)sizeof(CSmem<kCRows>);
+    cudaError_t e =
+        cudaFuncSetAttribute(k_cepstrum_fused<kCRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    // Runs of sectors per tile: the fewest whose waves of clusters, each as long as
-    // a run, come within 2% of the least.  Two images of 64x64 have 16 tiles, and
-    // walking their 45 sectors in turn left the other SMs idle: 1009 us with one
-    // run, 342 with eight (one image of 256x256: 2568 and 733).  16 images of
-    // 512x512 (2048 tiles, 13.5 waves of 152): 34.7 ms in one run, 34.0 in two.
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     cudaLaunchConfig_t cfg = {};
@@ -383,24 +412,49 @@ cudaError_t launch_cepstrum_f32(const BatchTables& t, int images, const DevGeome
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    int runs = 1;
-    double least = 0.0;
+    if (!best) {
+        attr.val.clusterDim = {1, 1, (unsigned)runs};
+        cfg.gridDim = dim3((unsigned)blocks, (unsigned)images, (unsigned)runs);
+        return cudaLaunchKernelEx(&cfg, k_cepstrum_fused<kCRows>, t, g, tl, dim, tiles_x, tiles_y);
+    }
+    int types = 0, most = 0;
+    for (int k = 0; k < 4; k++) {
+        types += tl.count[k] > 0;
+        most = std::max(most, tl.count[k]);
+    }
+    const int64_t clusters = (int64_t)types * tiles_x * tiles_y * images;
+    const int band = std::min(kCRows, dim) + 34 + 24;  // and what a sector costs besides its rows
     for (int s = 1; s <= 8; s *= 2) {
         attr.val.clusterDim = {1, 1, (unsigned)s};
         cfg.gridDim = dim3((unsigned)blocks, (unsigned)images, (unsigned)s);
-        int resident = 0;
-        if (cudaOccupancyMaxActiveClusters(&resident, k_cepstrum_fused, &cfg) != cudaSuccess) cudaGetLastError();
+        const int resident = resident_clusters<kCRows>(s, cfg);
         if (resident < 1) continue;
-        const int64_t clusters = blocks * images;
-        const double time = (double)((clusters + resident - 1) / resident) / s;
-        if (s == 1 || time < 0.98 * least) {
-            least = time;
-            runs = s;
-        }
+        const int64_t waves = (clusters + resident - 1) / resident;
+        const double length = waves > 1 ? std::max(1.0, (double)most / s) : (double)((most + s - 1) / s);
+        const double time = (double)waves * length * band;
+        if (best->rows == 0 || time < 0.98 * best->time) *best = FusedLaunch{kCRows, s, time};
     }
-    attr.val.clusterDim = {1, 1, (unsigned)runs};
-    cfg.gridDim = dim3((unsigned)blocks, (unsigned)images, (unsigned)runs);
-    return cudaLaunchKernelEx(&cfg, k_cepstrum_fused, t, g, tl, dim, tiles_x, tiles_y);
+    return cudaSuccess;
+}
+
+// Tall tiles, 256 rows, form 1.13 cepstra per skewed cell, low ones, 64, 1.5.  The rows
+// and the runs of sectors per tile: of the choices whose waves of clusters, each as
+// long as a run, come within 2% of the least the first, tall tiles and few runs
+// before low and many.  Two images of 64x64 have 16 tiles, and walking their 45
+// sectors in turn left the other SMs idle: 1009 us with one run, 342 with eight (one
+// image of 256x256: 2568 and 733).  16 images of 512x512 (2048 tiles, 13.5 waves of
+// 152): 34.7 ms in one run, 34.0 in two.  One sector of 512x512, 32 tall tiles or 128
+// low ones: 113 and 71 us, flat 207 and 107; eight of one type, one run or four: 498
+// and 169.
+cudaError_t launch_cepstrum_f32(const BatchTables& t, int images, const DevGeometry& g, const TypeLists& tl, int dim,
+                                cudaStream_t st) {
+    if (images <= 0) return cudaSuccess;
+    FusedLaunch best;
+    cudaError_t e = fused<kCTall>(t, images, g, tl, dim, st, &best, 0);
+    if (e == cudaSuccess && dim > kCLow) e = fused<kCLow>(t, images, g, tl, dim, st, &best, 0);
+    if (e != cudaSuccess) return e;
+    return best.rows == kCLow ? fused<kCLow>(t, images, g, tl, dim, st, nullptr, best.runs)
+                              : fused<kCTall>(t, images, g, tl, dim, st, nullptr, best.runs);
 }
 
 }  // namespace ske
