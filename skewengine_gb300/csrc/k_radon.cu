@@ -211,22 +211,6 @@ struct RowPart {
     }
 };
 
-// Two floats at a time (f32x2): plain IEEE additions of both halves.
-__device__ __forceinline__ float2 add_pair(float2 a, float2 b) {
-    float2 r;
-    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2,%3}; mov.b64 y, {%4,%5}; add.rn.f32x2 z, x, y; mov.b64 {%0,%1}, z; }"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-__device__ __forceinline__ float2 sub_pair(float2 a, float2 b) {
-    float2 r;
-    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2,%3}; mov.b64 y, {%4,%5}; sub.rn.f32x2 z, x, y; mov.b64 {%0,%1}, z; }"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
-}
-
 template <bool kF32, bool kOver, int kFlight>
 __global__ void __launch_bounds__(kRowWarps * 32)
     k_radon_rows(DevGeometry g, Batch b, const float* __restrict__ orient, int64_t n_cells, int dimx, int dimy,
@@ -359,26 +343,33 @@ __global__ void __launch_bounds__(kRowWarps * 32)
         const float c1 = __uint_as_float((unsigned)(e1 + 23 + 127) << 23 | 0x400000u);
         const float c2 = __uint_as_float((unsigned)(e2 + 23 + 127) << 23 | 0x400000u);
         const float c3 = __uint_as_float((unsigned)(e3 + 23 + 127) << 23 | 0x400000u);
-        const float2 C1 = make_float2(c1, c1), C2 = make_float2(c2, c2), C3 = make_float2(c3, c3);
-        float2 s1 = make_float2(0.0f, 0.0f), s2 = s1, s3 = s1, left = s1;
+        const f2 C1 = pk(c1, c1), C2 = pk(c2, c2), C3 = pk(c3, c3);
+        f2 s1 = 0, s2 = 0, s3 = 0;
+        float left[2] = {0.0f, 0.0f};
         walk([&](const float* v) {
 #pragma unroll
             for (int q = 0; q < kRowStep; q += 2) {
-                const float2 x = make_float2(v[q], v[q + 1]);
-                const float2 h1 = sub_pair(add_pair(x, C1), C1), x1 = sub_pair(x, h1);
-                const float2 h2 = sub_pair(add_pair(x1, C2), C2), x2 = sub_pair(x1, h2);
-                const float2 h3 = sub_pair(add_pair(x2, C3), C3), x3 = sub_pair(x2, h3);
-                s1 = add_pair(s1, h1);
-                s2 = add_pair(s2, h2);
-                s3 = add_pair(s3, h3);
-                left.x += fabsf(x3.x);  // not zero, or NaN: something is left
-                left.y += fabsf(x3.y);
+                const f2 x = pk(v[q], v[q + 1]);
+                const f2 h1 = sub2(add2(x, C1), C1), x1 = sub2(x, h1);
+                const f2 h2 = sub2(add2(x1, C2), C2), x2 = sub2(x1, h2);
+                const f2 h3 = sub2(add2(x2, C3), C3), x3 = sub2(x2, h3);
+                s1 = add2(s1, h1);
+                s2 = add2(s2, h2);
+                s3 = add2(s3, h3);
+                float r0, r1;
+                upk(x3, r0, r1);
+                left[0] += fabsf(r0);  // not zero, or NaN: something is left
+                left[1] += fabsf(r1);
             }
         });
-        rest = !(left.x + left.y == 0.0f);
-        sums[0][warp][lane] = s1.x + s1.y;
-        sums[1][warp][lane] = s2.x + s2.y;
-        sums[2][warp][lane] = s3.x + s3.y;
+        rest = !(left[0] + left[1] == 0.0f);
+        const f2 cut[3] = {s1, s2, s3};
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            float a, c;
+            upk(cut[k], a, c);
+            sums[k][warp][lane] = a + c;
+        }
     }
     marks[warp][lane] = rest;
     const bool again = __syncthreads_or(rest);
