@@ -24,9 +24,10 @@
 //    product, whose logarithm is formed anyway; |window|^2 comes from the spectrum
 //    (Parseval), off by 10^-5 of itself against the 3 10^-3 the bound has to spare.
 //  * A thread evaluates two windows in the halves of f32x2 registers, from samples
-//    staged as such pairs: the transform and the sums take half the instructions
-//    (650 a cell against 1290).  What is left to the FMA pipe is the same, and it
-//    is the bound now (f32x2 occupies it for two cycles).
+//    staged as such pairs: the transform and the sums take the instructions of one
+//    (a 512 x 512 texture, 180 angles: 2.2 ms with one window a thread, 1.86 with two).
+//    What is left to the FMA pipe is the same, and it is the bound now (f32x2 occupies
+//    it for two cycles).
 //  * c_4 .. c_15 are cosine sums folded over n, 16 - n and 8 - n: 62
 //    multiply-adds; their roundings stay below 14 u times the sum of the logs, at most 17
 //    times the largest.

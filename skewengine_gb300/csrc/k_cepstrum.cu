@@ -22,8 +22,8 @@
 // pipe 84% busy).  So the cepstrum is formed in float with a bound on its error
 // (a thread per two cells, the windows in registers), and only the cells whose bin
 // that leaves open run the exact kernel.  The whole run of a 512 x 512 texture
-// (180 angles): 353.3 ms with every cell in binary64, 2.75 ms so (the float
-// kernel 1.9, the open cells 0.56); 3.20 with a thread per cell.
+// (180 angles): 353.3 ms with every cell in binary64, 2.57 ms so (the float
+// kernel 1.86, the open cells 0.40).
 // cepstrum_bin.cuh has the evaluation and its bounds.
 #include "cepstrum_bin.cuh"
 

@@ -875,7 +875,7 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* dw, int n, i
 // sum is plain float32 additions (27 pixels of a million of 32 channels), from
 // there on the roundings are carried along: plain to the end, the gradient was up
 // to twice as far from float64 as the tensor reduction's.  Memory bound (6 bytes a
-// value): 100 MB at 16 x 128 x 128 x 64, 17 us against 195 us for the comparison,
+// value): 100 MB at 16 x 128 x 128 x 64, 16 us against 195 us for the comparison,
 // product, conversion and reduction one after another.
 constexpr int kReluBlocks = 608;   // 4 per SM
 constexpr int kReluMaxC = 2048;    // channels: C / 8 divides 256

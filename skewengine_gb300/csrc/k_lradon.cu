@@ -15,7 +15,7 @@
 // per 512 x 512 image at all 180 angles, that pipe 83% busy).  Every value the
 // output depends on is a comparison or one rounding to float, so a cheaper
 // evaluation with a proven error decides it unless it falls within that error
-// of a tie (the whole run of that image: 278.7 ms before, 3.4 ms so, of it 0.25 ms
+// of a tie (the whole run of that image: 278.7 ms before, 3.34 ms so, of it 0.25 ms
 // in step 1, 2.4 in step 2 and 0.35 in step 3):
 //  1. k_lradon_sums: W of every row, once per column (the tile-by-tile form
 //     recomputed each about three times), as exact 64-bit integer prefix sums

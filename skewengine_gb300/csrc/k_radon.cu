@@ -149,11 +149,11 @@ __global__ void __launch_bounds__(kSumWarps * 32)
 // its columns, touched up to 32 lines a load at 45 degrees, took 15 integer
 // operations a cell to add it up exactly and reduced every row over the lanes:
 // 137 us per 512 x 512 image at 180 angles, this form 62 us in binary64's stead
-// (13 instructions a cell are the cuts) and 45 us in float at 383 x 509.
+// (13 instructions a cell are the cuts) and 48 us in float at 383 x 509.
 // Where all 32 rows hold a batch of 32 columns with both their sources, which is
 // most of a sector, a cell is two loads at one address, two products and a sum,
-// 16 columns in flight; elsewhere each source is tested, 69 us for all of them
-// (both shapes).  The next batch's shifts and weights are on their way meanwhile.
+// 16 columns in flight; elsewhere each source is tested, about 70 us for all of
+// them (both shapes).  The next batch's shifts and weights are on their way meanwhile.
 // A cell is the skew's, w x[r-t-1] + (1-w) x[r-t], up to the sign of a zero.
 //
 // Exact sums in float.  With |cell| <= 2^E (E from the grid's largest finite
