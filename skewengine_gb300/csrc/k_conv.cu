@@ -1980,7 +1980,8 @@ static int ske_conv3x3_wgrad_bf16_impl(const void* x, const void* dy, float* dw,
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0 &&
         wg_geometry(&wg, n, h, w_, cin, cout, sms)) {
         const int smem = std::max(kWsMinSmem, kWgStages * wg.sbytes + 256);
-        if (cudaFuncSetAttribute(k_conv3x3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        if (smem > 227 * 1024 ||
+            cudaFuncSetAttribute(k_conv3x3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
             return SKE_ERR_CUDA;
         const dim3 g3((unsigned)((cin + wg.nblk - 1) / wg.nblk), (unsigned)((cout + 127) / 128),
                       (unsigned)((wg.total + wg.chunk - 1) / wg.chunk));

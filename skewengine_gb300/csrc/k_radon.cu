@@ -846,7 +846,7 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
         if (e != cudaSuccess) return e;
         const int smem = max_H2 * (int)sizeof(float2);
         if (smem > 48 * 1024) {
-            e = cudaFuncSetAttribute(k_radon_transform_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = allow_smem(k_radon_transform_f32, smem);
             if (e != cudaSuccess) return e;
         }
         k_radon_transform_f32<<<b.count, kTransformThreads, smem, st>>>(g, b, Pc, pstride, twiddles, tw_off);
@@ -860,7 +860,7 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
     if (orient && in_width && max_H2 <= kSmemH2 && g_radon_path == 0) {  // one fused launch: a cluster per sector
         const int smem = max_H2 * (int)sizeof(cd);
         cudaError_t e = cudaSuccess;
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(k_radon_sector, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (smem > 48 * 1024) e = allow_smem(k_radon_sector, smem);
         if (e != cudaSuccess) return e;
         k_radon_sector<<<dim3(kClusterCtas, b.count), kTransformThreads, smem, st>>>(g, b, orient, n_cells, Pc, pstride,
                                                                                    twiddles, tw_off);
@@ -881,7 +881,7 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
     if (max_H2 <= kSmemH2 && min_H2 >= kQuadMinH2) {  // H2 / 4 entries twice, and H2 row sums
         const int smem = max_H2 * (int)(sizeof(cd) / 2 + sizeof(double));
         if (smem > 48 * 1024) {
-            e = cudaFuncSetAttribute(k_radon_transform_quad, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            e = allow_smem(k_radon_transform_quad, smem);
             if (e != cudaSuccess) return e;
         }
         k_radon_transform_quad<<<kQuad * b.count, kQuadThreads, smem, st>>>(g, b, Pc, pstride, twiddles, tw_off);
@@ -894,7 +894,7 @@ cudaError_t launch_radon(const DevGeometry& g, const Batch& b, const float* SI, 
     }
     const int smem = max_H2 <= kSmemH2 ? max_H2 * (int)sizeof(cd) : 0;
     if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(k_radon_transform, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_smem(k_radon_transform, smem);
         if (e != cudaSuccess) return e;
     }
     k_radon_transform<<<b.count, kTransformThreads, smem, st>>>(g, b, Pc, pstride, twiddles, tw_off, smem);

@@ -381,7 +381,7 @@ void sdem_items(const Geometry& geo, const Batch& b, std::vector<uint64_t>& item
 cudaError_t launch_sdem_chunked(const SdemLaunch& a, int num_sms, cudaStream_t st) {
     if (a.n_items == 0) return cudaSuccess;
     const size_t smem = sizeof(float) * (size_t)warp_floats(a.max_row) * kWarps;
-    cudaError_t e = cudaFuncSetAttribute(k_sdem_chunked, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k_sdem_chunked, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sdem_chunked, kWarps * 32, smem);

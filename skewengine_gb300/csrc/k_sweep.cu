@@ -549,7 +549,7 @@ size_t sdem_list_bytes(int max_row, int num_sms) {
 int sdem_max_ctas_per_sm(const SdemLaunch& a) {
     const size_t smem = sizeof(float) * (size_t)LLayout(std::max(a.max_row, 1)).total * kLWarps;
     auto kern = a.batched ? k_sweep<true> : k_sweep<false>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (allow_smem(kern, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
@@ -567,7 +567,7 @@ cudaError_t launch_sdem(const SdemLaunch& a, int num_sms, cudaStream_t st) {
     if (!level_ok(a.lvl0) || (a.lvl1 != 0 && !level_ok(a.lvl1)) || a.ctas_per_sm < 0) return cudaErrorInvalidValue;
     const size_t smem = sizeof(float) * (size_t)LLayout(a.max_row).total * kLWarps;
     auto kern = a.batched ? k_sweep<true> : k_sweep<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLWarps * 32, smem);

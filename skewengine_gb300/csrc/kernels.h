@@ -285,6 +285,16 @@ cudaError_t launch_cepstrum_bins(const DevGeometry& g, const Batch& b, const flo
 cudaError_t sdem_init_tables();   // both sweeps'
 cudaError_t sweep_init_tables();  // the compacting sweep's
 
+// Lets a kernel without static shared memory be launched with `bytes` of dynamic.
+// The limit belongs to the kernel, not to the launch: set to the bytes of each, it
+// could be another thread's smaller one by the time of the launch.
+template <typename Kernel>
+cudaError_t allow_smem(Kernel* kernel, size_t bytes) {
+    constexpr size_t kMost = 227 * 1024;
+    if (bytes > kMost) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
+}
+
 // Record `msg` as the calling thread's last error (ske_last_error) and return code.
 int set_last_error(int code, const char* msg);
 
