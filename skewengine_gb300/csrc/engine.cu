@@ -1238,7 +1238,12 @@ int build_image_plan(int dim, int count, const int32_t* angles, int nangles, Ima
     p->angles.assign(angles, angles + nangles);
     SKE_TRY(make_grid_geo(dim, dim, &p->geo));
     memset(&p->tl, 0, sizeof(p->tl));
+    // Of an angle listed more than once the last place counts: the maximum has its bins
+    // by then, or it empties the cell again.  (So a type has no more than its angles.)
+    std::vector<int> last(kMaxSectors, -1);
+    for (int k = 0; k < nangles; k++) last[angles[k]] = k;
     for (int k = 0; k < nangles; k++) {
+        if (last[angles[k]] != k) continue;
         const int t = p->geo->geo.desc[angles[k]].type;
         p->tl.angle[t][p->tl.count[t]] = angles[k];
         p->tl.slot[t][p->tl.count[t]] = k;
