@@ -230,20 +230,19 @@ struct CellSmem {
 
 // Binary64 w in units of 2^(emax - 1023 - 26), emax at least w's exponent field:
 // hi the nearest integer, lo the rest to 2^-25 (bit operations: conversions run
-// on the FP64 pipe).  lo is 2^-26 at least where w is not zero and hi is, so that
-// only zeros have neither (a texture beside 1e17 lies below 2^-26 units).
+// on the FP64 pipe).  A w below 2^-26 units counts as one of them, so that only zeros
+// have neither (a texture beside 1e17 lies below).
 __device__ __forceinline__ void split(double w, int emax, int* hi, float* lo) {
     const long long bits = __double_as_longlong(w);
     const int e = (int)((bits >> 52) & 0x7ff);
     const long long s = (bits & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
-    const int t = min(26 + emax - e, 88);  // w = s 2^-t units
+    const int t = min(26 + emax - e, 78);  // w = s 2^-t units
     long long h = 0, rem = s;
     if (t <= 60) {
         h = (s + (1ll << (t - 1))) >> t;
         rem = s - (h << t);
     }
-    const int low = (int)(rem >> min(t - 26, 63)) | (t > 60 && s != 0);
-    const float l = __fmul_rn(__int2float_rn(low), 1.4901161193847656e-8f);  // 2^-26
+    const float l = __fmul_rn(__int2float_rn((int)(rem >> (t - 26))), 1.4901161193847656e-8f);  // 2^-26
     *hi = bits < 0 ? -(int)h : (int)h;
     *lo = bits < 0 ? -l : l;
 }
